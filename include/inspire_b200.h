@@ -277,8 +277,7 @@ int ipir_b200_autotune(ipir_server* srv);
 /* The schedule the handle uses for `count` queries. */
 int ipir_b200_get_schedule(const ipir_server* srv, size_t count, ipir_serve_schedule* out);
 /* Pin the schedule the handle uses for `count` queries (tp_pass at most
- * the handle's tensor-pass capacity, min(max_batch, 32) or less for large
- * group counts): 0, 1 null argument, 2 out of range. */
+ * min(max_batch, 32)): 0, 1 null argument, 2 out of range. */
 int ipir_b200_set_schedule(ipir_server* srv, size_t count, const ipir_serve_schedule* sc);
 /* Kernels launched by the handle's answer pipeline since create. */
 int ipir_b200_launch_count(const ipir_server* srv, unsigned long long* out);

@@ -132,6 +132,13 @@ void build_tables(DevTables& T) {
     T.crt_c[1] = (uint32_t)powmod(kQ0 % kQ1, kQ1 - 2, kQ1);
     T.crt_cp[0] = shoup(T.crt_c[0], kQ0);
     T.crt_cp[1] = shoup(T.crt_c[1], kQ1);
+    uint32_t p5 = 1;
+    for (uint32_t m = 0; m < (uint32_t)kHalf; ++m, p5 = p5 * 5 % (2 * kN))
+        for (uint32_t rho = 0; rho < 2; ++rho) {
+            const uint32_t slot = brev(((rho ? 2 * kN - p5 : p5) - 1) / 2, kLogN);
+            T.slot_of[rho * kHalf + m] = (uint16_t)slot;
+            T.exp_of[slot] = (uint16_t)(rho * kHalf + m);
+        }
 }
 
 // ------------------------------------------------------------------ setup

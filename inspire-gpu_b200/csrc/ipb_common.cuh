@@ -56,6 +56,10 @@ struct LimbTables {
 struct DevTables {
     LimbTables limb[2];
     uint32_t crt_c[2], crt_cp[2];  // q1^-1 mod q0, q0^-1 mod q1 and Shoup factors
+    // The slots' odd exponents 2 BR(slot) + 1 = (-1)^rho 5^m mod 2N:
+    // slot_of[rho * N/2 + m] and its inverse.
+    alignas(16) uint16_t slot_of[kN];
+    uint16_t exp_of[kN];
 };
 
 // ------------------------------------------------------------ arithmetic

@@ -13,12 +13,14 @@ struct DevTables;
 // ---------------------------------------------------------------- online
 // Flat per-query device input (u64, the capi.h flat query layout):
 //   [b0: rows][b1: rows][ksk5: blk][kskneg1: blk][rgsw: 4 blk],  blk = 2*2*N.
-// qprep: keys [q][key(2)][limb][digit][N] NTT form, rgsw32 [q][4][digit][limb][N].
+// qprep: KSK5 byte planes kplanes [q][limb][byte][4096] (tensorpass_tc.cu),
+// KSK-1 keys [q][limb][digit][N] NTT form, rgsw32 [q][4][digit][limb][N].
 cudaError_t launch_qprep(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T,
-                         uint32_t* keys, uint32_t* rgsw32, int nq, cudaStream_t s);
+                         uint8_t* kplanes, uint32_t* keys, uint32_t* rgsw32, int nq, cudaStream_t s);
 // Only some of it: parts 1 = the keys, 2 = the RGSW parts, 3 = both.
 cudaError_t launch_qprep_parts(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T,
-                               uint32_t* keys, uint32_t* rgsw32, int nq, int parts, cudaStream_t s);
+                               uint8_t* kplanes, uint32_t* keys, uint32_t* rgsw32, int nq, int parts,
+                               cudaStream_t s);
 
 // Mat-vec row-split partials part[q][chunk][limb][cols] for nq <= 4 queries
 // sharing one DB stream.  chunks must divide rows.
@@ -64,39 +66,40 @@ cudaError_t launch_matvec_tc_ranges(const uint16_t* db, size_t rows, size_t ld, 
 cudaError_t launch_mv_chunk_reduce(const uint32_t* part, size_t part_qstride, int chunks, size_t cols,
                                    const DevTables* T, uint32_t* out, size_t out_qstride, int nq, cudaStream_t s);
 
-// Tensor pass on tcgen05 (tensorpass_tc.cu).  Dt: re-laid-out D tensors
-// [l][i][g*4 + a][4096] u8; keyt: per-pass key table scratch
-// (tp_keyt_bytes); tp_out: [l][i][q][g] u32 for the nq_total queries of
-// the batch.
+// Tensor pass on tcgen05 (tensorpass_tc.cu).  Dt: the re-laid-out D tensors,
+// 128-row tiles of 32 slots, 128 tiles per group in (group, limb, slot) order
+// (tp_tiles(groups) in all); kplanes: the queries' KSK5 byte planes,
+// kTpPlaneBytes apart; tp_out: [q][g][l][N] u32, out_qstride words per query.
+// A launch covers tiles [tile0, tile0 + n_tiles) for nq <= kTpMaxQueries
+// queries; query p's results go to row qmap[p] of tp_out (p without a map).
+constexpr int kTpMaxQueries = 32;
+constexpr size_t kTpPlaneBytes = (size_t)2 * 4 * 4096;
 size_t tp_dt_bytes(size_t groups);
-size_t tp_keyt_bytes(int max_pass);
-int tp_pass_queries(size_t groups);
-cudaError_t launch_dt_transpose(const uint32_t* dp, const uint32_t* dm, size_t g0, size_t nw, size_t G, uint8_t* Dt,
-                                cudaStream_t s);
-cudaError_t launch_dt_export(const uint8_t* Dt, size_t g, size_t G, uint32_t* dp, uint32_t* dm, cudaStream_t s);
-cudaError_t launch_tensor_pass(const uint8_t* Dt, size_t G, const uint32_t* keys, size_t key_qstride, int nq,
-                               int nq_total, int q0, uint32_t* keyt, uint32_t* tp_out, int* err, unsigned* tiles,
+int tp_tiles(size_t groups);
+cudaError_t launch_tensor_pass(const uint8_t* Dt, int tile0, int n_tiles, const uint8_t* kplanes, int nq,
+                               const uint8_t* qmap, uint32_t* tp_out, size_t out_qstride, int* err, unsigned* tiles,
                                int num_sms, cudaStream_t s);
-// The same for the (limb, slot) indices l * N + i in [li0, li0 + n_li) only
-// (multiples of 32), all groups: writes tp_out[l][i][q'][g] for those
-// indices, q' = qmap[q0 + p] for pass query p when qmap (the output rows of
-// queries 0 .. q0 + nq - 1 of the pass, < nq_total) is given, else q0 + p.
-cudaError_t launch_tensor_pass_slots(const uint8_t* Dt, size_t G, int li0, int n_li, const uint32_t* keys,
-                                     size_t key_qstride, int nq, int nq_total, int q0, const uint8_t* qmap,
-                                     uint32_t* keyt, uint32_t* tp_out, int* err, unsigned* tiles, int num_sms,
-                                     cudaStream_t s);
+// Groups [g0, g0 + nw) from one wave in the reference layout into Dt.
+cudaError_t launch_dt_transpose(const uint32_t* dp, const uint32_t* dm, size_t g0, size_t nw, const DevTables* T,
+                                uint8_t* Dt, cudaStream_t s);
+cudaError_t launch_dt_export(const uint8_t* Dt, size_t g, const DevTables* T, uint32_t* dp, uint32_t* dm,
+                             cudaStream_t s);
+// nrows 4096-byte rows, from row0 on, of the checkpoint files' order of the
+// tensors of G groups, copied between `file` (device memory) and Dt.
+cudaError_t launch_dt_file_rows(uint8_t* Dt, size_t G, size_t row0, size_t nrows, uint8_t* file, bool to_file,
+                                const DevTables* T, cudaStream_t s);
 
-// packed_b[q][g][limb][N] = NTT(sum_y mvpart) - tp_out - Dfinal (.) Kn1.
+// packed_b[q][g][limb][N] = NTT(sum_y mvpart) - tp_out - Dfinal (.) Kn1
+// (tp_out strided as packed_b).
 cudaError_t launch_finalize(const uint32_t* mvpart, size_t mv_qstride, int mv_chunks, size_t cols,
                             const uint32_t* tp_out, const uint32_t* df, const uint32_t* keys, size_t key_qstride,
                             const DevTables* T, uint32_t* packed_b, size_t pb_qstride, size_t groups, int nq,
                             cudaStream_t s);
-// The same for the groups [g0, g0 + gn) of nq queries whose tensor-pass
-// results are queries tp_q0 .. tp_q0 + nq - 1 of a pass of tp_nq_total.
+// The same for the groups [g0, g0 + gn).
 cudaError_t launch_finalize_range(const uint32_t* mvpart, size_t mv_qstride, int mv_chunks, size_t cols,
-                                  const uint32_t* tp_out, int tp_nq_total, int tp_q0, const uint32_t* df,
-                                  const uint32_t* keys, size_t key_qstride, const DevTables* T, uint32_t* packed_b,
-                                  size_t pb_qstride, size_t groups, size_t g0, size_t gn, int nq, cudaStream_t s);
+                                  const uint32_t* tp_out, const uint32_t* df, const uint32_t* keys,
+                                  size_t key_qstride, const DevTables* T, uint32_t* packed_b, size_t pb_qstride,
+                                  size_t groups, size_t g0, size_t gn, int nq, cudaStream_t s);
 
 // Horner chains, one CTA per (ct, query): resp[q][ct][a|b][limb][N] u64.
 cudaError_t launch_horner(const uint32_t* pre_a, const uint32_t* packed_b, size_t pb_qstride,

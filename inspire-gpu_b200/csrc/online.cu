@@ -2,7 +2,7 @@
 //
 // One answer (gpu_answer / gpu_answer_batch, reference src/gpu_protocol.cu:
 // 1121-1535) runs these launches on one stream:
-//   qprep     key-switching keys to NTT form, RGSW to u32 residues
+//   qprep     key-switching keys to NTT form (KSK5 as byte planes), RGSW to u32 residues
 //   matvec    r_l[j] = sum_i db[i][j] * b_l[i] mod q_l   (DB pass, HBM bound)
 //   tensor pass (tensorpass_tc.cu): sum_{dir,s,j} D[s][j][i] * K5[j][perm_s(i)]
 //   finalize  per group: NTT(r slice) - tensor partials - D_final (.) Kneg1
@@ -18,17 +18,6 @@
 namespace ipb {
 
 namespace {
-
-__device__ __forceinline__ uint32_t pow5_mod2n(uint32_t e) {
-    uint32_t r = 1, b = 5;
-    while (e) {
-        if (e & 1) r = (r * b) & (2 * kN - 1);
-        b = (b * b) & (2 * kN - 1);
-        e >>= 1;
-    }
-    return r;
-}
-constexpr uint32_t kInv5 = 3277;  // 5^-1 mod 2N (5 * 3277 = 4*4096 + 1)
 
 __device__ __forceinline__ void ld8(const uint32_t* p, uint32_t (&v)[8]) {
     uint4 a = *reinterpret_cast<const uint4*>(p);
@@ -46,10 +35,13 @@ __device__ __forceinline__ void st8(uint32_t* p, const uint32_t (&v)[8]) {
 // quarter of the RGSW u64 -> u32 reduction.  The client sends KSK b-parts in
 // coefficient form and RGSW in NTT form (capi.h:47-54); the reference NTTs the
 // keys on the server (src/gpu_protocol.cu:1059-1094).  Inputs are reduced
-// mod q (identical to the reference on canonical inputs).
+// mod q (identical to the reference on canonical inputs).  KSK5 leaves as the
+// tensor pass's N operand: byte planes kplanes[q][limb][byte][4096], digit j's
+// slots in the order of T.slot_of at positions j * N ..; KSK-1 as
+// keys[q][limb][digit][N].
 __global__ void __launch_bounds__(256) qprep_kernel(const uint64_t* __restrict__ qraw, size_t qstride,
                                                     size_t rows, const DevTables* __restrict__ T,
-                                                    uint32_t* __restrict__ keys,
+                                                    uint8_t* __restrict__ kplanes, uint32_t* __restrict__ keys,
                                                     uint32_t* __restrict__ rgsw32, int y0) {
     __shared__ __align__(16) uint32_t sbuf[2 * kN];
     const int b = blockIdx.x, y = y0 + (int)blockIdx.y;
@@ -64,8 +56,26 @@ __global__ void __launch_bounds__(256) qprep_kernel(const uint64_t* __restrict__
 #pragma unroll
         for (int e = 0; e < 8; ++e) r[e] = mod_u64(src[t + 256 * e], L.cr, L.q);
         ntt_fwd(r, sbuf, L.fwd, L.q, t, 0);
-        uint32_t* dst = keys + (size_t)b * (4 * kDeff * kN) + (size_t)((key * 2 + l) * kDeff + j) * kN;
-        st8(dst + 8 * t, r);
+        if (key == 1) {
+            st8(keys + ((size_t)(b * 2 + l) * kDeff + j) * kN + 8 * t, r);
+            return;
+        }
+        // Slots 8t .. 8t + 7 are this warp's own region of the NTT's second buffer.
+        uint32_t* slots = sbuf + kN;
+        st8(slots + 8 * t, r);
+        __syncthreads();
+        const uint4 so = *reinterpret_cast<const uint4*>(T->slot_of + 8 * t);
+        const uint32_t sw[4] = {so.x, so.y, so.z, so.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r[e] = slots[(sw[e >> 1] >> (16 * (e & 1))) & 0xFFFFu];
+        uint8_t* dst = kplanes + ((size_t)(b * 2 + l) * 4) * (kDeff * kN) + (size_t)j * kN + 8 * t;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            uint32_t w[2] = {0, 0};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e >> 2] |= ((r[e] >> (8 * p)) & 0xFFu) << (8 * (e & 3));
+            *reinterpret_cast<uint2*>(dst + (size_t)p * (kDeff * kN)) = make_uint2(w[0], w[1]);
+        }
     } else {
         const uint64_t* src = qr + 2 * rows + 2 * blk;
         uint32_t* dst = rgsw32 + (size_t)b * 4 * blk;
@@ -152,10 +162,11 @@ __global__ void __launch_bounds__(256) matvec_kernel(const uint16_t* __restrict_
 // Per (group, limb, query): b = NTT(sum of the mat-vec partials of the
 // group's N columns) - tensor pass - sum_j D_final[j] (.) Kneg1[j]
 // (reference src/gpu_protocol.cu:1233-1274, src/gpu_online.cu:547-559).
-// The tensor pass result is tp_out[l][i][q][g] (tensorpass_tc.cu).
+// The tensor pass result is tp_out[q][g][l][N] (tensorpass_tc.cu), laid out as
+// packed_b is.
 __global__ void __launch_bounds__(256) finalize_kernel(
     const uint32_t* __restrict__ mvpart, size_t mv_qstride, int mv_chunks, size_t cols,
-    const uint32_t* __restrict__ tp_out, int nq_total, int q_off, int groups, int g0,
+    const uint32_t* __restrict__ tp_out, int g0,
     const uint32_t* __restrict__ df, const uint32_t* __restrict__ keys, size_t key_qstride,
     const DevTables* __restrict__ T, uint32_t* __restrict__ packed_b, size_t pb_qstride) {
     __shared__ __align__(16) uint32_t sbuf[2 * kN];
@@ -172,14 +183,11 @@ __global__ void __launch_bounds__(256) finalize_kernel(
         r[e] = mod_u64(s, L.cr, L.q);
     }
     ntt_fwd(r, sbuf, L.fwd, L.q, t, 0);
-    uint32_t cs[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-        cs[e] = tp_out[(((size_t)l * kN + 8 * t + e) * nq_total + q_off + b) * groups + g];
-    uint32_t d0[8], d1[8], k0[8], k1[8];
+    uint32_t cs[8], d0[8], d1[8], k0[8], k1[8];
+    ld8(tp_out + (size_t)b * pb_qstride + ((size_t)g * 2 + l) * kN + 8 * t, cs);
     ld8(df + ((size_t)g * 2 + l) * kDeff * kN + 8 * t, d0);
     ld8(df + (((size_t)g * 2 + l) * kDeff + 1) * kN + 8 * t, d1);
-    const uint32_t* kn = keys + (size_t)b * key_qstride + (size_t)((1 * 2 + l) * kDeff) * kN;  // key 1 = kskneg1
+    const uint32_t* kn = keys + (size_t)b * key_qstride + (size_t)l * kDeff * kN;
     ld8(kn + 8 * t, k0);
     ld8(kn + kN + 8 * t, k1);
     uint32_t o[8];
@@ -733,16 +741,17 @@ cudaError_t launch_fill_db(uint16_t* out, size_t count, uint64_t seed, cudaStrea
 
 // ==================================================================== wrappers
 cudaError_t launch_qprep(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T,
-                         uint32_t* keys, uint32_t* rgsw32, int nq, cudaStream_t s) {
-    return launch_qprep_parts(qraw, qstride, rows, T, keys, rgsw32, nq, 3, s);
+                         uint8_t* kplanes, uint32_t* keys, uint32_t* rgsw32, int nq, cudaStream_t s) {
+    return launch_qprep_parts(qraw, qstride, rows, T, kplanes, keys, rgsw32, nq, 3, s);
 }
 
 cudaError_t launch_qprep_parts(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T,
-                               uint32_t* keys, uint32_t* rgsw32, int nq, int parts, cudaStream_t s) {
+                               uint8_t* kplanes, uint32_t* keys, uint32_t* rgsw32, int nq, int parts,
+                               cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
     if (parts < 1 || parts > 3) return cudaErrorInvalidValue;
     const int y0 = (parts & 1) ? 0 : 8, y1 = (parts & 2) ? 12 : 8;  // rows 0-7: key NTTs, 8-11: RGSW
-    qprep_kernel<<<dim3(nq, y1 - y0), 256, 0, s>>>(qraw, qstride, rows, T, keys, rgsw32, y0);
+    qprep_kernel<<<dim3(nq, y1 - y0), 256, 0, s>>>(qraw, qstride, rows, T, kplanes, keys, rgsw32, y0);
     return cudaGetLastError();
 }
 
@@ -779,19 +788,18 @@ cudaError_t launch_finalize(const uint32_t* mvpart, size_t mv_qstride, int mv_ch
                             const uint32_t* tp_out, const uint32_t* df, const uint32_t* keys, size_t key_qstride,
                             const DevTables* T, uint32_t* packed_b, size_t pb_qstride, size_t groups, int nq,
                             cudaStream_t s) {
-    return launch_finalize_range(mvpart, mv_qstride, mv_chunks, cols, tp_out, nq, 0, df, keys, key_qstride, T,
-                                 packed_b, pb_qstride, groups, 0, groups, nq, s);
+    return launch_finalize_range(mvpart, mv_qstride, mv_chunks, cols, tp_out, df, keys, key_qstride, T, packed_b,
+                                 pb_qstride, groups, 0, groups, nq, s);
 }
 
 cudaError_t launch_finalize_range(const uint32_t* mvpart, size_t mv_qstride, int mv_chunks, size_t cols,
-                                  const uint32_t* tp_out, int tp_nq_total, int tp_q0, const uint32_t* df,
-                                  const uint32_t* keys, size_t key_qstride, const DevTables* T, uint32_t* packed_b,
-                                  size_t pb_qstride, size_t groups, size_t g0, size_t gn, int nq, cudaStream_t s) {
+                                  const uint32_t* tp_out, const uint32_t* df, const uint32_t* keys,
+                                  size_t key_qstride, const DevTables* T, uint32_t* packed_b, size_t pb_qstride,
+                                  size_t groups, size_t g0, size_t gn, int nq, cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
-    if (gn == 0 || g0 + gn > groups || tp_q0 < 0 || tp_q0 + nq > tp_nq_total) return cudaErrorInvalidValue;
+    if (gn == 0 || g0 + gn > groups) return cudaErrorInvalidValue;
     finalize_kernel<<<dim3((unsigned)gn, 2, nq), 256, 0, s>>>(mvpart, mv_qstride, mv_chunks, cols, tp_out,
-                                                              tp_nq_total, tp_q0, (int)groups, (int)g0, df, keys,
-                                                              key_qstride, T, packed_b, pb_qstride);
+                                                              (int)g0, df, keys, key_qstride, T, packed_b, pb_qstride);
     return cudaGetLastError();
 }
 

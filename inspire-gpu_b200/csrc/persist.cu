@@ -9,8 +9,12 @@
 //   u64 n_entries, entry_bytes, db_rows, db_cols, n_packed, interp_d, num_cts,
 //   u8[64] CRS seed, u64 section bytes[4], u64 section checksums[4],
 //   zero padding; sections: DB (u16 [rows][cols], encoded), a (u32
-//   [group][limb][N]), D byte planes (u8 [limb][slot][g*4+byte][4096]),
+//   [group][limb][N]), D byte planes (u8 [limb][slot][g*4+byte][4096], of the
+//   positions (dir * 1023 + step) * 2 + digit 4092 used, the rest zero),
 //   D_final (u32 [group][limb][digit][N]).
+// The D section has this order whatever order the tensor pass keeps the
+// tensors in: whole rows are converted on the device, chunk by chunk, on the
+// way out and in.
 // Checksum of a section: sum over its 8-byte words w_i of
 // mix64(w_i + i * 0x9E3779B97F4A7C15) mod 2^64 (mix64: the splitmix64
 // finalizer), computed on the device, so a flipped, missing or moved word
@@ -36,6 +40,7 @@ constexpr char kMagic[8] = {'I', 'P', 'I', 'R', 'B', '2', '0', '0'};
 constexpr uint32_t kVersion = 1;
 constexpr uint32_t kHeaderBytes = 256;
 constexpr size_t kChunk = (size_t)64 << 20;  // pinned staging per copy (two, alternating)
+constexpr int kSecD = 2;                     // the D byte planes
 const char* const kSectionName[4] = {"DB", "a", "D byte planes", "D_final"};
 
 struct Header {
@@ -61,11 +66,12 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
     return z ^ (z >> 31);
 }
 
-__global__ void __launch_bounds__(256) checksum_kernel(const uint64_t* __restrict__ w, size_t n,
+// Adds the checksum terms of words [i0, i0 + n) of a section, at w, to *out.
+__global__ void __launch_bounds__(256) checksum_kernel(const uint64_t* __restrict__ w, size_t i0, size_t n,
                                                        unsigned long long* __restrict__ out) {
     uint64_t acc = 0;
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
-        acc += mix64(w[i] + i * 0x9E3779B97F4A7C15ull);
+        acc += mix64(w[i] + (i0 + i) * 0x9E3779B97F4A7C15ull);
 #pragma unroll
     for (int o = 16; o; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(out, (unsigned long long)acc);
@@ -82,15 +88,30 @@ Sections sections_of(const Precomp& P) {
                      tp_dt_bytes(G), G * kGroupStrideF * sizeof(uint32_t)}};
 }
 
-uint64_t device_checksum(const void* d, size_t bytes, unsigned long long* scratch, int num_sms, cudaStream_t s) {
-    IPB_CK(cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), s));
-    const size_t n = bytes / 8;  // every section is a multiple of 8 bytes
-    checksum_kernel<<<std::max(1, num_sms) * 8, 256, 0, s>>>(static_cast<const uint64_t*>(d), n, scratch);
-    IPB_CK(cudaGetLastError());
+void add_checksum(const void* d, size_t off, size_t bytes, unsigned long long* sum, int num_sms, cudaStream_t s) {
+    checksum_kernel<<<std::max(1, num_sms) * 8, 256, 0, s>>>(static_cast<const uint64_t*>(d), off / 8, bytes / 8, sum);
+    IPB_CK(cudaGetLastError());  // every section and chunk is a multiple of 8 bytes
+}
+
+uint64_t read_checksum(const unsigned long long* sum, cudaStream_t s) {
     unsigned long long h = 0;
-    IPB_CK(cudaMemcpyAsync(&h, scratch, sizeof h, cudaMemcpyDeviceToHost, s));
+    IPB_CK(cudaMemcpyAsync(&h, sum, sizeof h, cudaMemcpyDeviceToHost, s));
     IPB_CK(cudaStreamSynchronize(s));
     return h;
+}
+
+uint64_t device_checksum(const void* d, size_t bytes, unsigned long long* scratch, int num_sms, cudaStream_t s) {
+    IPB_CK(cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), s));
+    add_checksum(d, 0, bytes, scratch, num_sms, s);
+    return read_checksum(scratch, s);
+}
+
+// Bytes [off, off + n) of the D section between the resident tensors and
+// `file` (device memory, file order).
+void convert_d(const Precomp& P, size_t off, size_t n, uint8_t* file, bool to_file, cudaStream_t s) {
+    constexpr size_t kRow = 4096;
+    static_assert(kChunk % kRow == 0, "chunks hold whole rows");
+    IPB_CK(launch_dt_file_rows(P.pre_dt, P.pp.n_packed, off / kRow, n / kRow, file, to_file, P.tables, s));
 }
 
 // RAII holders for the host file, a pinned staging buffer, a stream.
@@ -173,9 +194,12 @@ void save(const Server& S, const char* path) {
     const Precomp& P = *S.pre;
     const Sections sec = sections_of(P);
     Stream st;
-    DevArena tmp;
+    struct Tmp : DevArena {
+        ~Tmp() { free_all(); }
+    } tmp;
     Header h{};
-    try {
+    uint8_t* const d_file = tmp.alloc<uint8_t>(std::min(kChunk, sec.bytes[kSecD]));  // one chunk in file order
+    {
         unsigned long long* scratch = tmp.alloc<unsigned long long>(1);
         std::memcpy(h.magic, kMagic, 8);
         h.version = kVersion;
@@ -186,12 +210,18 @@ void save(const Server& S, const char* path) {
         std::memcpy(h.seed, pp.seed, kSeedBytes);
         for (int k = 0; k < 4; ++k) {
             h.bytes[k] = sec.bytes[k];
-            h.sums[k] = device_checksum(sec.dev[k], sec.bytes[k], scratch, S.num_sms, st.s);
+            if (k != kSecD) {
+                h.sums[k] = device_checksum(sec.dev[k], sec.bytes[k], scratch, S.num_sms, st.s);
+                continue;
+            }
+            IPB_CK(cudaMemsetAsync(scratch, 0, sizeof *scratch, st.s));
+            for (size_t off = 0; off < sec.bytes[k]; off += kChunk) {
+                const size_t n = std::min(kChunk, sec.bytes[k] - off);
+                convert_d(P, off, n, d_file, true, st.s);
+                add_checksum(d_file, off, n, scratch, S.num_sms, st.s);
+            }
+            h.sums[k] = read_checksum(scratch, st.s);
         }
-        tmp.free_all();
-    } catch (...) {
-        tmp.free_all();
-        throw;
     }
     File f;
     f.f = std::fopen(path, "wb");
@@ -215,7 +245,12 @@ void save(const Server& S, const char* path) {
             const uint8_t* d = static_cast<const uint8_t*>(sec.dev[k]);
             for (size_t off = 0; off < sec.bytes[k]; off += kChunk, ++c) {
                 const size_t n = std::min(kChunk, sec.bytes[k] - off);
-                IPB_CK(cudaMemcpyAsync(buf[c & 1], d + off, n, cudaMemcpyDeviceToHost, st.s));
+                const uint8_t* from = d + off;
+                if (k == kSecD) {
+                    convert_d(P, off, n, d_file, true, st.s);
+                    from = d_file;
+                }
+                IPB_CK(cudaMemcpyAsync(buf[c & 1], from, n, cudaMemcpyDeviceToHost, st.s));
                 IPB_CK(cudaEventRecord(ev.e[c & 1], st.s));
                 if (c > 0) {
                     IPB_CK(cudaEventSynchronize(ev.e[(c - 1) & 1]));
@@ -282,6 +317,15 @@ Server* load(const char* path, size_t max_batch) {
     Stream st;
     alloc_precomp(*P, st.s);
     const Sections sec = sections_of(*P);
+    int num_sms = 0;
+    IPB_CK(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, P->device));
+    struct Tmp : DevArena {
+        ~Tmp() { free_all(); }
+    } tmp;
+    unsigned long long* const scratch = tmp.alloc<unsigned long long>(1);
+    unsigned long long* const d_sum = tmp.alloc<unsigned long long>(1);              // of the D section as read
+    uint8_t* const d_file = tmp.alloc<uint8_t>(std::min(kChunk, sec.bytes[kSecD]));  // one chunk in file order
+    IPB_CK(cudaMemsetAsync(d_sum, 0, sizeof *d_sum, st.s));
     {
         // Chunk c is read into staging buffer c % 2 while chunk c - 1
         // crosses PCIe from the other one.
@@ -300,25 +344,22 @@ Server* load(const char* path, size_t max_batch) {
                 if (!file_io(fd, buf[c & 1], n, fpos, false))
                     throw IoError(std::string("read failed (") + kSectionName[k] + ")");
                 fpos += (off_t)n;
-                IPB_CK(cudaMemcpyAsync(d + off, buf[c & 1], n, cudaMemcpyHostToDevice, st.s));
+                IPB_CK(cudaMemcpyAsync(k == kSecD ? d_file : d + off, buf[c & 1], n, cudaMemcpyHostToDevice, st.s));
                 IPB_CK(cudaEventRecord(ev.e[c & 1], st.s));
+                if (k == kSecD) {
+                    add_checksum(d_file, off, n, d_sum, num_sms, st.s);
+                    convert_d(*P, off, n, d_file, false, st.s);
+                }
             }
         }
         IPB_CK(cudaStreamSynchronize(st.s));
     }
-    int num_sms = 0;
-    IPB_CK(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, P->device));
-    DevArena tmp;
-    try {
-        unsigned long long* scratch = tmp.alloc<unsigned long long>(1);
-        for (int k = 0; k < 4; ++k)
-            if (device_checksum(sec.dev[k], sec.bytes[k], scratch, num_sms, st.s) != h.sums[k])
-                throw IoError(std::string("checkpoint checksum mismatch (") + kSectionName[k] + ")");
-        tmp.free_all();
-    } catch (...) {
-        tmp.free_all();
-        throw;
+    for (int k = 0; k < 4; ++k) {
+        const uint64_t sum = k == kSecD ? read_checksum(d_sum, st.s)
+                                        : device_checksum(sec.dev[k], sec.bytes[k], scratch, num_sms, st.s);
+        if (sum != h.sums[k]) throw IoError(std::string("checkpoint checksum mismatch (") + kSectionName[k] + ")");
     }
+    tmp.free_all();
     return make_server(pp, std::move(P), max_batch);
 }
 

@@ -72,8 +72,8 @@ struct LaneRun {
 
 // Cyclic shared scan (ipir_serve_config.scan_segments = ns > 1): a
 // database's DB and tensor passes run as ns segments in rotation on one lane
-// (segment k: DB columns [k C/ns, (k + 1) C/ns) and the tensor pass's
-// (limb, slot) indices [k 2N/ns, (k + 1) 2N/ns), all groups).  The requests
+// (segment k: DB columns [k C/ns, (k + 1) C/ns) and the k-th of ns equal
+// ranges of the tensor pass's tiles).  The requests
 // waiting when a segment is enqueued join the rotation there, as one group
 // of contiguous lane query slots; each segment's kernels serve every active
 // query at once (one read of that part of the DB and tensors), writing
@@ -104,7 +104,7 @@ struct ScanState {
     cudaEvent_t ev_seg_end = nullptr;
     cudaStream_t hst = nullptr;        // Horner chains and response copies
     bool stepped = false;
-    uint32_t* keys_pos = nullptr;      // keys of the active queries in pass order (lane arena)
+    uint8_t* kplanes_pos = nullptr;    // key planes of the active queries in pass order (lane arena)
     std::vector<cudaEvent_t> all_events;
     ~ScanState() {
         if (hst) cudaStreamSynchronize(hst);
@@ -328,7 +328,7 @@ void Engine::scan_step(DbState& d, std::unique_lock<std::mutex>& lk) {
             enqueue_qprep_slots(S, L, fresh->s0, fresh->k, r.st);
             fresh->issue_ns = Clock::now().time_since_epoch().count() - fresh->t_issue0;
         }
-        enqueue_scan_segment(S, L, sc.keys_pos, runs, seg, sc.ns, r.st, sc.ev_next);
+        enqueue_scan_segment(S, L, sc.kplanes_pos, runs, seg, sc.ns, r.st, sc.ev_next);
         if (!done.empty()) {
             for (auto& g : done) enqueue_scan_finalize(S, L, SlotRun{g.s0, g.k}, r.st);
             IPB_CK(cudaEventRecord(sc.ev_seg_end, r.st));
@@ -706,7 +706,7 @@ ipir_serve* ipir_serve_create(ipir_server* const* dbs, size_t n_dbs, const ipir_
             }
             // Cyclic scan for databases whose columns split into scan_segments
             // parts of whole 128-column tiles (the tensor pass splits its
-            // 2N (limb, slot) indices the same way, in multiples of 32).
+            // tiles, 128 per group, the same way).
             // scan_segments < 0: per database, from its own plain answer.
             auto splits = [](const ipb::Server& S, size_t ns) {
                 return ns > 1 && S.pp.db_cols % (128 * ns) == 0 && (2 * ipb::kN) % (32 * ns) == 0;
@@ -728,9 +728,9 @@ ipir_serve* ipir_serve_create(ipir_server* const* dbs, size_t n_dbs, const ipir_
                 for (auto& d : E->dbs) {
                     if (scan_ok(*d)) {
                         const size_t c = std::min<size_t>(b, 32);
-                        t += ipb::lane_bytes(*d->S, c, ipb::lane_gt_pass(*d->S, c)) + c * ipb::kKeyStride * 4;
+                        t += ipb::lane_bytes(*d->S, c) + c * ipb::kTpPlaneBytes;
                     } else {
-                        t += l * ipb::lane_bytes(*d->S, b, ipb::lane_gt_pass(*d->S, b));
+                        t += l * ipb::lane_bytes(*d->S, b);
                     }
                 }
                 return t;
@@ -757,7 +757,7 @@ ipir_serve* ipir_serve_create(ipir_server* const* dbs, size_t n_dbs, const ipir_
                     IPB_CK(cudaEventCreate(&r->ev_start));
                     IPB_CK(cudaEventCreate(&r->ev_end));
                     IPB_CK(cudaEventCreateWithFlags(&r->ev_db, cudaEventDisableTiming));
-                    ipb::alloc_lane(*d.S, r->lane, d.max_batch, ipb::lane_gt_pass(*d.S, d.max_batch));
+                    ipb::alloc_lane(*d.S, r->lane, d.max_batch, ipb::lane_gt_pass(d.max_batch));
                     d.lanes.push_back(std::move(r));
                 }
                 d.sched = !cfg.disable_autotune ? ipb::autotune(*d.S, d.lanes[0]->lane, d.lanes[0]->st)
@@ -767,7 +767,7 @@ ipir_serve* ipir_serve_create(ipir_server* const* dbs, size_t n_dbs, const ipir_
                     sc->ns = (int)d.scan_ns;
                     sc->cap = d.max_batch;
                     sc->used.assign(sc->cap, 0);
-                    sc->keys_pos = d.lanes[0]->lane.arena.alloc<uint32_t>(sc->cap * ipb::kKeyStride);
+                    sc->kplanes_pos = d.lanes[0]->lane.arena.alloc<uint8_t>(sc->cap * ipb::kTpPlaneBytes);
                     int lo = 0, hi = 0;
                     IPB_CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
                     IPB_CK(cudaStreamCreateWithPriority(&sc->hst, cudaStreamNonBlocking, hi));

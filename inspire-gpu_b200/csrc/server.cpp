@@ -180,7 +180,7 @@ static void preprocess_into(Precomp& P, const uint16_t* db_host, cudaStream_t s,
                 IPB_CK(launch_embed_gather(Tm, a_post + (g - w0) * ap_gstride, s));
             }
             IPB_CK(launch_collapse_a(a_post, ap_gstride, k5, P.tables, dp_w, dm_w, ends, nw, s));
-            IPB_CK(launch_dt_transpose(dp_w, dm_w, w0, nw, G, P.pre_dt, s));
+            IPB_CK(launch_dt_transpose(dp_w, dm_w, w0, nw, P.tables, P.pre_dt, s));
             IPB_CK(launch_collapse_final(ends, kn1, P.tables, P.pre_df + w0 * kGroupStrideF,
                                          P.pre_a + w0 * kGroupStrideA, nw, s));
         }
@@ -213,10 +213,10 @@ static int pick_pow2_chunks(size_t target, size_t maxv) {
     return (int)c;
 }
 
-size_t lane_bytes(const Server& S, size_t cap, int gt_pass) {
+size_t lane_bytes(const Server& S, size_t cap) {
     const size_t R = S.pp.db_rows, G = S.pp.n_packed;
     return cap * S.qstride * 8 + cap * kKeyStride * 4 + cap * kRgswStride * 4 + cap * S.mv_qstride * 4 +
-           tp_keyt_bytes(gt_pass) + (size_t)2 * kN * cap * G * 4 + cap * S.pb_qstride * 4 + cap * S.resp_qstride * 8 +
+           cap * kTpPlaneBytes + (size_t)2 * kN * cap * G * 4 + cap * S.pb_qstride * 4 + cap * S.resp_qstride * 8 +
            mv_tc_planes_bytes(R, (int)cap) + sizeof(int) + 2 * sizeof(unsigned) + cap * S.wire_q +
            cap * std::max(S.wire_r, S.wire_c) + cap * S.pp.num_cts * 4 * kN * 4;
 }
@@ -230,8 +230,8 @@ void alloc_lane(const Server& S, Lane& L, size_t cap, int gt_pass) {
     L.keys = A.alloc<uint32_t>(cap * kKeyStride);
     L.rgsw32 = A.alloc<uint32_t>(cap * kRgswStride);
     L.mvpart = A.alloc<uint32_t>(cap * S.mv_qstride);
-    L.keyt = A.alloc<uint32_t>(tp_keyt_bytes(gt_pass) / 4);
-    L.tp_out = A.alloc<uint32_t>((size_t)2 * kN * cap * G);
+    L.kplanes = A.alloc<uint8_t>(cap * kTpPlaneBytes);
+    L.tp_out = A.alloc<uint32_t>(cap * G * 2 * kN);
     L.packed_b = A.alloc<uint32_t>(cap * S.pb_qstride);
     L.resp = A.alloc<uint64_t>(cap * S.resp_qstride);
     L.planes = A.alloc<uint8_t>(mv_tc_planes_bytes(R, (int)cap));
@@ -282,7 +282,7 @@ Server* make_server(const Params& pp, std::shared_ptr<Precomp> pre, size_t max_b
     S->wire_q = wire_query_bytes(R);
     S->wire_r = wire_response_bytes(pp.num_cts);
     S->wire_c = wire_compressed_bytes(pp.num_cts);
-    const int gt_pass = lane_gt_pass(*S, max_batch);
+    const int gt_pass = lane_gt_pass(max_batch);
     S->sched = default_sched(*S, max_batch, gt_pass);
     alloc_lane(*S, S->lane, max_batch, gt_pass);
     S->ev.assign(6 * ((max_batch + kSliceQueries - 1) / kSliceQueries), nullptr);
@@ -376,9 +376,7 @@ void stage_parts(const Server& S, const ipir_query_view* qs, size_t count, int p
 
 const Sched& sched_for(const Server& S, size_t c) { return S.sched[std::min(c, S.sched.size() - 1)]; }
 
-int lane_gt_pass(const Server& S, size_t cap) {
-    return (int)std::min<size_t>(cap, (size_t)tp_pass_queries(S.pp.n_packed));
-}
+int lane_gt_pass(size_t cap) { return (int)std::min<size_t>(cap, (size_t)kTpMaxQueries); }
 
 static bool chunked_ok(const Server& S, const Sched& sc, size_t count);
 
@@ -417,8 +415,7 @@ std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
 // (query prep, tensor pass) then runs first and the mat-vec after the event.
 // The RGSW parts are then prepared on that other stream as well.
 // q_off: the batch's first lane slot (slices of a batch larger than one DB
-// pass run the whole phase on slots [q_off, q_off + count)); the tensor-pass
-// rows (tp_out) and key table are shared by slices run one after the other.
+// pass run the whole phase on slots [q_off, q_off + count)).
 // qprep_parts: 3 prepares keys and RGSW parts here, 1 the keys only (the
 // RGSW parts are prepared elsewhere).
 int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t count, cudaStream_t st,
@@ -433,8 +430,10 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
     uint8_t* const planes = L.planes + mv_tc_planes_offset(q_off, R);
     int launches = 0;
     if (ev) IPB_CK(cudaEventRecord(ev[0], st));
-    IPB_CK(launch_qprep_parts(qraw, S.qstride, R, P.tables, keys, L.rgsw32 + q_off * kRgswStride, nq, qprep_parts,
-                              st));
+    uint8_t* const kplanes = L.kplanes + q_off * kTpPlaneBytes;
+    uint32_t* const tp_out = L.tp_out + q_off * S.pb_qstride;
+    IPB_CK(launch_qprep_parts(qraw, S.qstride, R, P.tables, kplanes, keys, L.rgsw32 + q_off * kRgswStride, nq,
+                              qprep_parts, st));
     ++launches;
     if (ev) IPB_CK(cudaEventRecord(ev[1], st));
     // Beside: the tensor pass (keys only) on sc.tp_sms SMs from the lane's
@@ -444,9 +443,9 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
     auto tensor_pass = [&](cudaStream_t ts, int sms) {
         for (size_t c0 = 0; c0 < count; c0 += (size_t)sc.tp_pass) {
             const int n = (int)std::min<size_t>((size_t)sc.tp_pass, count - c0);
-            IPB_CK(launch_tensor_pass(P.pre_dt, G, keys + c0 * kKeyStride, kKeyStride, n, nq, (int)c0, L.keyt,
-                                      L.tp_out, L.d_err, L.tiles + 1, sms, ts));
-            launches += 2;  // key table + GEMM
+            IPB_CK(launch_tensor_pass(P.pre_dt, 0, tp_tiles(G), kplanes + c0 * kTpPlaneBytes, n, nullptr,
+                                      tp_out + c0 * S.pb_qstride, S.pb_qstride, L.d_err, L.tiles + 1, sms, ts));
+            ++launches;
         }
     };
     if (beside) {
@@ -485,7 +484,7 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
     if (ev) IPB_CK(cudaEventRecord(ev[2], st));
     if (!beside && !lwe_ready) tensor_pass(st, S.num_sms);
     if (ev) IPB_CK(cudaEventRecord(ev[3], st));
-    IPB_CK(launch_finalize(mvpart, S.mv_qstride, mv_parts, C, L.tp_out, P.pre_df, keys, kKeyStride, P.tables,
+    IPB_CK(launch_finalize(mvpart, S.mv_qstride, mv_parts, C, tp_out, P.pre_df, keys, kKeyStride, P.tables,
                            L.packed_b + q_off * S.pb_qstride, S.pb_qstride, G, nq, st));
     return launches + 1;
 }
@@ -615,13 +614,13 @@ static int run_chunked(const Server& S, Lane& L, const Sched& sc, size_t count, 
     const size_t R = pp.db_rows, C = pp.db_cols, G = pp.n_packed;
     const int nq = (int)count;
     int launches = 0;
-    IPB_CK(launch_qprep_parts(L.qraw, S.qstride, R, P.tables, L.keys, L.rgsw32, nq, qprep_parts, st));
+    IPB_CK(launch_qprep_parts(L.qraw, S.qstride, R, P.tables, L.kplanes, L.keys, L.rgsw32, nq, qprep_parts, st));
     ++launches;
     for (size_t c0 = 0; c0 < count; c0 += (size_t)sc.tp_pass) {
         const int n = (int)std::min<size_t>((size_t)sc.tp_pass, count - c0);
-        IPB_CK(launch_tensor_pass(P.pre_dt, G, L.keys + c0 * kKeyStride, kKeyStride, n, nq, (int)c0, L.keyt,
-                                  L.tp_out, L.d_err, L.tiles + 1, S.num_sms, st));
-        launches += 2;
+        IPB_CK(launch_tensor_pass(P.pre_dt, 0, tp_tiles(G), L.kplanes + c0 * kTpPlaneBytes, n, nullptr,
+                                  L.tp_out + c0 * S.pb_qstride, S.pb_qstride, L.d_err, L.tiles + 1, S.num_sms, st));
+        ++launches;
     }
     if (lwe_ready) IPB_CK(cudaStreamWaitEvent(st, lwe_ready, 0));
     IPB_CK(launch_qplanes(L.qraw, S.qstride, R, P.tables, L.planes, nq, st));
@@ -644,7 +643,7 @@ static int run_chunked(const Server& S, Lane& L, const Sched& sc, size_t count, 
                                        P.tables, L.mvpart, S.mv_qstride, nullptr, L.d_err, L.tiles, S.num_sms,
                                        S.tc_kchunk_rows, st));
         for (size_t t = 0; t < nct; ++t) {
-            IPB_CK(launch_finalize_range(L.mvpart, S.mv_qstride, S.tc_kchunks, C, L.tp_out, nq, 0, P.pre_df, L.keys,
+            IPB_CK(launch_finalize_range(L.mvpart, S.mv_qstride, S.tc_kchunks, C, L.tp_out, P.pre_df, L.keys,
                                          kKeyStride, P.tables, L.packed_b, S.pb_qstride, G, t * d_act + lo, hi - lo,
                                          nq, st));
             ++launches;
@@ -687,11 +686,12 @@ void enqueue_horner(const Server& S, const Sched& sc, const uint32_t* packed_b, 
 }
 
 void enqueue_qprep_slots(const Server& S, Lane& L, size_t s0, size_t count, cudaStream_t st) {
-    IPB_CK(launch_qprep(L.qraw + s0 * S.qstride, S.qstride, S.pp.db_rows, S.pre->tables, L.keys + s0 * kKeyStride,
-                        L.rgsw32 + s0 * kRgswStride, (int)count, st));
+    IPB_CK(launch_qprep(L.qraw + s0 * S.qstride, S.qstride, S.pp.db_rows, S.pre->tables,
+                        L.kplanes + s0 * kTpPlaneBytes, L.keys + s0 * kKeyStride, L.rgsw32 + s0 * kRgswStride,
+                        (int)count, st));
 }
 
-void enqueue_scan_segment(const Server& S, Lane& L, uint32_t* keys_pos, const std::vector<SlotRun>& runs, int seg,
+void enqueue_scan_segment(const Server& S, Lane& L, uint8_t* kplanes_pos, const std::vector<SlotRun>& runs, int seg,
                           int ns, cudaStream_t st, cudaEvent_t after_matvec) {
     const Params& pp = S.pp;
     const Precomp& P = *S.pre;
@@ -700,11 +700,11 @@ void enqueue_scan_segment(const Server& S, Lane& L, uint32_t* keys_pos, const st
     size_t n = 0;
     for (const SlotRun& r : runs) {
         if (n + r.k > 32 || r.s0 + r.k > L.cap) throw std::invalid_argument("scan segment: 1..32 queries per pass");
-        // positions n .. n + k - 1 of this segment's pass: query planes and keys
+        // positions n .. n + k - 1 of this segment's pass: query and key planes
         IPB_CK(launch_qplanes(L.qraw + r.s0 * S.qstride, S.qstride, R, P.tables, L.planes + mv_tc_planes_offset(n, R),
                               (int)r.k, st));
-        IPB_CK(cudaMemcpyAsync(keys_pos + n * kKeyStride, L.keys + r.s0 * kKeyStride, r.k * kKeyStride * 4,
-                               cudaMemcpyDeviceToDevice, st));
+        IPB_CK(cudaMemcpyAsync(kplanes_pos + n * kTpPlaneBytes, L.kplanes + r.s0 * kTpPlaneBytes,
+                               r.k * kTpPlaneBytes, cudaMemcpyDeviceToDevice, st));
         for (size_t i = 0; i < r.k; ++i) qmap[n + i] = (uint8_t)(r.s0 + i);
         n += r.k;
     }
@@ -714,12 +714,11 @@ void enqueue_scan_segment(const Server& S, Lane& L, uint32_t* keys_pos, const st
     IPB_CK(launch_matvec_tc_range(P.db, R, C, c0, c1, L.planes, (int)n, P.tables, L.mvpart, S.mv_qstride, qmap,
                                   L.d_err, L.tiles, S.num_sms, S.tc_kchunk_rows, st));
     if (after_matvec) IPB_CK(cudaEventRecord(after_matvec, st));
-    const int n_li = (int)(2 * kN) / ns, li0 = n_li * seg;
+    const int n_tiles = tp_tiles(G) / ns;  // 128 tiles per group, ns a power of two <= 128
     for (size_t q0 = 0; q0 < n; q0 += (size_t)L.gt_pass) {
         const int k = (int)std::min<size_t>((size_t)L.gt_pass, n - q0);
-        IPB_CK(launch_tensor_pass_slots(P.pre_dt, G, li0, n_li, keys_pos + q0 * kKeyStride, kKeyStride, k,
-                                        (int)L.cap, (int)q0, qmap, L.keyt, L.tp_out, L.d_err, L.tiles + 1, S.num_sms,
-                                        st));
+        IPB_CK(launch_tensor_pass(P.pre_dt, n_tiles * seg, n_tiles, kplanes_pos + q0 * kTpPlaneBytes, k, qmap + q0,
+                                  L.tp_out, S.pb_qstride, L.d_err, L.tiles + 1, S.num_sms, st));
     }
 }
 
@@ -727,8 +726,9 @@ void enqueue_scan_finalize(const Server& S, Lane& L, const SlotRun& r, cudaStrea
     const Params& pp = S.pp;
     const Precomp& P = *S.pre;
     const size_t C = pp.db_cols, G = pp.n_packed;
-    IPB_CK(launch_finalize_range(L.mvpart + r.s0 * S.mv_qstride, S.mv_qstride, S.tc_kchunks, C, L.tp_out, (int)L.cap,
-                                 (int)r.s0, P.pre_df, L.keys + r.s0 * kKeyStride, kKeyStride, P.tables,
+    IPB_CK(launch_finalize_range(L.mvpart + r.s0 * S.mv_qstride, S.mv_qstride, S.tc_kchunks, C,
+                                 L.tp_out + r.s0 * S.pb_qstride, P.pre_df, L.keys + r.s0 * kKeyStride, kKeyStride,
+                                 P.tables,
                                  L.packed_b + r.s0 * S.pb_qstride, S.pb_qstride, G, 0, G, (int)r.k, st));
 }
 
@@ -795,8 +795,8 @@ static void stage_and_run(Server* S, const ipir_query_view* qs, size_t count) {
     stage_parts(*S, qs, count, 0, 2, L.aux);      // LWE vectors: needed by the mat-vec
     IPB_CK(cudaEventRecord(L.join, L.aux));
     stage_parts(*S, qs, count, 4, 1, L.aux);      // RGSW parts: needed by the Horner chains
-    IPB_CK(launch_qprep_parts(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, L.keys, L.rgsw32, (int)count, 2,
-                              L.aux));
+    IPB_CK(launch_qprep_parts(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, L.kplanes, L.keys, L.rgsw32,
+                              (int)count, 2, L.aux));
     IPB_CK(cudaEventRecord(L.rgsw_ready, L.aux));
     S->staged = count;
     S->launches += 1;
@@ -1433,7 +1433,7 @@ int ipir_b200_export_precomp(const ipir_server* srv, size_t group, uint32_t* a, 
                 try {
                     uint32_t* tp = tmp.alloc<uint32_t>(ipb::kGroupStrideD);
                     uint32_t* tm = tmp.alloc<uint32_t>(ipb::kGroupStrideD);
-                    IPB_CK(ipb::launch_dt_export(P.pre_dt, group, S->pp.n_packed, tp, tm, 0));
+                    IPB_CK(ipb::launch_dt_export(P.pre_dt, group, P.tables, tp, tm, 0));
                     IPB_CK(cudaDeviceSynchronize());
                     if (d_plus) IPB_CK(cudaMemcpy(d_plus, tp, ipb::kGroupStrideD * 4, cudaMemcpyDeviceToHost));
                     if (d_minus) IPB_CK(cudaMemcpy(d_minus, tm, ipb::kGroupStrideD * 4, cudaMemcpyDeviceToHost));

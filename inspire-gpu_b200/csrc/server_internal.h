@@ -72,7 +72,7 @@ constexpr size_t kGroupStrideD = (size_t)2 * kSteps * kDeff * kN;  // u32 per gr
 constexpr size_t kGroupStrideF = (size_t)2 * kDeff * kN;
 constexpr size_t kGroupStrideA = (size_t)2 * kN;
 constexpr size_t kBlk = (size_t)kDeff * 2 * kN;                    // one KSK / RGSW part
-constexpr size_t kKeyStride = 4 * kDeff * kN;                      // keys per query (u32)
+constexpr size_t kKeyStride = 2 * kDeff * kN;                      // KSK-1 per query (u32)
 constexpr size_t kRgswStride = 4 * kBlk;                           // rgsw32 per query (u32)
 
 const DevTables& host_tables();
@@ -86,7 +86,7 @@ struct Precomp {
     DevTables* tables = nullptr;
     uint16_t* db = nullptr;
     uint32_t* pre_a = nullptr;
-    uint8_t* pre_dt = nullptr;  // D_plus / D_minus as GEMM byte planes [l][i][g*4+a][4096]
+    uint8_t* pre_dt = nullptr;  // D_plus / D_minus as GEMM byte planes (tensorpass_tc.cu)
     uint32_t* pre_df = nullptr;
     bool adopted = false;
     ~Precomp() {
@@ -100,7 +100,7 @@ struct Precomp {
 // Kernel choices for one batch size.
 struct Sched {
     int matvec_tc = 1;       // 1: tcgen05 int8 mat-vec, 0: CUDA-core mat-vec
-    int tp_pass = 32;        // queries per tensor-pass GEMM (<= the lane's Gt capacity)
+    int tp_pass = 32;        // queries per tensor-pass GEMM (<= the lane's gt_pass)
     int horner_cluster = 1;  // 1: 4-CTA cluster per chain, 2: 8-CTA cluster, 0: one CTA per chain
     int tp_sms = 0;          // > 0: tensor pass on this many SMs beside the tcgen05 mat-vec on the
                              // others (the lane's second stream); 0: tensor pass after the mat-vec
@@ -125,13 +125,13 @@ inline size_t slices_of(size_t c, const Sched& sc) {
 struct Lane {
     DevArena arena;
     size_t cap = 0;
-    int gt_pass = 0;  // queries per tensor pass the key-table buffer holds
+    int gt_pass = 0;  // most queries per tensor-pass GEMM
     uint64_t* qraw = nullptr;
     uint32_t* keys = nullptr;
     uint32_t* rgsw32 = nullptr;
     uint32_t* mvpart = nullptr;
-    uint32_t* keyt = nullptr;    // per-pass key table the tensor-pass GEMM gathers its N operand from
-    uint32_t* tp_out = nullptr;  // tensor-pass result [l][i][q][g]
+    uint8_t* kplanes = nullptr;  // KSK5 byte planes, the tensor-pass GEMM's N operand
+    uint32_t* tp_out = nullptr;  // tensor-pass result [q][g][l][N]
     uint32_t* packed_b = nullptr;
     uint64_t* resp = nullptr;
     uint8_t* planes = nullptr;   // query byte planes for the tensor-core mat-vec
@@ -187,8 +187,8 @@ struct Server {
     ~Server();
 };
 
-// Bytes of a lane of `cap` queries whose Gt holds `gt_pass` queries.
-size_t lane_bytes(const Server& S, size_t cap, int gt_pass);
+// Bytes of a lane of `cap` queries.
+size_t lane_bytes(const Server& S, size_t cap);
 void alloc_lane(const Server& S, Lane& L, size_t cap, int gt_pass);
 // Device buffers of a server's resident state (tables, DB, a, D byte planes,
 // D_final) for P.pp, on P.device.
@@ -243,14 +243,14 @@ std::shared_ptr<Precomp> run_preprocess_shard(const Params& global, const uint16
 // H2D of one flat query into query slot i of lane L.
 void stage_query_flat(const Server& S, Lane& L, size_t i, const uint64_t* flat, cudaStream_t st);
 // Schedule table (index = batch size, 0 unused) for a lane of `cap` queries
-// whose Gt holds gt_pass: the handle's defaults (env overrides included).
+// with gt_pass per tensor pass: the handle's defaults (env overrides included).
 std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass);
 // Measures candidate schedules per batch size on lane L; returns the table.
 std::vector<Sched> autotune(const Server& S, Lane& L, cudaStream_t st);
 // Sched for batch size c of the handle's own table.
 const Sched& sched_for(const Server& S, size_t c);
-// Queries per tensor-pass GEMM a lane of `cap` queries provisions Gt for.
-int lane_gt_pass(const Server& S, size_t cap);
+// Most queries per tensor-pass GEMM of a lane of `cap` queries.
+int lane_gt_pass(size_t cap);
 
 // Horner chains (variant sc.horner_cluster) of `count` queries whose
 // packed ciphertexts, RGSW parts and responses start at the given pointers
@@ -266,11 +266,11 @@ struct SlotRun {
 // One segment (seg of ns) of the cyclic scan for the queries in `runs`
 // (their positions in this pass follow the order of runs): the tensor-core
 // mat-vec over DB columns [seg C/ns, (seg + 1) C/ns) and the tensor pass
-// over the (limb, slot) indices [seg 2N/ns, (seg + 1) 2N/ns), all groups,
-// writing each query's mat-vec partials and tensor-pass rows under its own
-// lane slot.  keys_pos: scratch for the keys in pass order (<= 32 queries).
+// over the seg-th of ns equal ranges of its tiles, writing each query's
+// mat-vec partials and tensor-pass rows under its own lane slot.
+// kplanes_pos: scratch for the key planes in pass order (<= 32 queries).
 // after_matvec (may be null) is recorded once the mat-vec is enqueued.
-void enqueue_scan_segment(const Server& S, Lane& L, uint32_t* keys_pos, const std::vector<SlotRun>& runs, int seg,
+void enqueue_scan_segment(const Server& S, Lane& L, uint8_t* kplanes_pos, const std::vector<SlotRun>& runs, int seg,
                           int ns, cudaStream_t st, cudaEvent_t after_matvec);
 // Finalize (all groups) of lane slots r after their ns segments: packed
 // ciphertexts from the slots' mat-vec partials and tensor-pass rows.

@@ -198,8 +198,8 @@ int ipir_b200_horner_answer(ipir_horner* h, const uint32_t* packed_b, const ipir
         IPB_CK(cudaEventRecord(L.fork, static_cast<cudaStream_t>(stream)));
         IPB_CK(cudaStreamWaitEvent(S->stream, L.fork, 0));
         ipb::stage_parts(*S, queries, count, 4, 1, S->stream);  // RGSW parts only
-        IPB_CK(launch_qprep_parts(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, L.keys, L.rgsw32, (int)count,
-                                  2, S->stream));
+        IPB_CK(launch_qprep_parts(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, L.kplanes, L.keys, L.rgsw32,
+                                  (int)count, 2, S->stream));
         const size_t ns = ipb::slices_of(count, sc), slice = sc.slice > 0 ? (size_t)sc.slice : count;
         for (size_t k = 0; k < ns; ++k) {
             const size_t q0 = k * slice, n = std::min(slice, count - q0);

@@ -1,38 +1,39 @@
-// tensorpass_tc.cu -- the online tensor pass (InspiRINGOnline) as int8
-// tcgen05 GEMMs.
+// tensorpass_tc.cu -- the online tensor pass (InspiRINGOnline) as one int8
+// tcgen05 GEMM per limb.
 //
 // For group g, limb l and NTT slot i the reference subtracts
-//   T_g[l][i] = sum_{dir, s, j} D_g[dir][l][s][j][i] * K5[l][j][perm_{t(dir,s)}(i)]
-// (src/gpu_online.cu:593-714, permutations of src/gpu_protocol.cu:169-215),
-// re-reading and re-permuting the query key for every group.  Index the sum
-// by u = (dir*1023 + s)*2 + j < 4092 (padded to 4096).  The permuted key
-//   Gq[l][i][u] = K5_q[l][j][perm_{t(dir,s)}(i)]
-// does not depend on the group, so per (l, i) the pass over all groups and
-// all queries of a batch is one GEMM
-//   T[g][q] = sum_u D[g][u] * Gq[u],   M = groups, N = queries, K = 4096.
-// Both operands are < 2^27: split each into four bytes, put D's planes in M
-// (row g*4 + a) and Gq's planes in N (column q*4 + b); tcgen05.mma.kind::i8
+//   T_g[l][i] = sum_{dir, s, j} D_g[dir][l][s][j][i] * K5[l][j][perm_{t(dir,s)}(i)],
+// t(dir, s) = +-5^(1022-s) (src/gpu_online.cu:593-714, permutations of
+// src/gpu_protocol.cu:169-215), re-reading and re-permuting the query key for
+// every group.
+//
+// Slot i is the evaluation at psi^odd, odd = 2 BR(i) + 1 = sigma 5^k mod 2N
+// (sigma = +-1; 5 generates the residues = 1 mod 4), and perm_t(i) is the slot
+// of t * odd = +-sigma 5^(k + 1022 - s).  So the terms of slot i meet the
+// key's slots in one fixed order, whatever i is, once D is indexed by the key
+// position instead of the step: with rho = dir xor (sigma < 0) and
+// m = (k + 1022 - s) mod 1024, u = j * 2048 + rho * 1024 + m and
+//   D'_g[l][i][u] = D_g[dir][l][s][j][i]     (0 where s would be 1023),
+//   K'[l][u]      = K5[l][j][slot of (-1)^rho 5^m],
+//   T_g[l][i]     = sum_u D'_g[l][i][u] * K'[l][u].
+// K' depends on neither the slot nor the group: per limb the pass over all
+// groups, slots and queries is one GEMM, M = (group, slot), N = queries,
+// K = 4096, whose N operand is 16 KB per query and limb.  (With D in step
+// order every slot needed its own permuted key, gathered from L2 by the
+// kernel: 67 MB per query, which bounded the pass at few groups.)
+//
+// Both operands are < 2^27: split each into four bytes, D's planes in M (row
+// 4 i + a) and K's planes in N (column 4 q + b); tcgen05.mma.kind::i8
 // accumulates sum_u over bytes exactly in s32 (255^2 * 4096 < 2^31), and the
-// epilogue forms sum_{a,b} (256^(a+b) mod q_l) * P[g*4+a][q*4+b] < 2^59 and
-// reduces mod q_l.  Exact, so equal to the reference.
+// epilogue forms sum_{a,b} (256^(a+b) mod q_l) * P[4 i + a][4 q + b] < 2^59
+// and reduces mod q_l.  Exact, so equal to the reference.
 //
-// Layouts: Dt[l][i][g*4 + a][u] u8 (built once at preprocess by
-// dt_transpose_kernel) is the A operand, loaded by TMA.  The B operand, the
-// byte planes Gq[l][i][q*4 + b][u], is never stored: per pass keyt_kernel
-// writes the compact key table Kt[l][j][p][q] (u32, queries innermost,
-// <= 1 MB, stays in L2) and the GEMM's key warps gather from it straight
-// into each stage's swizzled B tile.  Output tp_out[l][i][q][g] (u32,
-// reduced).
-//
-// The GEMM kernel is persistent with dynamic work items: the producer takes
-// the next item from a per-launch atomic counter and publishes it to the MMA
-// thread, the key warps and the epilogue through a ring of shared slots
-// (-1 ends it), so SMs held by other kernels at launch take fewer items.
-// Warp roles (768 threads): 0 TMA producer (one thread), 1 TMEM allocation
-// and MMA issue (one thread), 4..7 epilogue, 8..23 key planes in four
-// groups of 128 threads, group g filling the K tiles kt = g mod 4, so four
-// stages' gathers are in flight at once.  With fewer stages than groups the
-// groups that fill none join the epilogue.
+// Layouts.  D' is stored as the kernel reads it: tile t = (2 g + l) * 64 +
+// i / 32 holds the 128 rows of 32 slots, as 32 K blocks of 128 rows x 128
+// bytes (16 KB), rows already in the SWIZZLE_128B pattern.  A block is one
+// contiguous bulk copy, and the pass streams the tensors in address order.
+// K' planes: kplanes[q][l][b][4096] u8, written by the query prep.  Output:
+// tp_out[q][g][l][N] u32, reduced.
 #include <cuda.h>
 
 #include <algorithm>
@@ -47,118 +48,124 @@ namespace ipb {
 namespace {
 using namespace tc;
 
-constexpr int kUPad = 4096;       // u range, 4092 used
-constexpr int kRing = 8;          // published work items in flight
-constexpr int kKeyGroups = 4;
-constexpr int kKeyGroup = 128;    // threads per key group
-constexpr int kKeyThreads = kKeyGroups * kKeyGroup;  // warps 8..23
-constexpr int kTpThreads = 256 + kKeyThreads;
-constexpr int kUsed = 2 * 2 * kSteps;
+constexpr int kK = 4096;                // u range
+constexpr int kKBlock = 128;            // bytes of K per stage
+constexpr int kKTiles = kK / kKBlock;
+constexpr uint32_t kTile = 128 * 128;   // bytes of one 128-row K block
+constexpr int kTilesPerPoly = kN / 32;  // 128-row tiles of one (group, limb)
+constexpr int kRing = 8;                // published work items in flight
+constexpr int kEpiWarps = 8;
+constexpr int kTpThreads = 64 + 32 * kEpiWarps;
 
-__device__ __forceinline__ uint32_t pow5_mod2n(uint32_t e) {
-    uint32_t r = 1, b = 5;
-    while (e) {
-        if (e & 1) r = (r * b) & (2 * kN - 1);
-        b = (b * b) & (2 * kN - 1);
-        e >>= 1;
-    }
-    return r;
+// Byte (row 4 i + a, position u) of group-limb gl = 2 g + l.
+__device__ __forceinline__ size_t dt_addr(size_t gl, uint32_t i, uint32_t a, uint32_t u) {
+    const uint32_t r = (i & 31) * 4 + a;
+    return ((gl * kTilesPerPoly + (i >> 5)) * kKTiles + (u >> 7)) * kTile + r * 128 +
+           ((((u >> 4) ^ r) & 7) << 4) + (u & 15);
 }
+// Step of slot exponent k at key exponent m (1023: no such step).
+__device__ __forceinline__ uint32_t dt_step(uint32_t k, uint32_t m) { return (k + kHalf - 2 - m) & (kHalf - 1); }
 
 // ------------------------------------------------------------------ D re-layout
 // Source: one wave of groups in the reference layout [l][s][j][N] (u32) for
-// each direction; destination Dt rows g*4 + a.  Tile 32 u x 32 slots.
+// each direction.  CTA: 8 slots x all steps of one (direction, digit), read a
+// 32-byte sector per step, written as whole 128-byte rows of the K blocks.
+constexpr int kTrStride = kHalf + 4;  // tile row stride: the 8 slots of a step land in distinct banks
 __global__ void __launch_bounds__(256) dt_transpose_kernel(const uint32_t* __restrict__ dp,
-                                                           const uint32_t* __restrict__ dm, size_t g0, size_t G,
-                                                           uint8_t* __restrict__ Dt) {
-    __shared__ uint32_t tile[32][33];
-    const int ut = blockIdx.x, it = blockIdx.y;
+                                                           const uint32_t* __restrict__ dm, size_t g0,
+                                                           const DevTables* __restrict__ T, uint8_t* __restrict__ Dt) {
+    __shared__ uint32_t tile[8 * kTrStride];
+    const uint32_t i0 = blockIdx.x * 8;
+    const int dir = blockIdx.y >> 1, j = blockIdx.y & 1;
     const int gw = blockIdx.z >> 1, l = blockIdx.z & 1;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const size_t gstride = (size_t)2 * kSteps * kDeff * kN;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int r = ty + 8 * k;
-        const int u = ut * 32 + r;
-        uint32_t v = 0;
-        if (u < kUsed) {
-            const int w = u >> 1, j = u & 1;
-            const int dir = w >= kSteps;
-            const int s = w - dir * kSteps;
-            v = (dir ? dm : dp)[(size_t)gw * gstride + ((size_t)(l * kSteps + s) * kDeff + j) * kN + it * 32 + tx];
-        }
-        tile[r][tx] = v;
-    }
+    const uint32_t t = threadIdx.x;
+    const uint32_t* src = (dir ? dm : dp) + (size_t)gw * (2 * (size_t)kSteps * kDeff * kN) +
+                          ((size_t)l * kSteps * kDeff + j) * kN + i0 + (t & 7);
+    for (uint32_t s = t >> 3; s < (uint32_t)kHalf; s += 32)
+        tile[(t & 7) * kTrStride + s] = s < (uint32_t)kSteps ? src[(size_t)s * kDeff * kN] : 0u;
     __syncthreads();
-    const size_t g = g0 + gw;
+    const size_t gl = (g0 + gw) * 2 + l;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int op = threadIdx.x + 256 * k;
-        const int il = op >> 5, rem = op & 31;
-        const int a = rem >> 3, c = rem & 7;
-        uint32_t word = 0;
+    for (uint32_t x = 0; x < 8; ++x) {
+        const uint32_t i = i0 + x, ex = T->exp_of[i];
+        const uint32_t k = ex & (kHalf - 1), rho = (uint32_t)dir ^ (ex >> 10);
+        uint32_t v[4];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) word |= ((tile[4 * c + m][il] >> (8 * a)) & 0xFFu) << (8 * m);
-        const size_t row = ((size_t)(l * kN + it * 32 + il)) * 4 * G + g * 4 + a;
-        *reinterpret_cast<uint32_t*>(Dt + row * kUPad + ut * 32 + 4 * c) = word;
+        for (uint32_t e = 0; e < 4; ++e) v[e] = tile[x * kTrStride + dt_step(k, 4 * t + e)];
+#pragma unroll
+        for (uint32_t a = 0; a < 4; ++a) {
+            uint32_t w = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w |= ((v[e] >> (8 * a)) & 0xFFu) << (8 * e);
+            *reinterpret_cast<uint32_t*>(Dt + dt_addr(gl, i, a, j * kN + rho * kHalf + 4 * t)) = w;
+        }
     }
 }
 
 // Inverse of the re-layout for one group (precomp export): [l][s][j][N] u32.
-__global__ void __launch_bounds__(256) dt_export_kernel(const uint8_t* __restrict__ Dt, size_t g, size_t G,
-                                                        uint32_t* __restrict__ dp, uint32_t* __restrict__ dm) {
+__global__ void __launch_bounds__(256) dt_export_kernel(const uint8_t* __restrict__ Dt, size_t g,
+                                                        const DevTables* __restrict__ T, uint32_t* __restrict__ dp,
+                                                        uint32_t* __restrict__ dm) {
     const size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x;  // over l, i, u
-    if (idx >= (size_t)2 * kN * kUsed) return;
-    const int u = (int)(idx % kUsed);
-    const size_t li = idx / kUsed;
-    const int l = (int)(li / kN), i = (int)(li % kN);
-    const uint8_t* src = Dt + (li * 4 * G + g * 4) * kUPad + u;
-    const uint32_t v = (uint32_t)src[0] | ((uint32_t)src[kUPad] << 8) | ((uint32_t)src[2 * kUPad] << 16) |
-                       ((uint32_t)src[3 * kUPad] << 24);
-    const int w = u >> 1, j = u & 1;
-    const int dir = w >= kSteps;
-    const int s = w - dir * kSteps;
-    (dir ? dm : dp)[((size_t)(l * kSteps + s) * kDeff + j) * kN + i] = v;
-}
-
-// ------------------------------------------------------------------ key table
-// Kt[l][j][p][qq] = K5_q[l][j][p] (key 0 of query qq of the pass, NTT form)
-// for qq < nq, zero for nq <= qq < W, W = 8 ceil(nq / 8): the W values of one
-// position fill whole 32-byte sectors.
-__global__ void __launch_bounds__(256) keyt_kernel(const uint32_t* __restrict__ keys, size_t key_qstride, int nq,
-                                                   int W, uint32_t* __restrict__ Kt) {
-    const size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x;  // over ((l*kDeff + j)*kN + p)*W + qq
-    if (idx >= (size_t)2 * kDeff * kN * W) return;
-    const int qq = (int)(idx % (size_t)W);
-    const size_t ljp = idx / (size_t)W;
+    const uint32_t u = (uint32_t)(idx % kK), i = (uint32_t)(idx / kK % kN), l = (uint32_t)(idx / kK / kN);
+    const uint32_t ex = T->exp_of[i], j = u >> 11, rho = (u >> 10) & 1;
+    const uint32_t s = dt_step(ex & (kHalf - 1), u & (kHalf - 1));
+    if (s >= (uint32_t)kSteps) return;
     uint32_t v = 0;
-    if (qq < nq) v = keys[(size_t)qq * key_qstride + ljp];  // keys[q][key 0][l][j][p]
-    Kt[idx] = v;
+#pragma unroll
+    for (uint32_t a = 0; a < 4; ++a) v |= (uint32_t)Dt[dt_addr(g * 2 + l, i, a, u)] << (8 * a);
+    ((rho ^ (ex >> 10)) ? dm : dp)[(((size_t)l * kSteps + s) * kDeff + j) * kN + i] = v;
 }
 
-// One 32-byte sector (8 queries' key words) in a single 256-bit load.
-__device__ __forceinline__ void ld_sector(const uint32_t* p, uint32_t (&v)[8]) {
-    asm volatile("ld.global.nc.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                 : "l"(p));
-}
-// 32-bit store into a K-major SWIZZLE_128B tile (1024-byte aligned base):
-// row r's 16-byte chunk c sits at chunk c ^ (r & 7).
-__device__ __forceinline__ void st_sw128(uint8_t* tile, uint32_t row, uint32_t col, uint32_t w) {
-    *reinterpret_cast<uint32_t*>(tile + row * 128 + ((((col >> 4) ^ (row & 7)) & 7) << 4) + (col & 15)) = w;
+// Rows [row0, row0 + gridDim.x) of the checkpoint files' order of the same
+// bytes: row ((l * N + i) * G + g) * 4 + a, positions (dir * 1023 + s) * 2 + j
+// (4092 used, the last four zero).  One CTA copies one row to or from the
+// resident layout.
+template <bool kToFile>
+__global__ void __launch_bounds__(256) dt_file_rows_kernel(uint8_t* __restrict__ Dt, size_t G, size_t row0,
+                                                           uint8_t* __restrict__ file,
+                                                           const DevTables* __restrict__ T) {
+    __shared__ __align__(16) uint8_t row[kK];
+    const size_t fr = row0 + blockIdx.x;
+    const uint32_t a = (uint32_t)(fr & 3);
+    const size_t g = (fr >> 2) % G, li = (fr >> 2) / G;
+    const uint32_t i = (uint32_t)(li % kN), l = (uint32_t)(li / kN);
+    const uint32_t t = threadIdx.x, ex = T->exp_of[i], k = ex & (kHalf - 1), neg = ex >> 10;
+    uint8_t* frow = file + (size_t)blockIdx.x * kK + 16 * t;
+    uint8_t* drow = Dt + dt_addr(g * 2 + l, i, a, 16 * t);
+    *reinterpret_cast<uint4*>(row + 16 * t) = *reinterpret_cast<const uint4*>(kToFile ? drow : frow);
+    __syncthreads();
+    uint32_t out[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (uint32_t e = 0; e < 16; ++e) {
+        const uint32_t p = 16 * t + e;
+        uint32_t src;
+        bool used;
+        if (kToFile) {
+            const uint32_t w = p >> 1, j = p & 1, dir = w >= (uint32_t)kSteps, s = w - dir * kSteps;
+            used = w < 2u * kSteps;
+            src = j * kN + (dir ^ neg) * kHalf + dt_step(k, s);  // m and s are each other's step
+        } else {
+            const uint32_t s = dt_step(k, p & (kHalf - 1)), dir = ((p >> 10) & 1) ^ neg;
+            used = s < (uint32_t)kSteps;
+            src = (dir * kSteps + s) * 2 + (p >> 11);
+        }
+        if (used) out[e >> 2] |= (uint32_t)row[src] << (8 * (e & 3));
+    }
+    *reinterpret_cast<uint4*>(kToFile ? frow : drow) = make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-// One lane's row (g, a) over 4 queries' 16 accumulator columns (byte plane
+// One lane's row (slot, a) over 4 queries' 16 accumulator columns (byte plane
 // b of query k at column 4k + b): part_k = sum_b (256^(a+b) mod q) P[4k + b]
-// (< 2^60, unreduced), then summed over the 4 lanes a of group g as a
+// (< 2^60, unreduced), then summed over the 4 lanes a of a slot as a
 // reduce-scatter, so that lane a returns query a's total.  Round 1 (xor 1)
 // keeps queries a & 1 and (a & 1) + 2, round 2 (xor 2) keeps query a.
-__device__ __forceinline__ uint64_t tp_reduce4(const uint32_t (&v)[16], const uint32_t* c, int a) {
+__device__ __forceinline__ uint64_t tp_reduce4(const uint32_t (&v)[16], const uint32_t (&c)[4], int a) {
     uint64_t part[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-        part[k] = (uint64_t)c[a] * v[4 * k] + (uint64_t)c[a + 1] * v[4 * k + 1] + (uint64_t)c[a + 2] * v[4 * k + 2] +
-                  (uint64_t)c[a + 3] * v[4 * k + 3];
+        part[k] = (uint64_t)c[0] * v[4 * k] + (uint64_t)c[1] * v[4 * k + 1] + (uint64_t)c[2] * v[4 * k + 2] +
+                  (uint64_t)c[3] * v[4 * k + 3];
     const int b0 = a & 1, b1 = (a >> 1) & 1;
     const uint64_t keep0 = b0 ? part[1] : part[0], keep1 = b0 ? part[3] : part[2];
     const uint64_t send0 = b0 ? part[0] : part[1], send1 = b0 ? part[2] : part[3];
@@ -169,27 +176,19 @@ __device__ __forceinline__ uint64_t tp_reduce4(const uint32_t (&v)[16], const ui
 
 // ------------------------------------------------------------------ GEMM
 struct TpParams {
-    uint32_t* out;         // tp_out[l][i][q][g]
-    int nq_total;          // queries in the batch (out stride)
-    int q0;                // first query of this pass
+    const uint8_t* dt;     // D' tiles
+    uint32_t* out;         // tp_out, row of query 0 of the pass (row qmap[0] .. with a map)
+    size_t out_qstride;
     int nq;                // queries in this pass
-    int rq;                // key rows per slot in the B tile (4 nq)
-    int nb;                // N = key rows per item, roundup16(spi * rq)
-    int w8;                // 8-query groups per key-table position
-    const uint32_t* keyt;  // Kt[l][j][p][8 * w8], 32-byte aligned rows
-    int G;                 // groups (Dt rows per slot: 4G)
-    int li0;               // first (limb, slot) index l * N + i of this launch
-    int n_li;              // (limb, slot) indices it covers
-    int mti;               // M tiles (128 rows) per item (4G >= 128)
-    int n_mg;              // M-tile groups per (l, i)
-    int spi;               // slots per item (4G < 128: several slots share one 128-row A tile)
-    int rows_box;          // rows per A box
+    int nb;                // N = roundup16(4 nq)
+    int tile0;             // first 128-row tile of this launch
+    int n_items;           // work items of MTI tiles
     int stages;
     int acc_stages;
     uint32_t tmem_cols;
     int* err;
     unsigned* tiles;       // work-item counter, zero at launch
-    int has_qmap;          // output row of pass query p: qmap[p] (else q0 + p)
+    int has_qmap;          // output row of pass query p: qmap[p] (else p)
     uint8_t qmap[32];
     uint32_t c[2][7];      // 256^k mod q_l
     uint64_t cr[2];
@@ -198,56 +197,44 @@ struct TpParams {
                            // the abort path, IPB_TEST_ABORT_AFTER_ITEMS); 0: off
 };
 
-__global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_constant__ CUtensorMap map_a, TpParams P) {
+// Persistent, one CTA per SM, work items (MTI consecutive tiles) taken from a
+// per-launch atomic counter by the producer and published to the MMA thread
+// and the epilogue through a ring of shared slots (-1 ends it), so SMs held
+// by other kernels at launch take fewer items.  Warps: 0 producer (one
+// thread: MTI bulk copies of 16 KB and one key-plane tile per stage), 1 TMEM
+// allocation and MMA issue (one thread), 2..9 epilogue (two warps per TMEM
+// lane quarter).
+// Bound by HBM: the tensors are read once, 67 MB a group; 8.59 GB at 128
+// groups take 1.16 ms with 1 query (7.4 TB/s) and 1.23 ms with 32, 0.54 GB at
+// 8 groups 86 and 92 us.  (With the key planes gathered per slot: 1.20, 1.60,
+// 0.13 and 0.66 ms; 1 group, and any odd number, filled 4 rows of 128: 0.72 ms
+// against 20 us.)
+template <int MTI>
+__global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_constant__ CUtensorMap map_b, TpParams P) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int S = P.stages;
-    const uint32_t a_tile = 128 * 128;
-    const uint32_t a_region = (uint32_t)P.mti * a_tile;
-    const uint32_t b_bytes = (uint32_t)P.nb * 128;
-    const uint32_t stage_bytes = a_region + b_bytes;
-    const uint32_t tx_bytes = (uint32_t)P.mti * P.rows_box * 128;  // A only; B is written by the key warps
+    constexpr uint32_t a_region = (uint32_t)MTI * kTile;
+    const uint32_t stage_bytes = a_region + (uint32_t)P.nb * kKBlock;
+    const uint32_t tx_bytes = a_region + (uint32_t)P.nq * 4 * kKBlock;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)S * stage_bytes);
-    uint64_t* full = bars;               // the stage's A tiles have landed (TMA bytes)
+    uint64_t* full = bars;
     uint64_t* empty = bars + S;
     uint64_t* tfull = bars + 2 * S;
     uint64_t* tempty = bars + 2 * S + 2;
-    uint64_t* bfull = bars + 2 * S + 4;  // the stage's B tile is written (the key group's arrivals)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * S + 4);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 4);
     __shared__ volatile int abort_flag;
     __shared__ volatile int item_ring[kRing];
     __shared__ uint64_t ifull[kRing], iempty[kRing];
     __shared__ uint64_t mma_done;  // the MMA issuer's final commit: all its MMAs have completed
-    // tw[w] for w = dir * 1023 + s: t = 5^(1022 - s), or 2N - t when dir = 1;
-    // the two w of a 4-u group are one aligned 64-bit read.
-    __shared__ __align__(8) uint32_t tw[2 * kSteps + 2];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int w = threadIdx.x; w < 2 * kSteps + 2; w += blockDim.x) {
-        uint32_t t = 0;
-        if (w < 2 * kSteps) {
-            const int dir = w >= kSteps;
-            t = pow5_mod2n(kHalf - 2 - (w - dir * kSteps));
-            if (dir) t = (2 * kN - t) & (2 * kN - 1);
-        }
-        tw[w] = t;
-    }
     if (threadIdx.x == 0) {
         abort_flag = 0;
-        // full: the producer's expect_tx arrival (A bytes); bfull: the key
-        // group of the stage.  Kept apart so that the producer can wait for
-        // its own loads alone before the CTA exits.
-        for (int s = 0; s < S; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&bfull[s], kKeyGroup);
-            mbar_init(&empty[s], 1);
-        }
+        for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], 32 * kEpiWarps); }
+        for (int r = 0; r < kRing; ++r) { mbar_init(&ifull[r], 1); mbar_init(&iempty[r], 1 + 32 * kEpiWarps); }
         mbar_init(&mma_done, 1);
-        // tempty: 128 epilogue threads per share (warps 4..7 and each key
-        // group that fills no stages)
-        const int shares = 1 + kKeyGroups - (S < kKeyGroups ? S : kKeyGroups);
-        for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], 128 * shares); }
-        for (int r = 0; r < kRing; ++r) { mbar_init(&ifull[r], 1); mbar_init(&iempty[r], 1 + 128 + kKeyThreads); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -259,77 +246,8 @@ __global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const int n_items = (P.n_li / P.spi) * P.n_mg;
-    constexpr int ktiles = kUPad / 128;
-    const int acc_cols = P.mti * P.nb;
-    const int slot_rows = 4 * P.G;  // A rows of one slot
+    const int acc_cols = MTI * P.nb;
 
-    // Epilogue (TMEM -> reduced tensor-pass values) for the rows of lane
-    // quarter wq: warps 4..7 run it, and so do the warps of key groups that
-    // fill no stages (fewer stages than groups), each taking every nshare-th
-    // 16-column chunk, so the accumulators drain sooner when the MMA waits
-    // for them (one TMEM accumulator stage at 32 queries and G >= 97).
-    auto epilogue = [&](const int wq, const int share, const int nshare) {
-        const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-        int as = 0;
-        uint32_t aph = 0;
-        for (int it = 0;; ++it) {
-            const int r = it % kRing;
-            if (!mbar_wait_ab(&ifull[r], (uint32_t)(it / kRing) & 1, P.err, 18, &abort_flag)) { abort_flag = 1; break; }
-            const int item = item_ring[r];
-            mbar_arrive(&iempty[r]);
-            if (item < 0) break;
-            if (!mbar_wait_ab(&tfull[as], aph, P.err, 15, &abort_flag)) { abort_flag = 1; break; }
-            tc_fence_after();
-            const int li0 = P.li0 + (item / P.n_mg) * P.spi, mg = item % P.n_mg;
-            const int l = li0 / kN;
-            const uint32_t* c = P.c[l];
-            // spi == 1: TMEM block mt (columns mt * nb) holds M-tile mt of the
-            // slot's 4G rows.  spi > 1: lane row = sl * 4G + g*4 + a, and slot
-            // sl's keys are columns sl * rq ..; the loop runs over the slots
-            // this warp's 32 lanes touch (warp-uniform bounds for tcgen05.ld).
-            const int row = wq * 32 + lane;
-            const int nblk = P.spi > 1 ? min(P.spi - 1, (wq * 32 + 31) / slot_rows) - (wq * 32) / slot_rows + 1
-                                       : P.mti;
-            const int blk0 = P.spi > 1 ? (wq * 32) / slot_rows : 0;
-            const int nqc = (P.nq + 3) / 4;  // 16-column chunks per block
-            for (int bi = 0; bi < nblk; ++bi) {
-                const int mt = blk0 + bi;
-                const int li = li0 + (P.spi > 1 ? mt : 0);
-                const int grow = P.spi > 1 ? row - mt * slot_rows : (mg * P.mti + mt) * 128 + row;  // g*4 + a
-                const int g = grow >> 2, a = grow & 3;
-                const bool valid = grow >= 0 && grow < slot_rows;
-                // four queries (16 columns) per TMEM load where the block has
-                // them; the block's last columns one query at a time
-                const int lim = P.spi > 1 ? P.nb : (mt + 1) * P.nb;
-                for (int q = 0; q < P.nq; q += 4) {
-                    if ((bi * nqc + q / 4) % nshare != share) continue;  // this warp's share of the chunks
-                    const int col = (P.spi > 1 ? mt * P.rq : mt * P.nb) + 4 * q;
-                    const uint32_t ta = tmem_base + lane_base + (uint32_t)(as * acc_cols + col);
-                    uint32_t v[16];
-                    if (col + 16 <= lim) {
-                        tmem_ld16(ta, v);
-                    } else {
-    #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            uint32_t t[4] = {0, 0, 0, 0};
-                            if (col + 4 * k + 4 <= lim) tmem_ld4(ta + 4 * k, t);
-    #pragma unroll
-                            for (int e = 0; e < 4; ++e) v[4 * k + e] = t[e];
-                        }
-                    }
-                    const uint64_t tot = tp_reduce4(v, c, a);
-                    if (valid && q + a < P.nq) {
-                        const int qo = P.has_qmap ? P.qmap[P.q0 + q + a] : P.q0 + q + a;
-                        P.out[((size_t)li * P.nq_total + qo) * P.G + g] = mod_u64(tot, P.cr[l], P.q[l]);
-                    }
-                }
-            }
-            tc_fence_before();
-            mbar_arrive(&tempty[as]);
-            if (++as == P.acc_stages) { as = 0; aph ^= 1; }
-        }
-    };
     if (warp == 0) {
         if (lane == 0) {
             int s = 0;
@@ -340,21 +258,24 @@ __global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_const
                 int item = -1;
                 if (!abort_flag && mbar_wait_ab(&iempty[r], ((uint32_t)(it / kRing) & 1) ^ 1, P.err, 16, &abort_flag)) {
                     const unsigned t = atomicAdd(P.tiles, 1u);
-                    if (t < (unsigned)n_items) item = (int)t;
+                    if (t < (unsigned)P.n_items) item = (int)t;
                 } else {
                     abort_flag = 1;
                 }
                 item_ring[r] = item;
                 mbar_arrive(&ifull[r]);
                 if (item < 0) break;
-                const int li = P.li0 + (item / P.n_mg) * P.spi, mg = item % P.n_mg;
-                const int rowa = li * slot_rows + mg * P.mti * 128;
-                for (int kt = 0; kt < ktiles; ++kt) {
+                const int t0 = P.tile0 + item * MTI;
+                const int l = (t0 / kTilesPerPoly) & 1;  // an item's tiles are of one limb
+                const uint8_t* src = P.dt + (size_t)t0 * kKTiles * kTile;
+                for (int kt = 0; kt < kKTiles; ++kt) {
                     if (!mbar_wait_ab(&empty[s], ph ^ 1, P.err, 11, &abort_flag)) { abort_flag = 1; break; }
                     uint8_t* st = smem + (size_t)s * stage_bytes;
                     mbar_expect_tx(&full[s], tx_bytes);
-                    for (int mt = 0; mt < P.mti; ++mt)
-                        tma_load_2d(st + mt * a_tile, &map_a, &full[s], kt * 128, rowa + mt * 128);
+#pragma unroll
+                    for (int mt = 0; mt < MTI; ++mt)
+                        bulk_load(st + mt * kTile, src + ((size_t)mt * kKTiles + kt) * kTile, kTile, &full[s]);
+                    tma_load_4d(st + a_region, &map_b, &full[s], kt * kKBlock, 0, l, 0);
                     ++issued;
                     if (++s == S) { s = 0; ph ^= 1; }
                 }
@@ -370,10 +291,11 @@ __global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_const
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            // Packed slots: one M = 128 MMA over all spi slots' rows against all
-            // their key rows (N = nb); the epilogue keeps the diagonal blocks
-            // (slot rows x the same slot's key columns).
+            // One thread issues every MMA: descriptors are one 32-bit add each
+            // (address field of the low word), the loops unrolled.
             const uint32_t idesc = idesc_i8_kk(P.nb);
+            constexpr uint32_t kDescHi = smem_desc_hi_sw128(1024);
+            const uint32_t desc0 = smem_desc_lo(smem, 16);
             int s = 0, as = 0;
             uint32_t ph = 0, aph = 0;
             bool any_mma = false;
@@ -391,27 +313,16 @@ __global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_const
                 if (!mbar_wait_ab(&tempty[as], aph ^ 1, P.err, 13, &abort_flag)) { abort_flag = 1; break; }
                 tc_fence_after();
                 const uint32_t d0 = tmem_base + (uint32_t)(as * acc_cols);
-                for (int kt = 0; kt < ktiles; ++kt) {
-                    if (!mbar_wait_ab(&full[s], ph, P.err, 14, &abort_flag) || !mbar_wait_ab(&bfull[s], ph, P.err, 21, &abort_flag)) {
-                        abort_flag = 1;
-                        break;
-                    }
+                for (int kt = 0; kt < kKTiles; ++kt) {
+                    if (!mbar_wait_ab(&full[s], ph, P.err, 14, &abort_flag)) { abort_flag = 1; break; }
                     tc_fence_after();
-                    const uint8_t* st = smem + (size_t)s * stage_bytes;
-                    const uint8_t* bt = st + a_region;
+                    const uint32_t ad = desc0 + (uint32_t)s * (stage_bytes >> 4), bd = ad + (a_region >> 4);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
-                        if (P.spi == 1) {
-                            const uint64_t b = smem_desc(bt + kk * 32, 16, 1024);
-                            for (int mt = 0; mt < P.mti; ++mt)
-                                mma_i8(d0 + (uint32_t)(mt * P.nb), smem_desc(st + mt * a_tile + kk * 32, 16, 1024),
-                                       b, idesc, acc);
-                        } else {
-                            mma_i8(d0, smem_desc(st + kk * 32, 16, 1024), smem_desc(bt + kk * 32, 16, 1024), idesc,
-                                   acc);
-                        }
-                    }
+                    for (int kk = 0; kk < kKBlock / 32; ++kk)
+#pragma unroll
+                        for (int mt = 0; mt < MTI; ++mt)
+                            mma_i8_lo(d0 + (uint32_t)(mt * P.nb), ad + mt * (kTile >> 4) + kk * 2, bd + kk * 2, kDescHi,
+                                      kDescHi, idesc, (kt > 0 || kk > 0) ? 1u : 0u);
                     mma_commit(&empty[s]);
                     any_mma = true;
                     if (++s == S) { s = 0; ph ^= 1; }
@@ -426,87 +337,46 @@ __global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_const
                 mbar_wait(&mma_done, 0, P.err, 22);
             }
         }
-    } else if (warp >= 8) {
-        // ---------------- key planes: the B tile of every stage, gathered from
-        // the key table.  Unit = (slot sl, 8-query group q8, 4 consecutive u
-        // = steps w0, w0+1 x digits j = 0, 1): both digits of a step share the
-        // permuted position, so 2 permutations and 4 sector loads; bytes are
-        // regrouped into one 32-bit word per (query, byte plane) covering the
-        // 4 u.  Lanes take consecutive u groups, so a warp's stores hit 32
-        // distinct banks.  The stage of K tile kt of the n-th item is
-        // n * ktiles + kt in the producer's sequence (slot and phase follow).
-        //
-        // Groups take K tiles round robin, so a group can run ahead of the MMA
-        // by its stride of stages; an mbarrier parity wait tells the awaited
-        // phase apart from one two phases older only if the group's stride
-        // is <= the stage count.  So at most min(kKeyGroups, S) groups fill
-        // stages; the others only follow the item ring.
-        const int kid = (warp - 8) * 32 + lane;
-        const int grp = kid / kKeyGroup, gk = kid % kKeyGroup;
-        const int ngrp = S < kKeyGroups ? S : kKeyGroups;
-        if (grp >= ngrp) {
-            epilogue(warp & 3, 1 + grp - ngrp, 1 + kKeyGroups - ngrp);
-        } else {
-            const int units = P.spi * P.w8 * 32;
-            const int W = 8 * P.w8;
-            int base = 0;  // stages issued before this item
-            for (int it = 0;; ++it, base += ktiles) {
-                const int r = it % kRing;
-                if (!mbar_wait_ab(&ifull[r], (uint32_t)(it / kRing) & 1, P.err, 19, &abort_flag)) { abort_flag = 1; break; }
-                const int item = item_ring[r];
-                mbar_arrive(&iempty[r]);
-                if (item < 0) break;
-                const int li0 = P.li0 + (item / P.n_mg) * P.spi;
-                const int l = li0 / kN;
-                const uint32_t* kl = P.keyt + (size_t)l * kDeff * kN * W;  // [j][p][W]
-                for (int kt = grp; grp < ngrp && kt < ktiles; kt += ngrp) {
-                    const int seq = base + kt, s = seq % S;
-                    const uint32_t ph = (uint32_t)(seq / S) & 1;
-                    if (!mbar_wait_ab(&empty[s], ph ^ 1, P.err, 20, &abort_flag)) { abort_flag = 1; break; }
-                    uint8_t* bt = smem + (size_t)s * stage_bytes + a_region;
-                    for (int unit = gk; unit < units; unit += kKeyGroup) {
-                        const int u4 = unit & 31, sq = unit >> 5;
-                        const int sl = sq / P.w8, q8 = sq - sl * P.w8;
-                        const uint32_t odd = 2 * brev11((uint32_t)((li0 + sl) & (kN - 1))) + 1;
-                        const int w0 = kt * 64 + u4 * 2;  // even: w0 and w0 + 1 both < 2046 or both not
-                        uint32_t v[4][8];
-                        if (w0 < 2 * kSteps) {
-                            const uint2 tt = *reinterpret_cast<const uint2*>(&tw[w0]);
-                            const uint32_t p0 = perm_from_odd(tt.x, odd), p1 = perm_from_odd(tt.y, odd);
-                            ld_sector(kl + (size_t)p0 * W + 8 * q8, v[0]);          // w0, j = 0
-                            ld_sector(kl + ((size_t)kN + p0) * W + 8 * q8, v[1]);   // w0, j = 1
-                            ld_sector(kl + (size_t)p1 * W + 8 * q8, v[2]);          // w0 + 1, j = 0
-                            ld_sector(kl + ((size_t)kN + p1) * W + 8 * q8, v[3]);   // w0 + 1, j = 1
-                        } else {
+    } else {
+        // ---------------- epilogue: TMEM -> reduced tensor-pass values.  The
+        // two warps of a lane quarter take alternate 16-column chunks.
+        const int wq = warp & 3, share = (warp - 2) >> 2;
+        const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
+        const int a = lane & 3;
+        const int nqc = (P.nq + 3) / 4, chunks = MTI * nqc;
+        int as = 0;
+        uint32_t aph = 0;
+        for (int it = 0;; ++it) {
+            const int r = it % kRing;
+            if (!mbar_wait_ab(&ifull[r], (uint32_t)(it / kRing) & 1, P.err, 18, &abort_flag)) { abort_flag = 1; break; }
+            const int item = item_ring[r];
+            mbar_arrive(&iempty[r]);
+            if (item < 0) break;
+            if (!mbar_wait_ab(&tfull[as], aph, P.err, 15, &abort_flag)) { abort_flag = 1; break; }
+            tc_fence_after();
+            const int t0 = P.tile0 + item * MTI;
+            const int l = (t0 / kTilesPerPoly) & 1;
+            const uint64_t cr = P.cr[l];
+            const uint32_t q = P.q[l];
+            uint32_t c[4];
 #pragma unroll
-                            for (int e = 0; e < 4; ++e)
-#pragma unroll
-                                for (int c = 0; c < 8; ++c) v[e][c] = 0;
-                        }
-                        const uint32_t col = (uint32_t)u4 * 4;
-#pragma unroll
-                        for (int c = 0; c < 8; ++c) {
-                            const int q = q8 * 8 + c;
-                            if (q >= P.nq) break;
-                            const uint32_t lo01 = __byte_perm(v[0][c], v[1][c], 0x5140);
-                            const uint32_t lo23 = __byte_perm(v[2][c], v[3][c], 0x5140);
-                            const uint32_t hi01 = __byte_perm(v[0][c], v[1][c], 0x7362);
-                            const uint32_t hi23 = __byte_perm(v[2][c], v[3][c], 0x7362);
-                            const uint32_t row0 = (uint32_t)(sl * P.rq + q * 4);
-                            st_sw128(bt, row0 + 0, col, __byte_perm(lo01, lo23, 0x5410));  // byte 0 of u..u+3
-                            st_sw128(bt, row0 + 1, col, __byte_perm(lo01, lo23, 0x7632));  // byte 1
-                            st_sw128(bt, row0 + 2, col, __byte_perm(hi01, hi23, 0x5410));  // byte 2
-                            st_sw128(bt, row0 + 3, col, __byte_perm(hi01, hi23, 0x7632));  // byte 3
-                        }
-                    }
-                    // generic-proxy stores -> visible to the tensor core's async proxy
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    mbar_arrive(&bfull[s]);
+            for (int b = 0; b < 4; ++b) c[b] = P.c[l][a + b];
+            for (int ch = share; ch < chunks; ch += kEpiWarps / 4) {
+                const int mt = ch / nqc, q0 = (ch - mt * nqc) * 4;
+                const uint32_t ta = tmem_base + lane_base + (uint32_t)(as * acc_cols + mt * P.nb + 4 * q0);
+                uint32_t v[16];
+                tmem_ld16(ta, v);
+                const uint64_t tot = tp_reduce4(v, c, a);
+                if (q0 + a < P.nq) {
+                    const int qo = P.has_qmap ? P.qmap[q0 + a] : q0 + a;
+                    P.out[(size_t)qo * P.out_qstride + (size_t)(t0 + mt) * 32 + wq * 8 + (lane >> 2)] =
+                        mod_u64(tot, cr, q);
                 }
             }
+            tc_fence_before();
+            mbar_arrive(&tempty[as]);
+            if (++as == P.acc_stages) { as = 0; aph ^= 1; }
         }
-    } else if (warp >= 4) {
-        epilogue(warp & 3, 0, 1 + kKeyGroups - (S < kKeyGroups ? S : kKeyGroups));
     }
     tc_fence_before();
     __syncthreads();
@@ -531,14 +401,16 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint32_t box_rows) {
+// kplanes[q][l][b][4096] of nq queries; box: one K block of every (q, b) row
+// of one limb, rows 4 q + b of the B tile.
+bool make_map_b(CUtensorMap* m, const void* base, int nq) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return false;
-    cuuint64_t dims[2] = {(cuuint64_t)kUPad, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)kUPad};
-    cuuint32_t box[2] = {128, box_rows};
-    cuuint32_t es[2] = {1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, es,
+    cuuint64_t dims[4] = {(cuuint64_t)kK, 4, 2, (cuuint64_t)nq};
+    cuuint64_t strides[3] = {(cuuint64_t)kK, (cuuint64_t)4 * kK, (cuuint64_t)8 * kK};
+    cuuint32_t box[4] = {(cuuint32_t)kKBlock, 4, 1, (cuuint32_t)nq};
+    cuuint32_t es[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(base), dims, strides, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -556,81 +428,57 @@ uint32_t powmod_host(uint64_t b, uint64_t e, uint64_t q) {
 
 }  // namespace
 
-size_t tp_dt_bytes(size_t groups) { return (size_t)2 * kN * 4 * groups * kUPad; }
-size_t tp_keyt_bytes(int max_pass) { return (size_t)2 * kDeff * kN * 8 * (size_t)((max_pass + 7) / 8) * 4; }
+size_t tp_dt_bytes(size_t groups) { return (size_t)2 * kN * 4 * groups * kK; }
+int tp_tiles(size_t groups) { return (int)(2 * groups) * kTilesPerPoly; }
 
-int tp_pass_queries(size_t groups) {
-    // queries per GEMM pass so that the accumulators fit TMEM (512 columns)
-    const int mti = (int)std::min<size_t>(4, std::max<size_t>(1, (4 * groups + 127) / 128));
-    int b = 32;
-    while (b > 1 && mti * ((4 * b + 15) / 16 * 16) > 512) b /= 2;
-    return b;
-}
-
-cudaError_t launch_dt_transpose(const uint32_t* dp, const uint32_t* dm, size_t g0, size_t nw, size_t G, uint8_t* Dt,
-                                cudaStream_t s) {
+cudaError_t launch_dt_transpose(const uint32_t* dp, const uint32_t* dm, size_t g0, size_t nw, const DevTables* T,
+                                uint8_t* Dt, cudaStream_t s) {
     if (nw == 0) return cudaSuccess;
-    dt_transpose_kernel<<<dim3(kUPad / 32, kN / 32, (unsigned)(nw * 2)), 256, 0, s>>>(dp, dm, g0, G, Dt);
+    dt_transpose_kernel<<<dim3(kN / 8, 4, (unsigned)(nw * 2)), 256, 0, s>>>(dp, dm, g0, T, Dt);
     return cudaGetLastError();
 }
 
-cudaError_t launch_dt_export(const uint8_t* Dt, size_t g, size_t G, uint32_t* dp, uint32_t* dm, cudaStream_t s) {
-    const size_t n = (size_t)2 * kN * kUsed;
-    dt_export_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(Dt, g, G, dp, dm);
+cudaError_t launch_dt_export(const uint8_t* Dt, size_t g, const DevTables* T, uint32_t* dp, uint32_t* dm,
+                             cudaStream_t s) {
+    dt_export_kernel<<<(unsigned)((size_t)2 * kN * kK / 256), 256, 0, s>>>(Dt, g, T, dp, dm);
     return cudaGetLastError();
 }
 
-cudaError_t launch_tensor_pass(const uint8_t* Dt, size_t G, const uint32_t* keys, size_t key_qstride, int nq,
-                               int nq_total, int q0, uint32_t* keyt, uint32_t* tp_out, int* err, unsigned* tiles,
+cudaError_t launch_dt_file_rows(uint8_t* Dt, size_t G, size_t row0, size_t nrows, uint8_t* file, bool to_file,
+                                const DevTables* T, cudaStream_t s) {
+    if (nrows == 0) return cudaSuccess;
+    if (to_file)
+        dt_file_rows_kernel<true><<<(unsigned)nrows, 256, 0, s>>>(Dt, G, row0, file, T);
+    else
+        dt_file_rows_kernel<false><<<(unsigned)nrows, 256, 0, s>>>(Dt, G, row0, file, T);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tensor_pass(const uint8_t* Dt, int tile0, int n_tiles, const uint8_t* kplanes, int nq,
+                               const uint8_t* qmap, uint32_t* tp_out, size_t out_qstride, int* err, unsigned* tiles,
                                int num_sms, cudaStream_t s) {
-    return launch_tensor_pass_slots(Dt, G, 0, 2 * kN, keys, key_qstride, nq, nq_total, q0, nullptr, keyt, tp_out, err,
-                                    tiles, num_sms, s);
-}
-
-cudaError_t launch_tensor_pass_slots(const uint8_t* Dt, size_t G, int li0, int n_li, const uint32_t* keys,
-                                     size_t key_qstride, int nq, int nq_total, int q0, const uint8_t* qmap,
-                                     uint32_t* keyt, uint32_t* tp_out, int* err, unsigned* tiles, int num_sms,
-                                     cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
-    if (nq > 32 || !tiles || (qmap && q0 + nq > 32)) return cudaErrorInvalidValue;
-    if (n_li <= 0 || li0 < 0 || li0 + n_li > 2 * kN || li0 % 32 || n_li % 32) return cudaErrorInvalidValue;
-    const int rq = 4 * nq;
-    const int W = 8 * ((nq + 7) / 8);
-    const size_t kt_n = (size_t)2 * kDeff * kN * W;
-    keyt_kernel<<<(unsigned)((kt_n + 255) / 256), 256, 0, s>>>(keys, key_qstride, nq, W, keyt);
-    cudaError_t e = cudaGetLastError();
-    if (e) return e;
+    if (nq > 32 || !tiles || tile0 < 0 || n_tiles <= 0) return cudaErrorInvalidValue;
     TpParams P{};
+    P.dt = Dt;
     P.out = tp_out;
-    P.nq_total = nq_total;
-    P.q0 = q0;
+    P.out_qstride = out_qstride;
     P.nq = nq;
-    P.rq = rq;
-    P.w8 = W / 8;
-    P.keyt = keyt;
-    P.G = (int)G;
-    P.li0 = li0;
-    P.n_li = n_li;
+    P.nb = (4 * nq + 15) / 16 * 16;
+    P.tile0 = tile0;
     P.has_qmap = qmap != nullptr;
     if (qmap)
-        for (int p = 0; p < q0 + nq; ++p) P.qmap[p] = qmap[p];
-    const int nmt = (int)std::max<size_t>(1, (4 * G + 127) / 128);
-    P.mti = std::min(nmt, 4);
-    P.n_mg = nmt / P.mti;
-    // Small G: pack spi slots (each 4G rows) into one 128-row A tile.  G even
-    // keeps every slot start on an 8-row (1024-byte) swizzle atom; spi a power
-    // of two divides kN, so a packed item never straddles the two limbs.
-    auto nb_of = [&](int sp) { return ((sp * rq + 15) / 16) * 16; };
-    P.spi = 1;
-    if (4 * G < 128 && G % 2 == 0) {
-        while (2 * P.spi * 4 * (int)G <= 128) P.spi *= 2;
-        while (P.spi > 1 && (nb_of(P.spi) > 256 || 2 * nb_of(P.spi) > 512)) P.spi /= 2;
-    }
-    P.nb = nb_of(P.spi);
-    P.rows_box = (int)std::min<size_t>(128, 4 * G * (size_t)P.spi);
-    if (P.mti * P.nb > 512) return cudaErrorInvalidValue;
-    P.acc_stages = (2 * P.mti * P.nb <= 512) ? 2 : 1;
-    uint32_t need = (uint32_t)(P.acc_stages * P.mti * P.nb), tc = 32;
+        for (int p = 0; p < nq; ++p) P.qmap[p] = qmap[p];
+    const int sms = std::max(1, num_sms);
+    // Two tiles per item (their MMAs share a stage's key planes) once that
+    // leaves an item per SM.  G = 1 (128 tiles), 32 queries: 20 us with one tile,
+    // 25 with two; G = 128, 32 queries: 1255 and 1227 us (four tiles, whose
+    // accumulators cannot be double-buffered: 1300); between, within 3 %.
+    const int mti = n_tiles % 2 == 0 && tile0 % 2 == 0 && n_tiles >= 2 * sms ? 2 : 1;
+    const auto kernel = mti == 2 ? tp_tc_kernel<2> : tp_tc_kernel<1>;
+    P.n_items = n_tiles / mti;
+    P.acc_stages = 2;  // at most 2 x 2 x 128 columns
+    uint32_t need = (uint32_t)(P.acc_stages * mti * P.nb), tc = 32;
     while (tc < need) tc <<= 1;
     P.tmem_cols = tc;
     P.err = err;
@@ -642,21 +490,19 @@ cudaError_t launch_tensor_pass_slots(const uint8_t* Dt, size_t G, int li0, int n
         P.cr[l] = ~0ULL / qs[l];
         P.q[l] = qs[l];
     }
-    const size_t a_region = (size_t)P.mti * 128 * 128;
-    const size_t stage_bytes = a_region + (size_t)P.nb * 128;
+    const size_t stage_bytes = (size_t)mti * kTile + (size_t)P.nb * kKBlock;
     // As many stages as the device's shared memory takes (1 KB alignment
-    // slack, 256 B of barriers): at 128 groups, three up to 16 queries.
+    // slack, 512 B of barriers).
     size_t max_dyn = 0;
-    e = allow_max_smem(tp_tc_kernel, &max_dyn);
+    cudaError_t e = allow_max_smem(kernel, &max_dyn);
     if (e) return e;
-    P.stages = (int)std::min<size_t>(8, (max_dyn - 1024 - 256) / stage_bytes);
+    P.stages = (int)std::min<size_t>(12, (max_dyn - 1024 - 512) / stage_bytes);
     if (P.stages < 2) return cudaErrorInvalidValue;
-    CUtensorMap ma;
-    if (!make_map(&ma, Dt, (uint64_t)2 * kN * 4 * G, (uint32_t)P.rows_box)) return cudaErrorInvalidValue;
-    const size_t smem = 1024 + (size_t)P.stages * stage_bytes + (3 * P.stages + 4) * 8 + 16;
-    const int items = (n_li / P.spi) * P.n_mg;
+    CUtensorMap mb;
+    if (!make_map_b(&mb, kplanes, nq)) return cudaErrorInvalidValue;
+    const size_t smem = 1024 + (size_t)P.stages * stage_bytes + (2 * P.stages + 4) * 8 + 16;
     if ((e = cudaMemsetAsync(tiles, 0, sizeof(unsigned), s))) return e;
-    tp_tc_kernel<<<std::min(items, std::max(1, num_sms)), kTpThreads, smem, s>>>(ma, P);
+    kernel<<<std::min(P.n_items, sms), kTpThreads, smem, s>>>(mb, P);
     return cudaGetLastError();
 }
 
