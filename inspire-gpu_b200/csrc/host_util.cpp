@@ -121,8 +121,8 @@ void build_tables(DevTables& T) {
         for (uint32_t i = 0; i < (uint32_t)kN; ++i) {
             uint32_t w = (uint32_t)powmod(psi, brev(i, kLogN), q);
             uint32_t wi = i ? (uint32_t)powmod(w, q - 2, q) : 1u;
-            L.fwd[i] = make_uint2(w, shoup(w, (uint32_t)q));
-            L.inv[i] = make_uint2(wi, shoup(wi, (uint32_t)q));
+            L.fwd[tw_index((int)i)] = make_uint2(w, shoup(w, (uint32_t)q));
+            L.inv[tw_index((int)i)] = make_uint2(wi, shoup(wi, (uint32_t)q));
         }
         L.inv_n = (uint32_t)powmod(kN, q - 2, q);
         L.inv_n_p = shoup(L.inv_n, (uint32_t)q);
@@ -132,6 +132,16 @@ void build_tables(DevTables& T) {
     T.crt_c[1] = (uint32_t)powmod(kQ0 % kQ1, kQ1 - 2, kQ1);
     T.crt_cp[0] = shoup(T.crt_c[0], kQ0);
     T.crt_cp[1] = shoup(T.crt_c[1], kQ1);
+    for (int l = 0; l < 2; ++l) {
+        LimbTables& L = T.limb[l];
+        const uint32_t q = L.q;
+        auto scale = [&](uint64_t c) {
+            const uint32_t w = (uint32_t)(c * L.inv[1].x % q);
+            return NttScale{make_uint2((uint32_t)c, shoup((uint32_t)c, q)), make_uint2(w, shoup(w, q))};
+        };
+        L.scale_n = scale(L.inv_n);
+        L.scale_crt = scale((uint64_t)L.inv_n * T.crt_c[l] % q);
+    }
     uint32_t p5 = 1;
     for (uint32_t m = 0; m < (uint32_t)kHalf; ++m, p5 = p5 * 5 % (2 * kN))
         for (uint32_t rho = 0; rho < 2; ++rho) {

@@ -8,23 +8,28 @@
 // src/ntt.cpp:107-149): Cooley-Tukey DIT forward with twiddles
 // fwd[i] = psi^BR(i), Gentleman-Sande inverse with inv[i] = fwd[i]^-1 and a
 // final N^-1 scale.  Output slot i holds the evaluation at psi^(2 BR(i)+1).
-// Every stage here computes the same mathematical transform with Harvey
-// lazy reduction and a final reduction to [0, q), so results are identical.
+// Every stage here computes the same mathematical transform lazily and
+// reduces to [0, q) at the end, so results are identical.  A 27-bit q leaves
+// room for 45 q in a word and Shoup multiplication takes any word, so a
+// forward stage only adds (its values grow by 2 q) and no forward transform
+// reduces before its end; an inverse stage doubles its sums, and two of a
+// thread's eight values are reduced after each three stages.  (With a
+// conditional subtraction in every butterfly a Horner step took 6.0 us on
+// 4 CTAs and 4.5 us on 8.)
 //
 // The transform runs on one "NTT group" of 256 threads holding 8 elements
-// each in registers; three shared-memory exchanges (XOR-swizzled, bank
-// conflict free) move between the four register layouts
+// each in registers; three shared-memory exchanges (four words of padding per
+// 32: bank-conflict free, and every address of a thread is one register plus a
+// constant) move between the four register layouts
 //   L1: x = t + 256 e        stages s = 10, 9, 8
 //   L2: x = (t&31) + 32 e + 256 (t>>5)   s = 7, 6, 5
 //   L3: x = (t&3) + 4 e + 32 (t>>2)      s = 4, 3, 2
 //   L4: x = 8 t + e          stages s = 1, 0
 // A forward NTT takes L1 in and leaves L4; the inverse takes L4 to L1.
 // Only L1 <-> L2 moves data between warps: in L2, L3 and L4 warp w holds
-// x in [256w, 256w + 256), a region the swizzle keeps in place, so those
-// exchanges need a warp barrier only.  Each transform starts with a group
-// barrier before its first store, which orders it after the previous
-// transform's reads of the same buffer; the second buffer is only ever
-// touched warp-locally.
+// x in [256w, 256w + 256), its own part of the buffer, so those exchanges need
+// warp barriers only.  Each transform starts with a group barrier before its
+// first store, which orders it after the previous transform's reads.
 // Several groups can share a CTA, each synchronising on its own named
 // barrier (bar.sync id, 256).
 #pragma once
@@ -45,10 +50,18 @@ constexpr uint32_t kQ1 = 95293441u;
 constexpr uint32_t kP = 65535u;        // plaintext modulus (Mersenne)
 constexpr uint64_t kQFull = (uint64_t)kQ0 * kQ1;
 
-// Per-limb tables, one set per device.  tw* entries are (w, floor(w 2^32/q)).
+// Per-limb tables, one set per device.  Entries are (w, floor(w 2^32/q)),
+// stored at tw_index.
+// An inverse transform scales by a constant c of its last stage: NttScale is
+// (c, c inv[1]) with Shoup factors.
+struct NttScale {
+    uint2 c, w;
+};
 struct LimbTables {
-    uint2 fwd[kN];
-    uint2 inv[kN];
+    alignas(16) uint2 fwd[kN];
+    alignas(16) uint2 inv[kN];
+    NttScale scale_n;            // N^-1
+    NttScale scale_crt;          // N^-1 times the limb's CRT factor crt_c
     uint32_t q;
     uint32_t inv_n, inv_n_p;     // N^-1 and its Shoup factor
     uint64_t cr;                 // floor(2^64 / q), exact u64 Barrett
@@ -94,158 +107,238 @@ __device__ __forceinline__ void gsync(int bar) {
     if (bar == 0) __syncthreads();
     else asm volatile("bar.sync %0, 256;" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ uint32_t swz(uint32_t x) { return x ^ ((x >> 3) & 0x1Cu); }
-
-// ------------------------------------------------------------ butterflies
-__device__ __forceinline__ void bf_fwd(uint32_t& u, uint32_t& v, uint2 w, uint32_t q) {
-    const uint32_t q2 = 2 * q;
-    uint32_t uu = csub(u, q2);                 // [0, 2q)
-    uint32_t tt = shoup_mul(v, w.x, w.y, q);   // [0, 2q)
-    u = uu + tt;                               // [0, 4q)
-    v = uu + q2 - tt;                          // (0, 4q)
-}
-__device__ __forceinline__ void bf_inv(uint32_t& u, uint32_t& v, uint2 w, uint32_t q) {
-    const uint32_t q2 = 2 * q;
-    uint32_t s = csub(u + v, q2);              // inputs < 2q -> [0, 2q)
-    uint32_t d = u + q2 - v;                   // (0, 4q)
-    v = shoup_mul(d, w.x, w.y, q);             // [0, 2q)
-    u = s;
+constexpr int kNttBuf = kN + kN / 8;  // words of one group's exchange buffer
+// Where the tables hold twiddle i: the four entries that one thread reads for
+// stage 0 (i = 1024 + 4t ..) and stage 2 (256 + 4h ..) lie as two pairs half
+// the stage's range apart, so the lanes of a warp read consecutive 16 bytes.
+__host__ __device__ constexpr int tw_index(int i) {
+    const int n = i >= 1024 ? 1024 : i >= 256 && i < 512 ? 256 : 0;
+    return n == 0 ? i : n + ((i >> 1) & 1) * (n / 2) + (i - n) / 4 * 2 + (i & 1);
 }
 
-// One stage on the register tile: e-bit k <-> x-bit (B0 + k).
-template <int B0, bool FWD>
-__device__ __forceinline__ void ntt_stage(uint32_t (&r)[8], const int k, const uint32_t xbase,
-                                          const uint2* __restrict__ tw, uint32_t q) {
-    const int s = B0 + k;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        if (e & (1 << k)) continue;
-        const int e2 = e | (1 << k);
-        const uint32_t x = xbase + ((uint32_t)e << B0);
-        const uint2 w = tw[(1u << (10 - s)) + (x >> (s + 1))];
-        if (FWD) bf_fwd(r[e], r[e2], w, q);
-        else bf_inv(r[e], r[e2], w, q);
-    }
-}
+// x mod q up to one q, for any word: [0, 2q).  floor(2^32 / q) is 45 for both
+// primes; the estimate of the quotient (< 46) is low by less than 1.5.
+__device__ __forceinline__ uint32_t red2(uint32_t x, uint32_t q) { return x - __umulhi(x, 45u) * q; }
+static_assert((1ull << 32) / kQ0 == 45 && (1ull << 32) / kQ1 == 45, "red2");
 
-// Layout helpers: xbase and B0 per layout id (1..4).
+// Layout helpers: a thread's first exchange-buffer word and the distance of
+// its elements (x + 4 (x >> 5) at the layout's x) per layout id (1..4).
 template <int L> __device__ __forceinline__ uint32_t lay_base(uint32_t t);
-template <> __device__ __forceinline__ uint32_t lay_base<1>(uint32_t t) { return t; }
-template <> __device__ __forceinline__ uint32_t lay_base<2>(uint32_t t) { return (t & 31) + 256 * (t >> 5); }
-template <> __device__ __forceinline__ uint32_t lay_base<3>(uint32_t t) { return (t & 3) + 32 * (t >> 2); }
-template <> __device__ __forceinline__ uint32_t lay_base<4>(uint32_t t) { return 8 * t; }
-template <int L> struct LayB0;
-template <> struct LayB0<1> { static constexpr int v = 8; };
-template <> struct LayB0<2> { static constexpr int v = 5; };
-template <> struct LayB0<3> { static constexpr int v = 2; };
-template <> struct LayB0<4> { static constexpr int v = 0; };
+template <> __device__ __forceinline__ uint32_t lay_base<1>(uint32_t t) { return t + 4 * (t >> 5); }
+template <> __device__ __forceinline__ uint32_t lay_base<2>(uint32_t t) { return (t & 31) + 288 * (t >> 5); }
+template <> __device__ __forceinline__ uint32_t lay_base<3>(uint32_t t) { return (t & 3) + 36 * (t >> 2); }
+template <> __device__ __forceinline__ uint32_t lay_base<4>(uint32_t t) { return 8 * t + 4 * (t >> 2); }
+template <int L> struct LayStep;
+template <> struct LayStep<1> { static constexpr int v = 288; };
+template <> struct LayStep<2> { static constexpr int v = 36; };
+template <> struct LayStep<3> { static constexpr int v = 4; };
+template <> struct LayStep<4> { static constexpr int v = 1; };
 
 template <int L>
 __device__ __forceinline__ void lay_store(const uint32_t (&r)[8], uint32_t* s, uint32_t t) {
+    uint32_t* p = s + lay_base<L>(t);
     if (L == 4) {
-        *reinterpret_cast<uint4*>(s + swz(8 * t)) = make_uint4(r[0], r[1], r[2], r[3]);
-        *reinterpret_cast<uint4*>(s + swz(8 * t + 4)) = make_uint4(r[4], r[5], r[6], r[7]);
+        *reinterpret_cast<uint4*>(p) = make_uint4(r[0], r[1], r[2], r[3]);
+        *reinterpret_cast<uint4*>(p + 4) = make_uint4(r[4], r[5], r[6], r[7]);
     } else {
-        const uint32_t b = lay_base<L>(t);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) s[swz(b + ((uint32_t)e << LayB0<L>::v))] = r[e];
+        for (int e = 0; e < 8; ++e) p[e * LayStep<L>::v] = r[e];
     }
 }
 template <int L>
 __device__ __forceinline__ void lay_load(uint32_t (&r)[8], const uint32_t* s, uint32_t t) {
+    const uint32_t* p = s + lay_base<L>(t);
     if (L == 4) {
-        uint4 a = *reinterpret_cast<const uint4*>(s + swz(8 * t));
-        uint4 b = *reinterpret_cast<const uint4*>(s + swz(8 * t + 4));
+        uint4 a = *reinterpret_cast<const uint4*>(p);
+        uint4 b = *reinterpret_cast<const uint4*>(p + 4);
         r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
         r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
     } else {
-        const uint32_t b = lay_base<L>(t);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) r[e] = s[swz(b + ((uint32_t)e << LayB0<L>::v))];
+        for (int e = 0; e < 8; ++e) r[e] = p[e * LayStep<L>::v];
     }
 }
 
-// Forward NTT: r in L1 (any values < 4q) -> r in L4, canonical [0, q).
-// sbuf: 2*2048 u32 private to this group.  All 256 threads must call.
-__device__ __forceinline__ void ntt_fwd(uint32_t (&r)[8], uint32_t* sbuf, const uint2* __restrict__ tw,
-                                        uint32_t q, uint32_t t, int bar) {
-    uint32_t* A = sbuf;
-    uint32_t* B = sbuf + kN;
-    ntt_stage<8, true>(r, 2, lay_base<1>(t), tw, q);
-    ntt_stage<8, true>(r, 1, lay_base<1>(t), tw, q);
-    ntt_stage<8, true>(r, 0, lay_base<1>(t), tw, q);
-    gsync(bar);
-    lay_store<1>(r, A, t); gsync(bar); lay_load<2>(r, A, t);
-    ntt_stage<5, true>(r, 2, lay_base<2>(t), tw, q);
-    ntt_stage<5, true>(r, 1, lay_base<2>(t), tw, q);
-    ntt_stage<5, true>(r, 0, lay_base<2>(t), tw, q);
-    lay_store<2>(r, B, t); __syncwarp(); lay_load<3>(r, B, t);
-    ntt_stage<2, true>(r, 2, lay_base<3>(t), tw, q);
-    ntt_stage<2, true>(r, 1, lay_base<3>(t), tw, q);
-    ntt_stage<2, true>(r, 0, lay_base<3>(t), tw, q);
-    lay_store<3>(r, A, t); __syncwarp(); lay_load<4>(r, A, t);
-    ntt_stage<0, true>(r, 1, lay_base<4>(t), tw, q);
-    ntt_stage<0, true>(r, 0, lay_base<4>(t), tw, q);
-    const uint32_t q2 = 2 * q;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) r[e] = csub(csub(r[e], q2), q);
+// ------------------------------------------------------------ twiddles
+// The twiddles of one register pass over layout L: w[0] for k = 2, w[1..2]
+// for k = 1, w[3..6] for k = 0 (stage s = B0 + k, k = bit of the register
+// index; L4 has k = 1, 0 only).  Entry of stage s at x: number 2^(10-s) + (x >> (s+1)).
+struct Tw {
+    uint2 w[7];
+};
+__device__ __forceinline__ void ld_tw2(uint2 (&w)[7], int i, const uint2* p) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    w[i] = make_uint2(v.x, v.y);
+    w[i + 1] = make_uint2(v.z, v.w);
+}
+template <int L>
+__device__ __forceinline__ Tw load_tw(const uint2* __restrict__ tw, uint32_t t) {
+    Tw r;
+    if (L == 4) {
+        ld_tw2(r.w, 1, tw + 512 + 2 * t);
+        ld_tw2(r.w, 3, tw + 1024 + 2 * t);
+        ld_tw2(r.w, 5, tw + 1536 + 2 * t);
+    } else if (L == 3) {
+        r.w[0] = tw[64 + (t >> 2)];
+        ld_tw2(r.w, 1, tw + 128 + 2 * (t >> 2));
+        ld_tw2(r.w, 3, tw + 256 + 2 * (t >> 2));
+        ld_tw2(r.w, 5, tw + 384 + 2 * (t >> 2));
+    } else {
+        const uint32_t h = L == 1 ? 0u : t >> 5;
+        constexpr int b = L == 1 ? 1 : 8;
+        r.w[0] = tw[b + h];
+        ld_tw2(r.w, 1, tw + 2 * b + 2 * h);
+        ld_tw2(r.w, 3, tw + 4 * b + 4 * h);
+        ld_tw2(r.w, 5, tw + 4 * b + 4 * h + 2);
+    }
+    return r;
 }
 
-// Inverse NTT incl. N^-1: r in L4 (values < 2q) -> r in L1, canonical.
-__device__ __forceinline__ void ntt_inv(uint32_t (&r)[8], uint32_t* sbuf, const uint2* __restrict__ tw,
-                                        uint32_t q, uint32_t inv_n, uint32_t inv_n_p, uint32_t t, int bar) {
-    uint32_t* A = sbuf;
-    uint32_t* B = sbuf + kN;
-    ntt_stage<0, false>(r, 0, lay_base<4>(t), tw, q);
-    ntt_stage<0, false>(r, 1, lay_base<4>(t), tw, q);
-    gsync(bar);
-    lay_store<4>(r, A, t); __syncwarp(); lay_load<3>(r, A, t);
-    ntt_stage<2, false>(r, 0, lay_base<3>(t), tw, q);
-    ntt_stage<2, false>(r, 1, lay_base<3>(t), tw, q);
-    ntt_stage<2, false>(r, 2, lay_base<3>(t), tw, q);
-    lay_store<3>(r, B, t); __syncwarp(); lay_load<2>(r, B, t);
-    ntt_stage<5, false>(r, 0, lay_base<2>(t), tw, q);
-    ntt_stage<5, false>(r, 1, lay_base<2>(t), tw, q);
-    ntt_stage<5, false>(r, 2, lay_base<2>(t), tw, q);
-    lay_store<2>(r, A, t); gsync(bar); lay_load<1>(r, A, t);
-    ntt_stage<8, false>(r, 0, lay_base<1>(t), tw, q);
-    ntt_stage<8, false>(r, 1, lay_base<1>(t), tw, q);
-    ntt_stage<8, false>(r, 2, lay_base<1>(t), tw, q);
+// Register pass of a forward transform: stages k = K - 1 .. 0.  Values grow
+// by 2q per stage.
+template <int K>
+__device__ __forceinline__ void pass_fwd(uint32_t (&r)[8], const Tw& T, uint32_t q) {
+    const uint32_t q2 = 2 * q;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) r[e] = csub(shoup_mul(r[e], inv_n, inv_n_p, q), q);
+    for (int k = K - 1; k >= 0; --k)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            if (e & (1 << k)) continue;
+            const uint2 w = T.w[(1 << (2 - k)) - 1 + (e >> (k + 1))];
+            const uint32_t v = shoup_mul(r[e | (1 << k)], w.x, w.y, q), u = r[e];
+            r[e] = u + v;
+            r[e | (1 << k)] = u + q2 - v;
+        }
+}
+// Register pass of an inverse transform: stages k = 0 .. K - 1 on values
+// <= B q.  bound[] (compile-time, in q) follows each value; what ends above
+// 4q is reduced, so the pass leaves values <= 4q.
+template <int K, int B>
+__device__ __forceinline__ void pass_inv(uint32_t (&r)[8], const Tw& T, uint32_t q) {
+    int bound[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) bound[e] = B;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            if (e & (1 << k)) continue;
+            const int e2 = e | (1 << k);
+            const uint2 w = T.w[(1 << (2 - k)) - 1 + (e >> (k + 1))];
+            const uint32_t u = r[e], v = r[e2];
+            r[e] = u + v;
+            r[e2] = shoup_mul(u + (uint32_t)bound[e2] * q - v, w.x, w.y, q);
+            bound[e] += bound[e2];
+            bound[e2] = 2;
+        }
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        if (bound[e] > 4) r[e] = red2(r[e], q);
+}
+// The last pass of an inverse transform (stages 8, 9, 10) on values <= 4q:
+// the scale goes into the last stage's two multiplications.  Leaves [0, q).
+__device__ __forceinline__ void pass_inv_last(uint32_t (&r)[8], const Tw& T, const NttScale& c, uint32_t q) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            if (e & (1 << k)) continue;
+            const int e2 = e | (1 << k);
+            const uint2 w = T.w[(1 << (2 - k)) - 1 + (e >> (k + 1))];
+            const uint32_t u = r[e], v = r[e2];
+            // bounds: k = 0: 4, 4; k = 1: 8, 8 (e even), 2, 2 (e odd)
+            r[e] = u + v;
+            r[e2] = shoup_mul(u + (k == 0 ? 4u : (e & 1) ? 2u : 8u) * q - v, w.x, w.y, q);
+        }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const uint32_t u = r[e], v = r[e + 4];  // <= 16q (e = 0), 4q, 2q
+        r[e] = csub(shoup_mul(u + v, c.c.x, c.c.y, q), q);
+        r[e + 4] = csub(shoup_mul(u + 16u * q - v, c.w.x, c.w.y, q), q);
+    }
+}
+
+// Forward NTT without the final reduction: r in L1 (values <= 4q) -> r in L4,
+// values < 26q.  buf: kNttBuf u32 private to this group.  All 256 threads must
+// call.
+__device__ __forceinline__ void ntt_fwd_lazy(uint32_t (&r)[8], uint32_t* buf, const uint2* __restrict__ tw, uint32_t q,
+                                             uint32_t t, int bar) {
+    pass_fwd<3>(r, load_tw<1>(tw, t), q);
+    const Tw w2 = load_tw<2>(tw, t);
+    gsync(bar);
+    lay_store<1>(r, buf, t); gsync(bar); lay_load<2>(r, buf, t);
+    pass_fwd<3>(r, w2, q);
+    const Tw w3 = load_tw<3>(tw, t);
+    __syncwarp(); lay_store<2>(r, buf, t); __syncwarp(); lay_load<3>(r, buf, t);
+    pass_fwd<3>(r, w3, q);
+    const Tw w4 = load_tw<4>(tw, t);
+    __syncwarp(); lay_store<3>(r, buf, t); __syncwarp(); lay_load<4>(r, buf, t);
+    pass_fwd<2>(r, w4, q);
+}
+// Forward NTT: r in L1 (values <= 4q) -> r in L4, canonical [0, q).
+__device__ __forceinline__ void ntt_fwd(uint32_t (&r)[8], uint32_t* buf, const uint2* __restrict__ tw,
+                                        uint32_t q, uint32_t t, int bar) {
+    ntt_fwd_lazy(r, buf, tw, q, t, bar);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) r[e] = csub(red2(r[e], q), q);
+}
+
+// Inverse NTT times a constant: r in L4 (values <= 2q) -> r in L1, canonical.
+// In two halves around the exchange between warps, for callers that read
+// shared state between the two group barriers.
+__device__ __forceinline__ void ntt_inv_head(uint32_t (&r)[8], uint32_t* buf, const uint2* __restrict__ tw, uint32_t q,
+                                             uint32_t t, int bar) {
+    pass_inv<2, 2>(r, load_tw<4>(tw, t), q);
+    const Tw w3 = load_tw<3>(tw, t);
+    gsync(bar);
+    lay_store<4>(r, buf, t); __syncwarp(); lay_load<3>(r, buf, t);
+    pass_inv<3, 4>(r, w3, q);
+    const Tw w2 = load_tw<2>(tw, t);
+    __syncwarp(); lay_store<3>(r, buf, t); __syncwarp(); lay_load<2>(r, buf, t);
+    pass_inv<3, 4>(r, w2, q);
+    __syncwarp(); lay_store<2>(r, buf, t);
+}
+__device__ __forceinline__ void ntt_inv_tail(uint32_t (&r)[8], uint32_t* buf, const uint2* __restrict__ tw, uint32_t q,
+                                             const NttScale& c, uint32_t t, int bar) {
+    const Tw w1 = load_tw<1>(tw, t);
+    gsync(bar);
+    lay_load<1>(r, buf, t);
+    pass_inv_last(r, w1, c, q);
+}
+__device__ __forceinline__ void ntt_inv(uint32_t (&r)[8], uint32_t* buf, const uint2* __restrict__ tw, uint32_t q,
+                                        const NttScale& c, uint32_t t, int bar) {
+    ntt_inv_head(r, buf, tw, q, t, bar);
+    ntt_inv_tail(r, buf, tw, q, c, t, bar);
 }
 
 // ------------------------------------------------------------ gadget decomposition
 // One coefficient: CRT lift of (c0 mod q0, c1 mod q1) to [0, Q), center to
-// (-Q/2, Q/2], three signed base-2^18 digits, digit 0 dropped
-// (src/ring.cpp:205-246).  Returns digits 1 and 2 as signed values.
-// The CRT factors in registers: kernels whose loops contain asm with memory
-// clobbers (mbarrier waits, st.async) would otherwise reload them from the
-// table in global memory at every use.
-struct CrtK {
-    uint32_t c0, cp0, c1, cp1;
-};
-__device__ __forceinline__ CrtK crt_consts(const DevTables& T) {
-    return CrtK{T.crt_c[0], T.crt_cp[0], T.crt_c[1], T.crt_cp[1]};
+// r in (-Q/2, Q/2], three signed base-2^18 digits, digit 0 dropped
+// (src/ring.cpp:205-246).  t_l = c_l crt_c[l] mod q_l (canonical), so the lift
+// is t0 q1 + t1 q0 mod Q; digit 1 is bits 18..35 of r + 2^17 as a signed
+// number and digit 2 the bits from 36 on of r + 2^17 + 2^35 (the carries of
+// the balanced digits below).  lift_plus returns r + c from the
+// terms ta, tb of the two limbs (primes qa, qb) in either order.
+__device__ __forceinline__ uint64_t lift_plus(uint32_t ta, uint32_t tb, uint32_t qa, uint32_t qb, uint64_t c) {
+    uint64_t v = (uint64_t)ta * qb + ((uint64_t)tb * qa + c);  // < 2Q + c
+    uint64_t n = v > kQFull / 2 + c ? kQFull : 0;
+    if (v > kQFull + kQFull / 2 + c) n = 2 * kQFull;
+    return v - n;
 }
-__device__ __forceinline__ void decomp2(uint32_t c0, uint32_t c1, const CrtK& k, int64_t& d1, int64_t& d2) {
-    uint32_t t0 = csub(shoup_mul(c0, k.c0, k.cp0, kQ0), kQ0);
-    uint32_t t1 = csub(shoup_mul(c1, k.c1, k.cp1, kQ1), kQ1);
-    uint64_t v = (uint64_t)t0 * kQ1 + (uint64_t)t1 * kQ0;   // < 2Q
-    if (v >= kQFull) v -= kQFull;
-    int64_t r = (v <= kQFull / 2) ? (int64_t)v : (int64_t)v - (int64_t)kQFull;
-    constexpr int K = 64 - kBaseLog;
-    int64_t d0 = (int64_t)((uint64_t)r << K) >> K;
-    r = (r - d0) >> kBaseLog;
-    d1 = (int64_t)((uint64_t)r << K) >> K;
-    r = (r - d1) >> kBaseLog;
-    d2 = (int64_t)((uint64_t)r << K) >> K;
+constexpr uint64_t kCarry1 = 1ull << (kBaseLog - 1), kCarry2 = kCarry1 + (1ull << (2 * kBaseLog - 1));
+__device__ __forceinline__ int32_t digit1(uint64_t r_carry1) { return (int32_t)(r_carry1 >> 4) >> 14; }
+__device__ __forceinline__ int32_t digit2(uint64_t r_carry2) { return (int32_t)(r_carry2 >> 32) >> 4; }
+static_assert(kBaseLog == 18, "digit1, digit2");
+
+__device__ __forceinline__ void decomp_lifted(uint32_t t0, uint32_t t1, int32_t& d1, int32_t& d2) {
+    const uint64_t r = lift_plus(t0, t1, kQ0, kQ1, kCarry1);
+    d1 = digit1(r);
+    d2 = digit2(r + (kCarry2 - kCarry1));
 }
-__device__ __forceinline__ void decomp2(uint32_t c0, uint32_t c1, const DevTables& T, int64_t& d1, int64_t& d2) {
-    decomp2(c0, c1, crt_consts(T), d1, d2);
+__device__ __forceinline__ void decomp2(uint32_t c0, uint32_t c1, const DevTables& T, int32_t& d1, int32_t& d2) {
+    decomp_lifted(csub(shoup_mul(c0, T.crt_c[0], T.crt_cp[0], kQ0), kQ0),
+                  csub(shoup_mul(c1, T.crt_c[1], T.crt_cp[1], kQ1), kQ1), d1, d2);
 }
-__device__ __forceinline__ uint32_t signed_res(int64_t d, uint32_t q) {
-    return d >= 0 ? (uint32_t)d : (uint32_t)((int64_t)q + d);
-}
+__device__ __forceinline__ uint32_t signed_res(int32_t d, uint32_t q) { return d >= 0 ? (uint32_t)d : q + (uint32_t)d; }
 
 }  // namespace ipb

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(256) qprep_kernel(const uint64_t* __restrict__
                                                     size_t rows, const DevTables* __restrict__ T,
                                                     uint8_t* __restrict__ kplanes, uint32_t* __restrict__ keys,
                                                     uint32_t* __restrict__ rgsw32, int y0) {
-    __shared__ __align__(16) uint32_t sbuf[2 * kN];
+    __shared__ __align__(16) uint32_t sbuf[kNttBuf], slots[kN];
     const int b = blockIdx.x, y = y0 + (int)blockIdx.y;
     const uint32_t t = threadIdx.x;
     const uint64_t* qr = qraw + (size_t)b * qstride;
@@ -60,8 +60,6 @@ __global__ void __launch_bounds__(256) qprep_kernel(const uint64_t* __restrict__
             st8(keys + ((size_t)(b * 2 + l) * kDeff + j) * kN + 8 * t, r);
             return;
         }
-        // Slots 8t .. 8t + 7 are this warp's own region of the NTT's second buffer.
-        uint32_t* slots = sbuf + kN;
         st8(slots + 8 * t, r);
         __syncthreads();
         const uint4 so = *reinterpret_cast<const uint4*>(T->slot_of + 8 * t);
@@ -169,7 +167,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(
     const uint32_t* __restrict__ tp_out, int g0,
     const uint32_t* __restrict__ df, const uint32_t* __restrict__ keys, size_t key_qstride,
     const DevTables* __restrict__ T, uint32_t* __restrict__ packed_b, size_t pb_qstride) {
-    __shared__ __align__(16) uint32_t sbuf[2 * kN];
+    __shared__ __align__(16) uint32_t sbuf[kNttBuf];
     const int g = g0 + (int)blockIdx.x, l = blockIdx.y, b = blockIdx.z;
     const uint32_t t = threadIdx.x;
     const LimbTables& L = T->limb[l];
@@ -209,7 +207,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(
 // two forward NTTs, the RGSW multiply-accumulate (digits of a meet the top
 // row, digits of b the bottom row) and a cross-group sum.  The chain never
 // leaves the SM; the reference spends ~12 launches per step.
-constexpr size_t kHornerSmem = 4 * kN * sizeof(uint2) + (4 * 2 * kN + 2 * 2 * kN + 2 * 2 * kN) * sizeof(uint32_t);
+constexpr size_t kHornerSmem = 4 * kN * sizeof(uint2) + (4 * kNttBuf + 2 * 2 * kN + 2 * 2 * kN) * sizeof(uint32_t);
 
 __global__ void __launch_bounds__(1024, 1) horner_kernel(const uint32_t* __restrict__ pre_a,
                                                          const uint32_t* __restrict__ packed_b, size_t pb_qstride,
@@ -219,8 +217,8 @@ __global__ void __launch_bounds__(1024, 1) horner_kernel(const uint32_t* __restr
                                                          size_t resp_qstride) {
     extern __shared__ __align__(16) uint8_t smem[];
     uint2* tw = reinterpret_cast<uint2*>(smem);                       // [fwd0|fwd1|inv0|inv1][N]
-    uint32_t* nbuf = reinterpret_cast<uint32_t*>(smem + 4 * kN * sizeof(uint2));  // [4][2][N]
-    uint32_t* xcoef = nbuf + 4 * 2 * kN;                              // [p][l][N]
+    uint32_t* nbuf = reinterpret_cast<uint32_t*>(smem + 4 * kN * sizeof(uint2));  // [4][kNttBuf]
+    uint32_t* xcoef = nbuf + 4 * kNttBuf;                             // [p][l][N]
     uint32_t* xch = xcoef + 2 * 2 * kN;                               // [p][l][N]
     const int ct = blockIdx.x, b = blockIdx.y;
     const int gp = threadIdx.x >> 8, p = gp >> 1, l = gp & 1;
@@ -237,7 +235,7 @@ __global__ void __launch_bounds__(1024, 1) horner_kernel(const uint32_t* __restr
     const uint32_t q = L.q;
     const uint2* twf = tw + l * kN;
     const uint2* twi = tw + (2 + l) * kN;
-    uint32_t* mybuf = nbuf + gp * 2 * kN;
+    uint32_t* mybuf = nbuf + gp * kNttBuf;
     const size_t start = (size_t)ct * d_act;
     const size_t len = (start + d_act <= groups) ? d_act : groups - start;
     const uint32_t* pbq = packed_b + (size_t)b * pb_qstride;
@@ -256,7 +254,7 @@ __global__ void __launch_bounds__(1024, 1) horner_kernel(const uint32_t* __restr
     uint32_t* xch_out = xch + ((1 - p) * 2 + l) * kN;
     const uint32_t* xch_in = xch + (p * 2 + l) * kN;
     for (long i = (long)len - 2; i >= 0; --i) {
-        ntt_inv(acc, mybuf, twi, q, L.inv_n, L.inv_n_p, t, bar);
+        ntt_inv(acc, mybuf, twi, q, L.scale_crt, t, bar);
 #pragma unroll
         for (int e = 0; e < 8; ++e) xc_me[t + 256 * e] = acc[e];
         __syncthreads();
@@ -264,10 +262,10 @@ __global__ void __launch_bounds__(1024, 1) horner_kernel(const uint32_t* __restr
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const uint32_t o = xc_ot[t + 256 * e];
-            int64_t s1, s2;
-            decomp2(l ? o : acc[e], l ? acc[e] : o, *T, s1, s2);
-            d0[e] = signed_res(s1, q);
-            d1[e] = signed_res(s2, q);
+            int32_t s1, s2;
+            decomp_lifted(l ? o : acc[e], l ? acc[e] : o, s1, s2);
+            d0[e] = q + (uint32_t)s1;
+            d1[e] = q + (uint32_t)s2;
         }
         ntt_fwd(d0, mybuf, twf, q, t, bar);
         ntt_fwd(d1, mybuf, twf, q, t, bar);
@@ -298,23 +296,53 @@ __global__ void __launch_bounds__(1024, 1) horner_kernel(const uint32_t* __restr
         *reinterpret_cast<ulonglong2*>(dst + e) = make_ulonglong2(acc[e], acc[e + 1]);
 }
 
+// floor(w 2^32 / q) for w < q, without a 64-bit division.
+__device__ __forceinline__ uint32_t shoup_factor(uint32_t w, uint64_t cr, uint32_t q) {
+    const uint64_t x = (uint64_t)w << 32;
+    const uint64_t f = __umul64hi(x, cr);  // low by at most 1
+    return (uint32_t)f + (x - f * q >= q ? 1u : 0u);
+}
+// Digit j + 1 as a residue in (0, 2q) from the lift terms of this limb and the
+// other one (q and q_oth their primes).
+__device__ __forceinline__ uint32_t digit_res(uint32_t own, uint32_t oth, uint32_t q, uint32_t q_oth, uint64_t carry,
+                                              int j) {
+    const uint64_t v = lift_plus(own, oth, q, q_oth, carry);
+    return q + (uint32_t)(j ? digit2(v) : digit1(v));
+}
+// Eight values per thread in shared memory, four and four N/2 words apart: the
+// lanes of a warp access consecutive 16 bytes.
+__device__ __forceinline__ void ld8_sh(const uint32_t* s, uint32_t t, uint32_t (&v)[8]) {
+    const uint4 a = *reinterpret_cast<const uint4*>(s + 4 * t), b = *reinterpret_cast<const uint4*>(s + kHalf + 4 * t);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void st8_sh(uint32_t* s, uint32_t t, const uint32_t (&v)[8]) {
+    *reinterpret_cast<uint4*>(s + 4 * t) = make_uint4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<uint4*>(s + kHalf + 4 * t) = make_uint4(v[4], v[5], v[6], v[7]);
+}
+
 // ------------------------------------------------------------------ horner (cluster)
 // The same chain on a cluster of four CTAs, CTA rank r = 2p + l owning
 // polynomial p (0 = a, 1 = b) in limb l.  Each CTA has two NTT groups:
-// group 0 holds the accumulator and runs the inverse NTT; both groups then
-// decompose (CRT needs the partner limb's coefficients) and transform one
-// gadget digit each; each digit is multiplied by the RGSW rows of its
-// polynomial (held in registers for the whole chain), the contribution to
-// the own polynomial stays local, the one to the other polynomial goes to
-// that CTA, and group 0 sums.  Remote data moves with st.async into the
-// receiver's shared memory and completes bytes on the receiver's mbarrier
-// (partner coefficients: 8 KB per step; other-poly contributions: 16 KB per
-// step), so the loop has no cluster-wide barrier.  Buffers alternate with
-// the step parity; a remote write for step t is issued only after its
-// receiver has finished reading the same buffer at step t - 2 (it depends on
-// data the receiver sent after that read).  Every wait is bounded.
-constexpr size_t kHornerClSmem =
-    2 * kN * sizeof(uint2) + (2 * 2 * kN + 2 * 2 * kN + 2 * 4 * kN) * sizeof(uint32_t) + 64;
+// group 0 holds the accumulator and runs the inverse NTT (scaled so that its
+// output is the CRT lift's term t_l, not the coefficient); both groups then
+// lift (which needs the partner limb's terms) and transform one gadget digit
+// each, and multiply it by the RGSW rows of their polynomial (held in
+// registers for the whole chain).  Group 0 sums the two digits' contributions
+// to the own polynomial, group 1 those to the other polynomial, which it
+// sends to that polynomial's CTA.  Values stay unreduced where the next
+// multiplication takes any word.
+// A step crosses SMs twice, 8 KB each way (partner terms, contributions): an
+// exchange between two SMs costs about 320 cycles and 50 more per KB with
+// st.async (bulk copies and plain remote stores measured 200-300 cycles more),
+// so the contributions are summed before they leave.  Data moves straight from
+// registers into the receiver's shared memory, in the order of the receiving
+// threads, and completes bytes on the receiver's mbarriers; the loop has no
+// cluster-wide barrier.  Received buffers alternate with the step parity; a
+// remote write for step t is issued only after its receiver has finished
+// reading the same buffer at step t - 2 (it depends on data the receiver sent
+// after that read).  Every wait is bounded.
+constexpr size_t kHornerClSmem = 2 * kN * sizeof(uint2) + (2 * kNttBuf + (1 + 2 + 2 + 2) * kN) * sizeof(uint32_t) + 64;
 
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -373,11 +401,13 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
     extern __shared__ __align__(16) uint8_t smem[];
     uint2* twf = reinterpret_cast<uint2*>(smem);
     uint2* twi = twf + kN;
-    uint32_t* nbuf = reinterpret_cast<uint32_t*>(twi + kN);   // [2 groups][2][N]
-    uint32_t* xc = nbuf + 2 * 2 * kN;                         // [parity][own | partner limb][N]
-    uint32_t* cin = xc + 2 * 2 * kN;                          // [parity][local j0 | local j1 | peer j0 | peer j1][N]
-    uint64_t* mbx = reinterpret_cast<uint64_t*>(cin + 2 * 4 * kN);  // [parity] partner coefficients
-    uint64_t* mbc = mbx + 2;                                         // [parity] other-poly contributions
+    uint32_t* nbuf = reinterpret_cast<uint32_t*>(twi + kN);         // [group][kNttBuf]
+    uint32_t* xown = nbuf + 2 * kNttBuf;                            // own lift terms, for group 1
+    uint32_t* xpart = xown + kN;                                    // [parity] partner limb's lift terms
+    uint32_t* cown = xpart + 2 * kN;                                // [group 0's to the other poly | group 1's to the own]
+    uint32_t* cin = cown + 2 * kN;                                  // [parity] the other poly's contribution
+    uint64_t* mbx = reinterpret_cast<uint64_t*>(cin + 2 * kN);      // [parity] partner terms
+    uint64_t* mbc = mbx + 2;                                        // [parity] contribution
     __shared__ volatile int abort_flag;
     const uint32_t rank = cluster_rank();
     const int p = (int)(rank >> 1), l = (int)(rank & 1);
@@ -386,9 +416,9 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
     const uint32_t t = threadIdx.x & 255;
     const int bar = 1 + gp;
     const LimbTables& L = T->limb[l];
-    const uint32_t q = L.q;
-    const uint32_t inv_n = L.inv_n, inv_n_p = L.inv_n_p;
-    const CrtK ck = crt_consts(*T);
+    const uint32_t q = L.q, q_oth = T->limb[1 - l].q;
+    const uint64_t carry = gp ? kCarry2 : kCarry1;
+    const NttScale scale = L.scale_crt;
     for (int i = threadIdx.x; i < kN; i += 512) { twf[i] = L.fwd[i]; twi[i] = L.inv[i]; }
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -413,79 +443,72 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
     uint32_t r_self_p[8], r_oth_p[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-        r_self_p[e] = (uint32_t)(((uint64_t)r_self[e] << 32) / q);
-        r_oth_p[e] = (uint32_t)(((uint64_t)r_oth[e] << 32) / q);
+        r_self_p[e] = shoup_factor(r_self[e], L.cr, q);
+        r_oth_p[e] = shoup_factor(r_oth[e], L.cr, q);
     }
-    uint32_t acc[8];
+    uint32_t acc[8] = {};
     uint32_t* const st_part = hr.state + (((size_t)b * (gridDim.x >> 2) + ct) * 4 + p * 2 + l) * kN;
     if (gp == 0) ld8((hr.i_first < 0 ? src_of(start + len - 1) : st_part) + 8 * t, acc);
     const long i_first = hr.i_first < 0 ? (long)len - 2 : (long)hr.i_first;
     cluster_sync_all();  // every CTA runs and its mbarriers are initialised before any remote access
-    const uint32_t peer_x = map_peer(xc, rank_limb);       // partner's xc base
-    const uint32_t peer_c = map_peer(cin, rank_poly);      // other poly CTA's cin base
+    const uint32_t peer_x = map_peer(xpart, rank_limb);
+    const uint32_t peer_c = map_peer(cin, rank_poly);
     const uint32_t peer_mbx = map_peer(mbx, rank_limb);
     const uint32_t peer_mbc = map_peer(mbc, rank_poly);
     int step = 0;
     for (long i = i_first; i >= (long)hr.i_last; --i, ++step) {
         const int par = step & 1;
         const uint32_t ph = (uint32_t)(step >> 1) & 1;
-        uint32_t* xown = xc + (par * 2 + 0) * kN;
-        const uint32_t* xpart = xc + (par * 2 + 1) * kN;
-        uint32_t* cp = cin + (size_t)par * 4 * kN;
         if (threadIdx.x == 0) {
             hb_expect(&mbx[par], kN * 4);
-            hb_expect(&mbc[par], 2 * kN * 4);
+            hb_expect(&mbc[par], kN * 4);
         }
         uint32_t pk[8];
         if (gp == 0) {
             ld8(src_of(start + (size_t)i) + 8 * t, pk);
-            ntt_inv(acc, nbuf, twi, q, inv_n, inv_n_p, t, bar);   // acc: index t + 256 e
-#pragma unroll
-            for (int e = 0; e < 8; ++e) xown[t + 256 * e] = acc[e];
+            ntt_inv(acc, nbuf, twi, q, scale, t, bar);   // acc: t_l at index t + 256 e
+            const uint32_t dst = peer_x + (uint32_t)(par * kN + 4 * t) * 4;
+            st_async4(dst, acc[0], acc[1], acc[2], acc[3], peer_mbx + 8 * par);
+            st_async4(dst + kHalf * 4, acc[4], acc[5], acc[6], acc[7], peer_mbx + 8 * par);
+            st8_sh(xown, t, acc);
         }
         __syncthreads();  // xown complete; abort_flag is read only here, after a block barrier,
                           // so every thread takes the same branch
         if (abort_flag) break;
-        if (gp == 0) {
-            // the partner's copy, sent as the contiguous block 8t..8t+7 (16-byte stores)
-            const uint32_t* src = xown + 8 * t;
-            const uint32_t dst = peer_x + (uint32_t)((par * 2 + 1) * kN + 8 * t) * 4;
-            st_async4(dst, src[0], src[1], src[2], src[3], peer_mbx + 8 * par);
-            st_async4(dst + 16, src[4], src[5], src[6], src[7], peer_mbx + 8 * par);
-        }
+        uint32_t d[8], v[8];
+        ld8_sh(xown, t, d);
         if (!hb_wait(&mbx[par], ph, err, 31)) abort_flag = 1;
-        uint32_t d[8];
+        ld8_sh(xpart + par * kN, t, v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) d[e] = digit_res(d[e], v[e], q, q_oth, carry, gp);
+        ntt_fwd_lazy(d, nbuf + gp * kNttBuf, twf, q, t, bar);
+        // The contribution that stays with this group, and the other one through
+        // shared memory ([0, 2q) each).
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const uint32_t own = xown[t + 256 * e], oth = xpart[t + 256 * e];
-            int64_t s1, s2;
-            decomp2(l ? oth : own, l ? own : oth, ck, s1, s2);
-            d[e] = signed_res(gp ? s2 : s1, q);
+            const uint32_t es = shoup_mul(d[e], r_self[e], r_self_p[e], q);
+            const uint32_t eo = shoup_mul(d[e], r_oth[e], r_oth_p[e], q);
+            d[e] = gp ? eo : es;
+            v[e] = gp ? es : eo;
         }
-        ntt_fwd(d, nbuf + gp * 2 * kN, twf, q, t, bar);
-        uint32_t es[8], eo[8];
+        st8_sh(cown + gp * kN, t, v);
+        __syncthreads();
+        ld8_sh(cown + (1 - gp) * kN, t, v);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            es[e] = csub(shoup_mul(d[e], r_self[e], r_self_p[e], q), q);
-            eo[e] = csub(shoup_mul(d[e], r_oth[e], r_oth_p[e], q), q);
-        }
-        st8(cp + (size_t)gp * kN + 8 * t, es);
-        const uint32_t dstc = peer_c + (uint32_t)((size_t)par * 4 * kN + (size_t)(2 + gp) * kN + 8 * t) * 4;
-        st_async4(dstc, eo[0], eo[1], eo[2], eo[3], peer_mbc + 8 * par);
-        st_async4(dstc + 16, eo[4], eo[5], eo[6], eo[7], peer_mbc + 8 * par);
-        __syncthreads();  // local contributions complete
-        if (gp == 0) {
+        for (int e = 0; e < 8; ++e) d[e] += v[e];
+        if (gp) {
+            const uint32_t dst = peer_c + (uint32_t)(par * kN + 4 * t) * 4;
+            st_async4(dst, d[0], d[1], d[2], d[3], peer_mbc + 8 * par);
+            st_async4(dst + kHalf * 4, d[4], d[5], d[6], d[7], peer_mbc + 8 * par);
+        } else {
             if (!hb_wait(&mbc[par], ph, err, 32)) abort_flag = 1;
-            uint32_t v0[8], v1[8], w0[8], w1[8];
-            ld8(cp + 8 * t, v0);
-            ld8(cp + kN + 8 * t, v1);
-            ld8(cp + 2 * kN + 8 * t, w0);
-            ld8(cp + 3 * kN + 8 * t, w1);
+            ld8_sh(cin + par * kN, t, v);
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-                acc[e] = add_mod(add_mod(add_mod(v0[e], v1[e], q), add_mod(w0[e], w1[e], q), q), pk[e], q);
+            for (int e = 0; e < 8; ++e) acc[e] = red2(d[e] + v[e] + pk[e], q);  // of at most 9q
         }
     }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = csub(acc[e], q);
     if (gp == 0 && hr.i_last == 0) {
         uint64_t* dst = resp + (size_t)b * resp_qstride + ((size_t)ct * 4 + p * 2 + l) * kN + 8 * t;
 #pragma unroll
@@ -501,20 +524,20 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
 // The chain on a cluster of eight CTAs of 256 threads, CTA rank
 // r = 4p + 2l + j owning polynomial p, limb l and gadget digit j.  Both digit
 // CTAs of (p, l) hold the same accumulator and run its inverse NTT; each
-// sends its coefficients to the other limb's CTA of the same digit (CRT needs
-// both limbs), decomposes and forward-transforms only its digit, and
+// sends its lift terms to the other limb's CTA of the same digit (the lift
+// needs both limbs), decomposes and forward-transforms only its digit, and
 // multiplies it by the RGSW rows of its polynomial.  The contribution to its
 // own polynomial goes to the sibling digit CTA, the one to the other
 // polynomial to both digit CTAs of that polynomial; every CTA then sums its
-// own, its sibling's and the two other-polynomial contributions (modular
-// sums of canonical residues: both siblings get the same accumulator).
+// own, its sibling's and the two other-polynomial contributions (both
+// siblings add the same residues: their accumulators agree mod q).
 // Remote data moves with st.async and completes on the receiver's
-// transaction mbarriers (8 KB of coefficients, 24 KB of contributions per
+// transaction mbarriers (8 KB of lift terms, 24 KB of contributions per
 // step); buffers alternate with the step parity, and every remote write for
 // step t depends on data its receiver sent after reading the same buffer at
 // step t - 2.  Half the warps per SM of the 4-CTA version, twice the SMs.
 constexpr size_t kHornerCl8Smem =
-    2 * kN * sizeof(uint2) + (2 * kN + 2 * 2 * kN + 2 * 4 * kN) * sizeof(uint32_t) + 64;
+    2 * kN * sizeof(uint2) + (kNttBuf + 2 * kN + 2 * 3 * kN) * sizeof(uint32_t) + 64;
 
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     horner_cl8_kernel(const uint32_t* __restrict__ pre_a, const uint32_t* __restrict__ packed_b, size_t pb_qstride,
@@ -523,10 +546,10 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     extern __shared__ __align__(16) uint8_t smem[];
     uint2* twf = reinterpret_cast<uint2*>(smem);
     uint2* twi = twf + kN;
-    uint32_t* nbuf = reinterpret_cast<uint32_t*>(twi + kN);  // [2][N] NTT scratch
-    uint32_t* xc = nbuf + 2 * kN;                            // [parity][own | partner limb][N]
-    uint32_t* cin = xc + 2 * 2 * kN;                         // [parity][own | sibling | other j0 | other j1][N]
-    uint64_t* mbx = reinterpret_cast<uint64_t*>(cin + 2 * 4 * kN);  // [parity] partner coefficients
+    uint32_t* nbuf = reinterpret_cast<uint32_t*>(twi + kN);  // NTT scratch
+    uint32_t* xc = nbuf + kNttBuf;                           // [parity] partner limb's lift terms
+    uint32_t* cin = xc + 2 * kN;                             // [parity][sibling | other j0 | other j1]
+    uint64_t* mbx = reinterpret_cast<uint64_t*>(cin + 2 * 3 * kN);  // [parity] partner terms
     uint64_t* mbc = mbx + 2;                                         // [parity] contributions
     __shared__ volatile int abort_flag;
     const uint32_t rank = cluster_rank();
@@ -535,8 +558,9 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     const uint32_t t = threadIdx.x;
     const LimbTables& L = T->limb[l];
     const uint32_t q = L.q;
-    const uint32_t inv_n = L.inv_n, inv_n_p = L.inv_n_p;
-    const CrtK ck = crt_consts(*T);
+    const uint32_t q_oth = T->limb[1 - l].q;
+    const uint64_t carry = j ? kCarry2 : kCarry1;
+    const NttScale scale = L.scale_crt;
     for (int i = threadIdx.x; i < kN; i += 256) { twf[i] = L.fwd[i]; twi[i] = L.inv[i]; }
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -562,8 +586,8 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     uint32_t r_self_p[8], r_oth_p[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-        r_self_p[e] = (uint32_t)(((uint64_t)r_self[e] << 32) / q);
-        r_oth_p[e] = (uint32_t)(((uint64_t)r_oth[e] << 32) / q);
+        r_self_p[e] = shoup_factor(r_self[e], L.cr, q);
+        r_oth_p[e] = shoup_factor(r_oth[e], L.cr, q);
     }
     uint32_t acc[8];
     uint32_t* const st_part = hr.state + (((size_t)b * (gridDim.x >> 3) + ct) * 4 + p * 2 + l) * kN;
@@ -579,59 +603,57 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     for (long i = i_first; i >= (long)hr.i_last; --i, ++step) {
         const int par = step & 1;
         const uint32_t ph = (uint32_t)(step >> 1) & 1;
-        uint32_t* xown = xc + (par * 2 + 0) * kN;
-        const uint32_t* xpart = xc + (par * 2 + 1) * kN;
-        uint32_t* cp = cin + (size_t)par * 4 * kN;
+        const uint32_t* xpart = xc + par * kN;
+        uint32_t* cp = cin + (size_t)par * 3 * kN;
         if (threadIdx.x == 0) {
             hb_expect(&mbx[par], kN * 4);
             hb_expect(&mbc[par], 3 * kN * 4);
         }
         uint32_t pk[8];
         ld8(src_of(start + (size_t)i) + 8 * t, pk);
-        ntt_inv(acc, nbuf, twi, q, inv_n, inv_n_p, t, 0);   // acc: index t + 256 e
-#pragma unroll
-        for (int e = 0; e < 8; ++e) xown[t + 256 * e] = acc[e];
-        __syncthreads();  // xown complete; abort_flag is read only here, after a block barrier
-        if (abort_flag) break;
+        ntt_inv_head(acc, nbuf, twi, q, t, 0);
+        // Read between the transform's two block barriers: the first follows
+        // every write of the previous step, the second precedes this step's,
+        // so every thread takes the same branch.
+        const int stop = abort_flag;
+        ntt_inv_tail(acc, nbuf, twi, q, scale, t, 0);   // acc: t_l at index t + 256 e
+        if (stop) break;
         {
-            const uint32_t* src = xown + 8 * t;
-            const uint32_t dst = peer_x + (uint32_t)((par * 2 + 1) * kN + 8 * t) * 4;
-            st_async4(dst, src[0], src[1], src[2], src[3], peer_mbx + 8 * par);
-            st_async4(dst + 16, src[4], src[5], src[6], src[7], peer_mbx + 8 * par);
+            const uint32_t dst = peer_x + (uint32_t)(par * kN + 4 * t) * 4;
+            st_async4(dst, acc[0], acc[1], acc[2], acc[3], peer_mbx + 8 * par);
+            st_async4(dst + kHalf * 4, acc[4], acc[5], acc[6], acc[7], peer_mbx + 8 * par);
         }
         if (!hb_wait(&mbx[par], ph, err, 33)) abort_flag = 1;
         uint32_t d[8];
+        ld8_sh(xpart, t, d);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const uint32_t own = acc[e], oth = xpart[t + 256 * e];  // own: still in registers
-            int64_t s1, s2;
-            decomp2(l ? oth : own, l ? own : oth, ck, s1, s2);
-            d[e] = signed_res(j ? s2 : s1, q);
-        }
-        ntt_fwd(d, nbuf, twf, q, t, 0);
+        for (int e = 0; e < 8; ++e) d[e] = digit_res(acc[e], d[e], q, q_oth, carry, j);
+        ntt_fwd_lazy(d, nbuf, twf, q, t, 0);
         uint32_t es[8], eo[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            es[e] = csub(shoup_mul(d[e], r_self[e], r_self_p[e], q), q);
-            eo[e] = csub(shoup_mul(d[e], r_oth[e], r_oth_p[e], q), q);
+        for (int e = 0; e < 8; ++e) {  // [0, 2q)
+            es[e] = shoup_mul(d[e], r_self[e], r_self_p[e], q);
+            eo[e] = shoup_mul(d[e], r_oth[e], r_oth_p[e], q);
         }
-        const uint32_t off = (uint32_t)((size_t)par * 4 * kN + 8 * t) * 4;
-        st_async4(sib_c + off + kN * 4, es[0], es[1], es[2], es[3], sib_mbc + 8 * par);
-        st_async4(sib_c + off + kN * 4 + 16, es[4], es[5], es[6], es[7], sib_mbc + 8 * par);
-        const uint32_t off_o = off + (uint32_t)(2 + j) * kN * 4;
-        st_async4(o0_c + off_o, eo[0], eo[1], eo[2], eo[3], o0_mbc + 8 * par);
-        st_async4(o0_c + off_o + 16, eo[4], eo[5], eo[6], eo[7], o0_mbc + 8 * par);
-        st_async4(o1_c + off_o, eo[0], eo[1], eo[2], eo[3], o1_mbc + 8 * par);
-        st_async4(o1_c + off_o + 16, eo[4], eo[5], eo[6], eo[7], o1_mbc + 8 * par);
+        const uint32_t off = (uint32_t)((size_t)par * 3 * kN + 4 * t) * 4;
+        const uint32_t off_o = off + (uint32_t)(1 + j) * kN * 4;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t o = h * kHalf * 4;
+            st_async4(sib_c + off + o, es[4 * h], es[4 * h + 1], es[4 * h + 2], es[4 * h + 3], sib_mbc + 8 * par);
+            st_async4(o0_c + off_o + o, eo[4 * h], eo[4 * h + 1], eo[4 * h + 2], eo[4 * h + 3], o0_mbc + 8 * par);
+            st_async4(o1_c + off_o + o, eo[4 * h], eo[4 * h + 1], eo[4 * h + 2], eo[4 * h + 3], o1_mbc + 8 * par);
+        }
         if (!hb_wait(&mbc[par], ph, err, 34)) abort_flag = 1;
         uint32_t v1[8], w0[8], w1[8];
-        ld8(cp + kN + 8 * t, v1);
-        ld8(cp + 2 * kN + 8 * t, w0);
-        ld8(cp + 3 * kN + 8 * t, w1);
+        ld8_sh(cp, t, v1);
+        ld8_sh(cp + kN, t, w0);
+        ld8_sh(cp + 2 * kN, t, w1);
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-            acc[e] = add_mod(add_mod(add_mod(es[e], v1[e], q), add_mod(w0[e], w1[e], q), q), pk[e], q);
+        for (int e = 0; e < 8; ++e) acc[e] = red2(es[e] + v1[e] + w0[e] + w1[e] + pk[e], q);  // sum < 9q
     }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = csub(acc[e], q);
     if (j == 0 && hr.i_last == 0) {
         uint64_t* dst = resp + (size_t)b * resp_qstride + ((size_t)ct * 4 + p * 2 + l) * kN + 8 * t;
 #pragma unroll
@@ -658,11 +680,11 @@ __global__ void __launch_bounds__(1024) ntt_batch_kernel(uint32_t* polys, size_t
     if (!inverse) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) r[e] = pp[t + 256 * e];
-        ntt_fwd(r, nb + gp * 2 * kN, L.fwd, L.q, t, 1 + gp);
+        ntt_fwd(r, nb + gp * kNttBuf, L.fwd, L.q, t, 1 + gp);
         st8(pp + 8 * t, r);
     } else {
         ld8(pp + 8 * t, r);
-        ntt_inv(r, nb + gp * 2 * kN, L.inv, L.q, L.inv_n, L.inv_n_p, t, 1 + gp);
+        ntt_inv(r, nb + gp * kNttBuf, L.inv, L.q, L.scale_n, t, 1 + gp);
 #pragma unroll
         for (int e = 0; e < 8; ++e) pp[t + 256 * e] = r[e];
     }
@@ -673,7 +695,7 @@ __global__ void decomp_kernel(const uint32_t* __restrict__ in, uint32_t* __restr
     const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n * kN) return;
     const size_t i = k / kN, x = k % kN;
-    int64_t s1, s2;
+    int32_t s1, s2;
     decomp2(in[(i * 2) * kN + x], in[(i * 2 + 1) * kN + x], *T, s1, s2);
     uint32_t* o = out + i * kDeff * 2 * kN;
     o[(0 * 2 + 0) * kN + x] = signed_res(s1, kQ0);
@@ -849,7 +871,7 @@ cudaError_t launch_horner_cluster8(const uint32_t* pre_a, const uint32_t* packed
 cudaError_t launch_ntt_batch(uint32_t* polys, size_t n, int limb_run, bool inverse, const DevTables* T,
                              cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    const size_t smem = 4 * 2 * kN * sizeof(uint32_t);
+    const size_t smem = 4 * kNttBuf * sizeof(uint32_t);
     cudaError_t e = allow_max_smem(ntt_batch_kernel);
     if (e) return e;
     ntt_batch_kernel<<<(unsigned)((n + 3) / 4), 1024, smem, s>>>(polys, n, limb_run, inverse, T);

@@ -135,15 +135,15 @@ __global__ void __launch_bounds__(256) encode_pass_kernel(const uint16_t* __rest
 // column-major in shared memory, forward-NTT each column, multiply by the
 // CRS poly crs_r and accumulate (all in registers, L4 layout).  The output
 // row p of V holds N^-1 * acc_j[N-1-p] for the tile's columns j.
-constexpr size_t kASideSmem = 8 * kN * sizeof(uint16_t) + 4 * 2 * kN * sizeof(uint32_t) + 2 * kN * sizeof(uint2);
+constexpr size_t kASideSmem = 8 * kN * sizeof(uint16_t) + 4 * kNttBuf * sizeof(uint32_t) + 2 * kN * sizeof(uint2);
 
 __global__ void __launch_bounds__(1024, 1) a_side_kernel(const uint16_t* __restrict__ db, size_t rows, size_t cols,
                                                          size_t g, const uint32_t* __restrict__ crs,
                                                          const DevTables* __restrict__ T, uint32_t* __restrict__ V) {
     extern __shared__ __align__(16) uint8_t smem[];
     uint16_t* tile = reinterpret_cast<uint16_t*>(smem);                               // [8][N]
-    uint32_t* nbuf = reinterpret_cast<uint32_t*>(smem + 8 * kN * sizeof(uint16_t));  // [4][2][N]
-    uint2* tw = reinterpret_cast<uint2*>(nbuf + 4 * 2 * kN);                           // [2][N]
+    uint32_t* nbuf = reinterpret_cast<uint32_t*>(smem + 8 * kN * sizeof(uint16_t));  // [4][kNttBuf]
+    uint2* tw = reinterpret_cast<uint2*>(nbuf + 4 * kNttBuf);                          // [2][N]
     const int tid = threadIdx.x, gp = tid >> 8;
     const uint32_t t = tid & 255;
     const size_t j0 = (size_t)blockIdx.x * 8;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(1024, 1) a_side_kernel(const uint16_t* __restr
             uint32_t x[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) x[e] = tile[c * kN + t + 256 * e];
-            ntt_fwd(x, nbuf + gp * 2 * kN, tw + l * kN, L.q, t, 1 + gp);
+            ntt_fwd(x, nbuf + gp * kNttBuf, tw + l * kN, L.q, t, 1 + gp);
             uint32_t a[8];
             ld8(crs + (r * 2 + l) * kN + 8 * t, a);
 #pragma unroll
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(1024) col_ntt_kernel(const uint32_t* __restric
     uint32_t x[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) x[e] = src[t + 256 * e];
-    ntt_fwd(x, nb + gp * 2 * kN, L.fwd, L.q, t, 1 + gp);
+    ntt_fwd(x, nb + gp * kNttBuf, L.fwd, L.q, t, 1 + gp);
     st8(Tout + ((size_t)l * kN + p) * kN + 8 * t, x);
 }
 
@@ -238,15 +238,15 @@ __global__ void __launch_bounds__(256) embed_gather_kernel(const uint32_t* __res
 // one CTA barrier per step), decompose, NTT the two digits, write
 // D[limb][s][digit], MAC against K5 permuted by 5^(1022-s) (or its
 // conjugate) and subtract from a_post[k-1].
-constexpr size_t kCollapseASmem = (2 * 2 * kN + 2 * 2 * kN + 2 * kDeff * kN) * sizeof(uint32_t);
+constexpr size_t kCollapseASmem = (2 * kNttBuf + 2 * 2 * kN + 2 * kDeff * kN) * sizeof(uint32_t);
 
 __global__ void __launch_bounds__(512) collapse_a_kernel(const uint32_t* __restrict__ a_post, size_t ap_gstride,
                                                          const uint32_t* __restrict__ k5,
                                                          const DevTables* __restrict__ T, uint32_t* __restrict__ dp,
                                                          uint32_t* __restrict__ dm, uint32_t* __restrict__ ends) {
     extern __shared__ __align__(16) uint32_t sm[];
-    uint32_t* nbuf = sm;                      // [2][2][N]
-    uint32_t* xc = nbuf + 2 * 2 * kN;         // [parity][limb][N]
+    uint32_t* nbuf = sm;                      // [2][kNttBuf]
+    uint32_t* xc = nbuf + 2 * kNttBuf;        // [parity][limb][N]
     uint32_t* sk = xc + 2 * 2 * kN;           // [limb][digit][N]
     const int g = blockIdx.x, dir = blockIdx.y;
     const int l = threadIdx.x >> 8;
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(512) collapse_a_kernel(const uint32_t* __restr
     const uint32_t* skl1 = sk + (l * kDeff + 1) * kN;
     for (int s = 0; s < kSteps; ++s) {
         const int k = kHalf - 1 - s;
-        ntt_inv(st, nbuf + l * 2 * kN, L.inv, q, L.inv_n, L.inv_n_p, t, bar);
+        ntt_inv(st, nbuf + l * kNttBuf, L.inv, q, L.scale_crt, t, bar);
         uint32_t* xme = xc + ((s & 1) * 2 + l) * kN;
         const uint32_t* xot = xc + ((s & 1) * 2 + (1 - l)) * kN;
 #pragma unroll
@@ -278,13 +278,13 @@ __global__ void __launch_bounds__(512) collapse_a_kernel(const uint32_t* __restr
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const uint32_t o = xot[t + 256 * e];
-            int64_t s1, s2;
-            decomp2(l ? o : st[e], l ? st[e] : o, *T, s1, s2);
-            d0[e] = signed_res(s1, q);
-            d1[e] = signed_res(s2, q);
+            int32_t s1, s2;
+            decomp_lifted(l ? o : st[e], l ? st[e] : o, s1, s2);
+            d0[e] = q + (uint32_t)s1;
+            d1[e] = q + (uint32_t)s2;
         }
-        ntt_fwd(d0, nbuf + l * 2 * kN, L.fwd, q, t, bar);
-        ntt_fwd(d1, nbuf + l * 2 * kN, L.fwd, q, t, bar);
+        ntt_fwd(d0, nbuf + l * kNttBuf, L.fwd, q, t, bar);
+        ntt_fwd(d1, nbuf + l * kNttBuf, L.fwd, q, t, bar);
         st8(Dout + (((size_t)l * kSteps + s) * kDeff + 0) * kN + 8 * t, d0);
         st8(Dout + (((size_t)l * kSteps + s) * kDeff + 1) * kN + 8 * t, d1);
         const uint32_t tt = dir ? ((2 * kN - tks) & (2 * kN - 1)) : tks;
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(512) collapse_final_kernel(const uint32_t* __r
                                                              const uint32_t* __restrict__ kn1,
                                                              const DevTables* __restrict__ T,
                                                              uint32_t* __restrict__ df, uint32_t* __restrict__ pre_a) {
-    __shared__ __align__(16) uint32_t nbuf[2 * 2 * kN];
+    __shared__ __align__(16) uint32_t nbuf[2 * kNttBuf];
     __shared__ __align__(16) uint32_t xc[2 * kN];
     const int g = blockIdx.x;
     const int l = threadIdx.x >> 8;
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(512) collapse_final_kernel(const uint32_t* __r
     const uint32_t q = L.q;
     uint32_t st[8];
     ld8(ends + (((size_t)g * 2 + 1) * 2 + l) * kN + 8 * t, st);
-    ntt_inv(st, nbuf + l * 2 * kN, L.inv, q, L.inv_n, L.inv_n_p, t, bar);
+    ntt_inv(st, nbuf + l * kNttBuf, L.inv, q, L.scale_crt, t, bar);
 #pragma unroll
     for (int e = 0; e < 8; ++e) xc[l * kN + t + 256 * e] = st[e];
     __syncthreads();
@@ -325,13 +325,13 @@ __global__ void __launch_bounds__(512) collapse_final_kernel(const uint32_t* __r
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         const uint32_t o = xc[(1 - l) * kN + t + 256 * e];
-        int64_t s1, s2;
-        decomp2(l ? o : st[e], l ? st[e] : o, *T, s1, s2);
-        d0[e] = signed_res(s1, q);
-        d1[e] = signed_res(s2, q);
+        int32_t s1, s2;
+        decomp_lifted(l ? o : st[e], l ? st[e] : o, s1, s2);
+        d0[e] = q + (uint32_t)s1;
+        d1[e] = q + (uint32_t)s2;
     }
-    ntt_fwd(d0, nbuf + l * 2 * kN, L.fwd, q, t, bar);
-    ntt_fwd(d1, nbuf + l * 2 * kN, L.fwd, q, t, bar);
+    ntt_fwd(d0, nbuf + l * kNttBuf, L.fwd, q, t, bar);
+    ntt_fwd(d1, nbuf + l * kNttBuf, L.fwd, q, t, bar);
     st8(df + (((size_t)g * 2 + l) * kDeff + 0) * kN + 8 * t, d0);
     st8(df + (((size_t)g * 2 + l) * kDeff + 1) * kN + 8 * t, d1);
     uint32_t sv[8], k0[8], k1[8], o[8];
@@ -369,7 +369,7 @@ cudaError_t launch_a_side(const uint16_t* db, size_t rows, size_t cols, size_t g
 }
 
 cudaError_t launch_col_ntt(const uint32_t* V, const DevTables* T, uint32_t* Tout, cudaStream_t s) {
-    const size_t smem = 4 * 2 * kN * sizeof(uint32_t);
+    const size_t smem = 4 * kNttBuf * sizeof(uint32_t);
     cudaError_t e = allow_max_smem(col_ntt_kernel);
     if (e) return e;
     col_ntt_kernel<<<dim3(kN / 4, 2), 1024, smem, s>>>(V, T, Tout);
