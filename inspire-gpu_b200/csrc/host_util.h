@@ -50,4 +50,23 @@ inline cudaError_t allow_max_smem(K* kernel, size_t* max_dynamic = nullptr) {
     return allow_max_dynamic_smem(reinterpret_cast<const void*>(kernel), max_dynamic);
 }
 
+// Launch with programmatic stream serialization (see after_previous() in
+// ipb_common.cuh).  Back-to-back kernels of one answer: 2-4 us less each on the
+// small databases, where launch gaps and prologues are most of the time.
+template <class... P, class... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                     A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 }  // namespace ipb

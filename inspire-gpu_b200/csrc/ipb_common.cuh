@@ -102,6 +102,17 @@ __device__ __forceinline__ uint32_t perm_from_odd(uint32_t t, uint32_t odd) {
     return brev11((e - 1) >> 1);
 }
 
+// ------------------------------------------------------------ launch overlap
+// Kernels of the answer pipeline launch with programmatic stream
+// serialization: the next one may start, and run its prologue, while this one
+// is still running.  after_previous() waits until the previous kernel of the
+// stream has completed and its writes are visible; every read or write of
+// memory that another kernel touches comes after it.  let_next_start() is
+// called first thing, so the next kernel's blocks take whatever this one leaves
+// free.  Both are no-ops in an ordinary launch.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------ barriers
 __device__ __forceinline__ void gsync(int bar) {
     if (bar == 0) __syncthreads();

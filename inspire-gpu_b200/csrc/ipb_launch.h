@@ -13,14 +13,15 @@ struct DevTables;
 // ---------------------------------------------------------------- online
 // Flat per-query device input (u64, the capi.h flat query layout):
 //   [b0: rows][b1: rows][ksk5: blk][kskneg1: blk][rgsw: 4 blk],  blk = 2*2*N.
-// qprep: KSK5 byte planes kplanes [q][limb][byte][4096] (tensorpass_tc.cu),
-// KSK-1 keys [q][limb][digit][N] NTT form, rgsw32 [q][4][digit][limb][N].
-cudaError_t launch_qprep(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T,
-                         uint8_t* kplanes, uint32_t* keys, uint32_t* rgsw32, int nq, cudaStream_t s);
-// Only some of it: parts 1 = the keys, 2 = the RGSW parts, 3 = both.
-cudaError_t launch_qprep_parts(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T,
-                               uint8_t* kplanes, uint32_t* keys, uint32_t* rgsw32, int nq, int parts,
-                               cudaStream_t s);
+// qprep, any of three parts: kPrepKeys writes KSK5's byte planes kplanes
+// [q][limb][byte][4096] (tensorpass_tc.cu) and KSK-1 as keys
+// [q][limb][digit][N] in NTT form, kPrepRgsw rgsw32 [q][4][digit][limb][N],
+// kPrepPlanes the tensor-core mat-vec's planes[7q + k][rows] (byte k of
+// CRT(b_0, b_1) < q0 q1; rows a multiple of 1024).  Pointers of parts that are
+// not asked for may be null.
+constexpr int kPrepKeys = 1, kPrepRgsw = 2, kPrepPlanes = 4;
+cudaError_t launch_qprep(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T, uint8_t* kplanes,
+                         uint32_t* keys, uint32_t* rgsw32, uint8_t* planes, int nq, int parts, cudaStream_t s);
 
 // Mat-vec row-split partials part[q][chunk][limb][cols] for nq <= 4 queries
 // sharing one DB stream.  chunks must divide rows.
@@ -28,9 +29,7 @@ cudaError_t launch_matvec(const uint16_t* db, size_t rows, size_t cols, int chun
                           const uint64_t* qraw, size_t qstride, const DevTables* T,
                           uint32_t* part, size_t part_qstride, int nq, cudaStream_t s);
 
-// Tensor-core mat-vec (tcgen05 kind::i8).  qplanes writes the CRT byte
-// planes planes[7q + k][rows] of nq queries (byte k of CRT(b_0, b_1) < q0 q1);
-// launch_matvec_tc runs nq <= 32 queries whose planes start at `planes`
+// Tensor-core mat-vec (tcgen05 kind::i8): launch_matvec_tc runs nq <= 32 queries whose planes start at `planes`
 // (mv_tc_planes_offset of the first query), writing
 // part[q][chunk][limb][cols] with chunks = rows / kchunk_rows.  *err
 // receives a nonzero code if a pipeline wait times out.
@@ -39,10 +38,8 @@ size_t mv_tc_planes_offset(size_t first_query, size_t rows);
 int matvec_tc_kchunk_rows(size_t rows, size_t cols, int num_sms);
 // DB columns per mat-vec work item (one m' tile of lo and hi bytes).
 int matvec_tc_item_cols();
-cudaError_t launch_qplanes(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T,
-                           uint8_t* planes, int nq, cudaStream_t s);
-// tiles: a device counter the launch zeroes and the kernel's CTAs draw work
-// items from (one per concurrently running launch).
+// tiles: two device words, zero between launches, that the kernel's CTAs draw
+// work items from (one pair per concurrently running launch).
 cudaError_t launch_matvec_tc(const uint16_t* db, size_t rows, size_t cols, const uint8_t* planes, int nq,
                              const DevTables* T, uint32_t* part, size_t part_qstride, int* err, unsigned* tiles,
                              int num_sms, int kchunk_rows, cudaStream_t s);

@@ -124,8 +124,8 @@ extern "C" int ipir_b200_matvec_noalloc(const uint16_t* db, size_t rows, size_t 
     int* err = reinterpret_cast<int*>(base + kNoAllocErrOff);
     unsigned* tiles = reinterpret_cast<unsigned*>(base + kNoAllocErrOff + 128);  // same 256-byte slot
     uint8_t* planes = base + kNoAllocPlanesOff;
-    e = cudaMemsetAsync(err, 0, sizeof(int), s);  // the array keeps the last call's contents
-    if (e == cudaSuccess) e = launch_qplanes(queries, 2 * rows, rows, T, planes, (int)count, s);
+    e = cudaMemsetAsync(err, 0, kNoAllocPlanesOff - kNoAllocErrOff, s);  // the array keeps the last call's contents
+    if (e == cudaSuccess) e = launch_qprep(queries, 2 * rows, rows, T, nullptr, nullptr, nullptr, planes, (int)count, kPrepPlanes, s);
     // rows <= 32768: one exact K-chunk, so the kernel writes the result directly.
     if (e == cudaSuccess)
         e = launch_matvec_tc(db, rows, cols, planes, (int)count, T, out, 2 * cols, err, tiles, sms, (int)rows, s);

@@ -24,8 +24,8 @@
 // bounded and reports a timeout through *err instead of hanging.
 //
 // Work items (m'-tile, K-chunk) are handed out dynamically: the producer
-// thread takes the next item from a per-launch atomic counter (zeroed by the
-// launcher) and publishes it to the MMA thread and the epilogue through a
+// thread takes the next item from an atomic counter (zero between launches: a
+// launch's last CTA puts it back) and publishes it to the MMA thread and the epilogue through a
 // ring of kRing shared slots; -1 ends the sequence.  SMs that other kernels
 // hold when this one starts (the previous batch's Horner, another lane)
 // simply take fewer items instead of delaying the whole pass.
@@ -69,7 +69,7 @@ struct TcParams {
     int acc_stages;
     uint32_t tmem_cols;
     int* err;
-    unsigned* tiles;       // work-item counter, zero at launch
+    unsigned* tiles;       // [0] work-item counter, [1] CTAs done: both zero between launches
     const DevTables* T;
     int has_qmap;          // output row of pass query q: qmap[q] (else q)
     uint8_t qmap[32];
@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(256, 1) mv_tc_kernel(const __grid_constant__ C
     __shared__ uint64_t ifull[kRing], iempty[kRing];
     __shared__ uint64_t mma_done;  // the MMA issuer's final commit: all its MMAs have completed
 
+    let_next_start();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(256, 1) mv_tc_kernel(const __grid_constant__ C
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    after_previous();
     const uint32_t tmem_base = *tmem_slot;
     const int n_items = P.n_mtiles * P.n_kchunks;
     const int ktiles = P.kchunk_rows / kKT;
@@ -291,38 +293,10 @@ __global__ void __launch_bounds__(256, 1) mv_tc_kernel(const __grid_constant__ C
     }
     tc_fence_before();
     __syncthreads();
+    if (threadIdx.x == 0) release_counter(P.tiles);
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(P.tmem_cols));
-    }
-}
-
-// CRT byte planes of the queries: planes[7q + k][rows] = byte k of
-// B[i] = CRT(b_0[i] mod q0, b_1[i] mod q1) < q0 q1
-// (Garner: b_1 + q1 ((b_0 - b_1) q1^-1 mod q0)).
-__global__ void __launch_bounds__(256) qplanes_kernel(const uint64_t* __restrict__ qraw, size_t qstride, size_t rows,
-                                                      const DevTables* __restrict__ T,
-                                                      uint8_t* __restrict__ planes) {
-    const int q = blockIdx.y;
-    const size_t i4 = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
-    if (i4 >= rows) return;
-    const uint64_t* src = qraw + (size_t)q * qstride;
-    uint64_t B[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const uint32_t v0 = mod_u64(src[i4 + c], T->limb[0].cr, kQ0);
-        const uint32_t v1 = mod_u64(src[rows + i4 + c], T->limb[1].cr, kQ1);
-        const uint32_t v1r = v1 >= kQ0 ? v1 - kQ0 : v1;
-        const uint32_t diff = v0 >= v1r ? v0 - v1r : v0 + kQ0 - v1r;
-        const uint32_t h = mod_u64((uint64_t)diff * T->crt_c[0], T->limb[0].cr, kQ0);
-        B[c] = (uint64_t)v1 + (uint64_t)kQ1 * h;
-    }
-#pragma unroll
-    for (int k = 0; k < kPlanes; ++k) {
-        uint32_t packed = 0;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) packed |= (uint32_t)((B[c] >> (8 * k)) & 0xFFu) << (8 * c);
-        *reinterpret_cast<uint32_t*>(planes + ((size_t)kPlanes * q + k) * rows + i4) = packed;
     }
 }
 
@@ -336,6 +310,7 @@ __global__ void __launch_bounds__(256) mv_chunk_reduce_kernel(const uint32_t* __
     const int l = (int)(idx / cols);
     const size_t c = idx % cols;
     uint64_t s = 0;
+#pragma unroll 8
     for (int ch = 0; ch < chunks; ++ch) s += part[(size_t)q * part_qstride + ((size_t)ch * 2 + l) * cols + c];
     out[(size_t)q * out_qstride + (size_t)l * cols + c] = mod_u64(s, T->limb[l].cr, T->limb[l].q);
 }
@@ -366,14 +341,6 @@ cudaError_t launch_mv_chunk_reduce(const uint32_t* part, size_t part_qstride, in
     if (nq <= 0) return cudaSuccess;
     mv_chunk_reduce_kernel<<<dim3((unsigned)((2 * cols + 255) / 256), nq), 256, 0, s>>>(part, part_qstride, chunks,
                                                                                          cols, T, out, out_qstride);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_qplanes(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T, uint8_t* planes,
-                           int nq, cudaStream_t s) {
-    if (nq <= 0) return cudaSuccess;
-    if (rows % 1024) return cudaErrorInvalidValue;
-    qplanes_kernel<<<dim3((unsigned)(rows / 1024), nq), 256, 0, s>>>(qraw, qstride, rows, T, planes);
     return cudaGetLastError();
 }
 
@@ -485,9 +452,7 @@ cudaError_t launch_matvec_tc_ranges(const uint16_t* db, size_t rows, size_t ld, 
     if (e) return e;
     const int items = P.n_mtiles * P.n_kchunks;
     const int grid = std::min(items, std::max(1, num_sms));
-    if ((e = cudaMemsetAsync(tiles, 0, sizeof(unsigned), s))) return e;
-    mv_tc_kernel<<<grid, 256, smem, s>>>(ma, mb, P);
-    return cudaGetLastError();
+    return launch_overlapped(mv_tc_kernel, grid, 256, smem, s, ma, mb, P);
 }
 
 }  // namespace ipb

@@ -2,7 +2,8 @@
 //
 // One answer (gpu_answer / gpu_answer_batch, reference src/gpu_protocol.cu:
 // 1121-1535) runs these launches on one stream:
-//   qprep     key-switching keys to NTT form (KSK5 as byte planes), RGSW to u32 residues
+//   qprep     key-switching keys to NTT form (KSK5 as byte planes), RGSW to
+//             u32 residues, LWE vectors to the mat-vec's byte planes
 //   matvec    r_l[j] = sum_i db[i][j] * b_l[i] mod q_l   (DB pass, HBM bound)
 //   tensor pass (tensorpass_tc.cu): sum_{dir,s,j} D[s][j][i] * K5[j][perm_s(i)]
 //   finalize  per group: NTT(r slice) - tensor partials - D_final (.) Kneg1
@@ -31,24 +32,38 @@ __device__ __forceinline__ void st8(uint32_t* p, const uint32_t (&v)[8]) {
 }
 
 // ------------------------------------------------------------------ qprep
-// grid (nq, 12): y < 8 -> one key poly NTT (key, digit, limb); y >= 8 -> a
-// quarter of the RGSW u64 -> u32 reduction.  The client sends KSK b-parts in
-// coefficient form and RGSW in NTT form (capi.h:47-54); the reference NTTs the
-// keys on the server (src/gpu_protocol.cu:1059-1094).  Inputs are reduced
-// mod q (identical to the reference on canonical inputs).  KSK5 leaves as the
-// tensor pass's N operand: byte planes kplanes[q][limb][byte][4096], digit j's
-// slots in the order of T.slot_of at positions j * N ..; KSK-1 as
-// keys[q][limb][digit][N].
+// Query preparation, grid (nq, n_key + n_rgsw + n_plane), any of the three parts:
+//   8 blocks       one key poly NTT (key, digit, limb) each.  The client sends
+//                  KSK b-parts in coefficient form and RGSW in NTT form
+//                  (capi.h:47-54); the reference NTTs the keys on the server
+//                  (src/gpu_protocol.cu:1059-1094).  KSK5 leaves as the tensor
+//                  pass's N operand: byte planes kplanes[q][limb][byte][4096],
+//                  digit j's slots in the order of T.slot_of at positions
+//                  j * N ..; KSK-1 as keys[q][limb][digit][N].
+//   16 blocks      an eighth of a row of the RGSW u64 -> u32 reduction each.
+//   rows / 1024    CRT byte planes of 1024 LWE coefficients each:
+//                  planes[7q + k][rows] = byte k of B[i] = CRT(b_0[i] mod q0,
+//                  b_1[i] mod q1) < q0 q1 (Garner: b_1 + q1 ((b_0 - b_1) q1^-1
+//                  mod q0)).
+// Inputs are reduced mod q (identical to the reference on canonical inputs).
+// Bound by latency at few queries: every thread's loads are independent, so a
+// block waits for memory once (the RGSW part took 14 us as 4 blocks of 32
+// dependent rounds).
+constexpr int kKeyBlocks = 8, kRgswBlocks = 16;
+constexpr int kPlanes = 7;
 __global__ void __launch_bounds__(256) qprep_kernel(const uint64_t* __restrict__ qraw, size_t qstride,
                                                     size_t rows, const DevTables* __restrict__ T,
                                                     uint8_t* __restrict__ kplanes, uint32_t* __restrict__ keys,
-                                                    uint32_t* __restrict__ rgsw32, int y0) {
+                                                    uint32_t* __restrict__ rgsw32, uint8_t* __restrict__ planes,
+                                                    int n_key, int n_rgsw) {
     __shared__ __align__(16) uint32_t sbuf[kNttBuf], slots[kN];
-    const int b = blockIdx.x, y = y0 + (int)blockIdx.y;
+    let_next_start();
+    after_previous();
+    const int b = blockIdx.x, y = blockIdx.y;
     const uint32_t t = threadIdx.x;
     const uint64_t* qr = qraw + (size_t)b * qstride;
     const size_t blk = (size_t)kDeff * 2 * kN;
-    if (y < 8) {
+    if (y < n_key) {
         const int key = y >> 2, j = (y >> 1) & 1, l = y & 1;
         const LimbTables& L = T->limb[l];
         const uint64_t* src = qr + 2 * rows + key * blk + (size_t)(j * 2 + l) * kN;
@@ -74,13 +89,32 @@ __global__ void __launch_bounds__(256) qprep_kernel(const uint64_t* __restrict__
             for (int e = 0; e < 8; ++e) w[e >> 2] |= ((r[e] >> (8 * p)) & 0xFFu) << (8 * (e & 3));
             *reinterpret_cast<uint2*>(dst + (size_t)p * (kDeff * kN)) = make_uint2(w[0], w[1]);
         }
+    } else if (y < n_key + n_rgsw) {
+        // 16 polynomials of N words, [row][digit][limb]
+        const size_t i0 = (size_t)(y - n_key) * kN + t;
+        const LimbTables& L = T->limb[(y - n_key) & 1];
+        const uint64_t* src = qr + 2 * rows + 2 * blk + i0;
+        uint32_t* dst = rgsw32 + (size_t)b * 4 * blk + i0;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dst[256 * e] = mod_u64(src[256 * e], L.cr, L.q);
     } else {
-        const uint64_t* src = qr + 2 * rows + 2 * blk;
-        uint32_t* dst = rgsw32 + (size_t)b * 4 * blk;
-        const size_t q4 = blk;  // 4*blk elements split over 4 CTAs
-        for (size_t i = (size_t)(y - 8) * q4 + t; i < (size_t)(y - 7) * q4; i += 256) {
-            const int l = (int)((i / kN) & 1);
-            dst[i] = mod_u64(src[i], T->limb[l].cr, T->limb[l].q);
+        const size_t i4 = ((size_t)(y - n_key - n_rgsw) * 256 + t) * 4;
+        uint64_t B[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const uint32_t v0 = mod_u64(qr[i4 + c], T->limb[0].cr, kQ0);
+            const uint32_t v1 = mod_u64(qr[rows + i4 + c], T->limb[1].cr, kQ1);
+            const uint32_t v1r = v1 >= kQ0 ? v1 - kQ0 : v1;
+            const uint32_t diff = v0 >= v1r ? v0 - v1r : v0 + kQ0 - v1r;
+            const uint32_t h = csub(shoup_mul(diff, T->crt_c[0], T->crt_cp[0], kQ0), kQ0);
+            B[c] = (uint64_t)v1 + (uint64_t)kQ1 * h;
+        }
+#pragma unroll
+        for (int k = 0; k < kPlanes; ++k) {
+            uint32_t packed = 0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) packed |= (uint32_t)((B[c] >> (8 * k)) & 0xFFu) << (8 * c);
+            *reinterpret_cast<uint32_t*>(planes + ((size_t)kPlanes * b + k) * rows + i4) = packed;
         }
     }
 }
@@ -162,39 +196,49 @@ __global__ void __launch_bounds__(256) matvec_kernel(const uint16_t* __restrict_
 // (reference src/gpu_protocol.cu:1233-1274, src/gpu_online.cu:547-559).
 // The tensor pass result is tp_out[q][g][l][N] (tensorpass_tc.cu), laid out as
 // packed_b is.
-__global__ void __launch_bounds__(256) finalize_kernel(
+__global__ void __launch_bounds__(256, 4) finalize_kernel(
     const uint32_t* __restrict__ mvpart, size_t mv_qstride, int mv_chunks, size_t cols,
     const uint32_t* __restrict__ tp_out, int g0,
     const uint32_t* __restrict__ df, const uint32_t* __restrict__ keys, size_t key_qstride,
     const DevTables* __restrict__ T, uint32_t* __restrict__ packed_b, size_t pb_qstride) {
     __shared__ __align__(16) uint32_t sbuf[kNttBuf];
+    let_next_start();
     const int g = g0 + (int)blockIdx.x, l = blockIdx.y, b = blockIdx.z;
     const uint32_t t = threadIdx.x;
     const LimbTables& L = T->limb[l];
-    uint32_t r[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const size_t x = (size_t)g * kN + t + 256 * e;
-        uint64_t s = 0;
-        const uint32_t* mp = mvpart + (size_t)b * mv_qstride + (size_t)l * cols + x;
-        for (int y = 0; y < mv_chunks; ++y) s += mp[(size_t)y * 2 * cols];
-        r[e] = mod_u64(s, L.cr, L.q);
-    }
-    ntt_fwd(r, sbuf, L.fwd, L.q, t, 0);
-    uint32_t cs[8], d0[8], d1[8], k0[8], k1[8];
-    ld8(tp_out + (size_t)b * pb_qstride + ((size_t)g * 2 + l) * kN + 8 * t, cs);
+    uint32_t d0[8], d1[8];
     ld8(df + ((size_t)g * 2 + l) * kDeff * kN + 8 * t, d0);
     ld8(df + (((size_t)g * 2 + l) * kDeff + 1) * kN + 8 * t, d1);
+    after_previous();
+    // Everything the block reads is asked for before the transform: one memory
+    // latency per block, not three.
+    uint32_t o[8], k0[8], k1[8];
+    ld8(tp_out + (size_t)b * pb_qstride + ((size_t)g * 2 + l) * kN + 8 * t, o);
     const uint32_t* kn = keys + (size_t)b * key_qstride + (size_t)l * kDeff * kN;
     ld8(kn + 8 * t, k0);
     ld8(kn + kN + 8 * t, k1);
-    uint32_t o[8];
+    const uint32_t* mp = mvpart + (size_t)b * mv_qstride + (size_t)l * cols + (size_t)g * kN + t;
+    uint32_t r[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const uint32_t fin = mod_u64((uint64_t)d0[e] * k0[e] + (uint64_t)d1[e] * k1[e], L.cr, L.q);
-        const uint32_t sub = add_mod(cs[e], fin, L.q);
-        o[e] = sub_mod(r[e], sub, L.q);
+    for (int e = 0; e < 8; ++e) r[e] = mp[256 * e];
+    if (mv_chunks > 1) {
+        uint64_t s[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] = r[e];
+        for (int y = 1; y < mv_chunks; ++y) {
+            mp += 2 * cols;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) s[e] += mp[256 * e];
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r[e] = mod_u64(s[e], L.cr, L.q);
     }
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        o[e] = add_mod(o[e], mod_u64((uint64_t)d0[e] * k0[e] + (uint64_t)d1[e] * k1[e], L.cr, L.q), L.q);
+    ntt_fwd(r, sbuf, L.fwd, L.q, t, 0);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] = sub_mod(r[e], o[e], L.q);
     st8(packed_b + (size_t)b * pb_qstride + ((size_t)g * 2 + l) * kN + 8 * t, o);
 }
 
@@ -409,6 +453,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
     uint64_t* mbx = reinterpret_cast<uint64_t*>(cin + 2 * kN);      // [parity] partner terms
     uint64_t* mbc = mbx + 2;                                        // [parity] contribution
     __shared__ volatile int abort_flag;
+    let_next_start();
     const uint32_t rank = cluster_rank();
     const int p = (int)(rank >> 1), l = (int)(rank & 1);
     const int ct = blockIdx.x >> 2, b = blockIdx.y;
@@ -425,6 +470,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
         for (int k = 0; k < 2; ++k) { hb_init(&mbx[k]); hb_init(&mbc[k]); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    after_previous();  // the tables above are constant; what follows was written by this answer's kernels
     const uint32_t rank_limb = (uint32_t)((p << 1) | (1 - l));   // same poly, other limb
     const uint32_t rank_poly = (uint32_t)(((1 - p) << 1) | l);   // other poly, same limb
     const size_t start = (size_t)ct * d_act;
@@ -552,6 +598,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     uint64_t* mbx = reinterpret_cast<uint64_t*>(cin + 2 * 3 * kN);  // [parity] partner terms
     uint64_t* mbc = mbx + 2;                                         // [parity] contributions
     __shared__ volatile int abort_flag;
+    let_next_start();
     const uint32_t rank = cluster_rank();
     const int p = (int)(rank >> 2), l = (int)((rank >> 1) & 1), j = (int)(rank & 1);
     const int ct = blockIdx.x >> 3, b = blockIdx.y;
@@ -567,6 +614,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
         for (int k = 0; k < 2; ++k) { hb_init(&mbx[k]); hb_init(&mbc[k]); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    after_previous();  // the tables above are constant; what follows was written by this answer's kernels
     const uint32_t rank_limb = (uint32_t)((p << 2) | ((1 - l) << 1) | j);   // same poly and digit, other limb
     const uint32_t rank_sib = (uint32_t)((p << 2) | (l << 1) | (1 - j));    // same poly and limb, other digit
     const uint32_t rank_o0 = (uint32_t)(((1 - p) << 2) | (l << 1) | 0);     // other poly, same limb, digit 0
@@ -762,19 +810,15 @@ cudaError_t launch_fill_db(uint16_t* out, size_t count, uint64_t seed, cudaStrea
 }
 
 // ==================================================================== wrappers
-cudaError_t launch_qprep(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T,
-                         uint8_t* kplanes, uint32_t* keys, uint32_t* rgsw32, int nq, cudaStream_t s) {
-    return launch_qprep_parts(qraw, qstride, rows, T, kplanes, keys, rgsw32, nq, 3, s);
-}
-
-cudaError_t launch_qprep_parts(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T,
-                               uint8_t* kplanes, uint32_t* keys, uint32_t* rgsw32, int nq, int parts,
-                               cudaStream_t s) {
+cudaError_t launch_qprep(const uint64_t* qraw, size_t qstride, size_t rows, const DevTables* T, uint8_t* kplanes,
+                         uint32_t* keys, uint32_t* rgsw32, uint8_t* planes, int nq, int parts, cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
-    if (parts < 1 || parts > 3) return cudaErrorInvalidValue;
-    const int y0 = (parts & 1) ? 0 : 8, y1 = (parts & 2) ? 12 : 8;  // rows 0-7: key NTTs, 8-11: RGSW
-    qprep_kernel<<<dim3(nq, y1 - y0), 256, 0, s>>>(qraw, qstride, rows, T, kplanes, keys, rgsw32, y0);
-    return cudaGetLastError();
+    if (parts < 1 || parts > (kPrepKeys | kPrepRgsw | kPrepPlanes)) return cudaErrorInvalidValue;
+    if ((parts & kPrepPlanes) && rows % 1024) return cudaErrorInvalidValue;
+    const int n_key = (parts & kPrepKeys) ? kKeyBlocks : 0, n_rgsw = (parts & kPrepRgsw) ? kRgswBlocks : 0;
+    const int n_plane = (parts & kPrepPlanes) ? (int)(rows / 1024) : 0;
+    return launch_overlapped(qprep_kernel, dim3(nq, n_key + n_rgsw + n_plane), 256, 0, s, qraw, qstride, rows, T, kplanes,
+                             keys, rgsw32, planes, n_key, n_rgsw);
 }
 
 cudaError_t launch_matvec(const uint16_t* db, size_t rows, size_t cols, int chunks, const uint64_t* qraw,
@@ -820,9 +864,8 @@ cudaError_t launch_finalize_range(const uint32_t* mvpart, size_t mv_qstride, int
                                   size_t groups, size_t g0, size_t gn, int nq, cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
     if (gn == 0 || g0 + gn > groups) return cudaErrorInvalidValue;
-    finalize_kernel<<<dim3((unsigned)gn, 2, nq), 256, 0, s>>>(mvpart, mv_qstride, mv_chunks, cols, tp_out,
-                                                              (int)g0, df, keys, key_qstride, T, packed_b, pb_qstride);
-    return cudaGetLastError();
+    return launch_overlapped(finalize_kernel, dim3((unsigned)gn, 2, nq), 256, 0, s, mvpart, mv_qstride, mv_chunks, cols,
+                             tp_out, (int)g0, df, keys, key_qstride, T, packed_b, pb_qstride);
 }
 
 cudaError_t launch_horner(const uint32_t* pre_a, const uint32_t* packed_b, size_t pb_qstride,
@@ -849,10 +892,8 @@ cudaError_t launch_horner_cluster(const uint32_t* pre_a, const uint32_t* packed_
     if (!horner_range_ok(hr, d_act)) return cudaErrorInvalidValue;
     cudaError_t e = allow_max_smem(horner_cl_kernel);
     if (e) return e;
-    horner_cl_kernel<<<dim3((unsigned)(4 * num_cts), nq), 512, kHornerClSmem, s>>>(pre_a, packed_b, pb_qstride,
-                                                                                   rgsw32, T, groups, d_act, resp,
-                                                                                   resp_qstride, err, hr);
-    return cudaGetLastError();
+    return launch_overlapped(horner_cl_kernel, dim3((unsigned)(4 * num_cts), nq), 512, kHornerClSmem, s, pre_a, packed_b,
+                             pb_qstride, rgsw32, T, groups, d_act, resp, resp_qstride, err, hr);
 }
 
 cudaError_t launch_horner_cluster8(const uint32_t* pre_a, const uint32_t* packed_b, size_t pb_qstride,
@@ -863,9 +904,8 @@ cudaError_t launch_horner_cluster8(const uint32_t* pre_a, const uint32_t* packed
     if (!horner_range_ok(hr, d_act)) return cudaErrorInvalidValue;
     cudaError_t e = allow_max_smem(horner_cl8_kernel);
     if (e) return e;
-    horner_cl8_kernel<<<dim3((unsigned)(8 * num_cts), nq), 256, kHornerCl8Smem, s>>>(
-        pre_a, packed_b, pb_qstride, rgsw32, T, groups, d_act, resp, resp_qstride, err, hr);
-    return cudaGetLastError();
+    return launch_overlapped(horner_cl8_kernel, dim3((unsigned)(8 * num_cts), nq), 256, kHornerCl8Smem, s, pre_a,
+                             packed_b, pb_qstride, rgsw32, T, groups, d_act, resp, resp_qstride, err, hr);
 }
 
 cudaError_t launch_ntt_batch(uint32_t* polys, size_t n, int limb_run, bool inverse, const DevTables* T,

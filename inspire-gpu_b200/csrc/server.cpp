@@ -217,7 +217,7 @@ size_t lane_bytes(const Server& S, size_t cap) {
     const size_t R = S.pp.db_rows, G = S.pp.n_packed;
     return cap * S.qstride * 8 + cap * kKeyStride * 4 + cap * kRgswStride * 4 + cap * S.mv_qstride * 4 +
            cap * kTpPlaneBytes + (size_t)2 * kN * cap * G * 4 + cap * S.pb_qstride * 4 + cap * S.resp_qstride * 8 +
-           mv_tc_planes_bytes(R, (int)cap) + sizeof(int) + 2 * sizeof(unsigned) + cap * S.wire_q +
+           mv_tc_planes_bytes(R, (int)cap) + sizeof(int) + 4 * sizeof(unsigned) + cap * S.wire_q +
            cap * std::max(S.wire_r, S.wire_c) + cap * S.pp.num_cts * 4 * kN * 4;
 }
 
@@ -236,7 +236,7 @@ void alloc_lane(const Server& S, Lane& L, size_t cap, int gt_pass) {
     L.resp = A.alloc<uint64_t>(cap * S.resp_qstride);
     L.planes = A.alloc<uint8_t>(mv_tc_planes_bytes(R, (int)cap));
     L.d_err = A.alloc<int>(1);
-    L.tiles = A.alloc<unsigned>(2);
+    L.tiles = A.alloc<unsigned>(4);
     L.wire_in = A.alloc<uint8_t>(cap * S.wire_q);
     L.wire_out = A.alloc<uint8_t>(cap * std::max(S.wire_r, S.wire_c));
     L.codec_tmp = A.alloc<uint32_t>(cap * S.pp.num_cts * 4 * kN);
@@ -245,12 +245,14 @@ void alloc_lane(const Server& S, Lane& L, size_t cap, int gt_pass) {
     IPB_CK(cudaEventCreateWithFlags(&L.join, cudaEventDisableTiming));
     IPB_CK(cudaEventCreateWithFlags(&L.rgsw_ready, cudaEventDisableTiming));
     IPB_CK(cudaStreamCreateWithFlags(&L.hstream, cudaStreamNonBlocking));
+    IPB_CK(cudaEventCreateWithFlags(&L.hfork, cudaEventDisableTiming));
     IPB_CK(cudaEventCreateWithFlags(&L.hjoin, cudaEventDisableTiming));
     for (auto& e : L.hev) IPB_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     // Defined contents before any pipeline run (the autotuner runs on them).
     IPB_CK(cudaMemset(L.qraw, 0, cap * S.qstride * 8));
     IPB_CK(cudaMemset(L.planes, 0, mv_tc_planes_bytes(R, (int)cap)));
     IPB_CK(cudaMemset(L.d_err, 0, sizeof(int)));
+    IPB_CK(cudaMemset(L.tiles, 0, 4 * sizeof(unsigned)));
     // The lanes run on non-blocking streams, which do not wait for the
     // legacy stream the memsets above went to.
     IPB_CK(cudaDeviceSynchronize());
@@ -380,31 +382,49 @@ int lane_gt_pass(size_t cap) { return (int)std::min<size_t>(cap, (size_t)kTpMaxQ
 
 static bool chunked_ok(const Server& S, const Sched& sc, size_t count);
 
+// Defaults per batch size, each line drawn where both sides measured alike
+// (one GPU, medians of interleaved runs):
+//   Horner kernel: 8 CTAs per chain while all clusters run at once (up to 8
+//     chains, 3.2 us a step), 4 CTAs beyond (4.0 us; 16 chains of 8 CTAs take
+//     5.0 us).
+//   Horner chain trailing the DB pass in chunks where a chunk's mat-vec lasts
+//     longer than its chain steps (32768 rows: 19 us a group against 4-11) and
+//     the chain is worth the extra launches: 128 groups, 16 GB: 1 query 3.68
+//     against 3.92 ms, 8: 3.99 / 4.08, 16: 4.19 / 4.39, 32: 5.42 / 5.40; 32
+//     groups, 4 GB: 1.14 / 1.10; 128 groups on 2048 rows: 1.84 / 1.75.
+//   Tensor pass beside the mat-vec, on two SMs of three, where the two streams
+//     are short enough for launch ramps and tails to count (up to 8 GB
+//     together): 1 GB 293 -> 281 us at 1 query, 410 -> 390 at 32; 4 GB (6.4 GB
+//     together) 1077 -> 1047 and 1472 -> 1383; 1 group on 2048 rows 62 -> 52 at
+//     32.  Beyond, either order streams at the HBM rate: 128 groups on 2048 rows
+//     (9.7 GB) 1733 / 1726 and 1792 / 2022 at 8, 16 GB 4.02 / 4.03 ms.
+// IPB_MATVEC, IPB_HORNER, IPB_TP_SMS and IPB_HCHUNKS pin a choice for every
+// batch size.
 std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
-    Sched def;
-    def.tp_pass = gt_pass;
-    if (const char* m = std::getenv("IPB_MATVEC")) def.matvec_tc = std::strcmp(m, "simt") != 0;
-    if (const char* h = std::getenv("IPB_HORNER"))
-        def.horner_cluster = std::strcmp(h, "cta") == 0 ? 0 : (std::strcmp(h, "cl8") == 0 ? 2 : 1);
-    if (const char* t = std::getenv("IPB_TP_SMS"))
-        def.tp_sms = def.matvec_tc ? std::max(0, std::min(std::atoi(t), S.num_sms - 1)) : 0;
-    std::vector<Sched> out(cap + 1, def);
-    // The Horner chain trails the DB pass in chunks by default where the
-    // geometry allows it, the chain is long enough to matter (at least 32
-    // groups per response ciphertext) and the batch has at most chain / 16
-    // queries (at most 16): the hidden chain then outweighs the extra
-    // launches.  Measured: 128 groups
-    // 2-8 % faster from 1 to 16 queries; 32 groups 4.5 % faster at 1 query
-    // and 1 % slower at 8; 8 groups 4-9 % slower.  IPB_HCHUNKS sets it for
-    // every batch size.
-    const size_t chain = std::min(S.pp.D, S.pp.n_packed);  // groups per response ciphertext
-    for (size_t c = 1; c <= cap; ++c) {
-        Sched probe = def;
-        probe.hchunks = 8;
-        if (chain >= 32 && c <= std::min<size_t>(16, chain / 16) && chunked_ok(S, probe, c)) out[c].hchunks = 8;
+    const size_t G = S.pp.n_packed, chain = std::min(S.pp.D, G);  // groups per response ciphertext
+    const double stream_bytes = 2.0 * (double)S.pp.db_rows * (double)S.pp.db_cols + (double)tp_dt_bytes(G);
+    const char* const m = std::getenv("IPB_MATVEC");
+    const char* const h = std::getenv("IPB_HORNER");
+    const char* const t = std::getenv("IPB_TP_SMS");
+    const char* const k = std::getenv("IPB_HCHUNKS");
+    std::vector<Sched> out(cap + 1);
+    for (size_t c = 0; c <= cap; ++c) {
+        Sched& sc = out[c];
+        sc.tp_pass = gt_pass;
+        if (m) sc.matvec_tc = std::strcmp(m, "simt") != 0;
+        sc.horner_cluster = c * S.pp.num_cts <= 8 ? 2 : 1;
+        if (chain >= 64 && S.pp.db_rows >= 16384 && c <= std::min<size_t>(16, chain / 8)) {
+            Sched chunked = sc;
+            chunked.horner_cluster = 1;
+            chunked.hchunks = 8;
+            if (chunked_ok(S, chunked, c)) sc = chunked;
+        }
+        if (h) sc.horner_cluster = std::strcmp(h, "cta") == 0 ? 0 : (std::strcmp(h, "cl8") == 0 ? 2 : 1);
+        if (k) sc.hchunks = std::max(0, std::min(std::atoi(k), kMaxHChunks));
+        if (!sc.matvec_tc) continue;
+        if (t) sc.tp_sms = std::max(0, std::min(std::atoi(t), S.num_sms - 1));
+        else if (sc.hchunks <= 1 && stream_bytes <= 8e9) sc.tp_sms = S.num_sms * 2 / 3;
     }
-    if (const char* h = std::getenv("IPB_HCHUNKS"))
-        for (auto& sc : out) sc.hchunks = std::max(0, std::min(std::atoi(h), kMaxHChunks));
     return out;
 }
 
@@ -413,13 +433,11 @@ std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
 // lwe_ready (optional): the queries' LWE vectors arrive later than their
 // key parts (copied on another stream, this event marks them); the key side
 // (query prep, tensor pass) then runs first and the mat-vec after the event.
-// The RGSW parts are then prepared on that other stream as well.
 // q_off: the batch's first lane slot (slices of a batch larger than one DB
 // pass run the whole phase on slots [q_off, q_off + count)).
-// qprep_parts: 3 prepares keys and RGSW parts here, 1 the keys only (the
-// RGSW parts are prepared elsewhere).
+// prep_rgsw: the RGSW parts are prepared here too.
 int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t count, cudaStream_t st,
-                 cudaEvent_t* ev, cudaEvent_t lwe_ready, int qprep_parts) {
+                 cudaEvent_t* ev, cudaEvent_t lwe_ready, bool prep_rgsw) {
     const Params& pp = S.pp;
     const Precomp& P = *S.pre;
     const size_t R = pp.db_rows, C = pp.db_cols, G = pp.n_packed;
@@ -432,41 +450,46 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
     if (ev) IPB_CK(cudaEventRecord(ev[0], st));
     uint8_t* const kplanes = L.kplanes + q_off * kTpPlaneBytes;
     uint32_t* const tp_out = L.tp_out + q_off * S.pb_qstride;
-    IPB_CK(launch_qprep_parts(qraw, S.qstride, R, P.tables, kplanes, keys, L.rgsw32 + q_off * kRgswStride, nq,
-                              qprep_parts, st));
-    ++launches;
+    auto prep = [&](int parts) {
+        IPB_CK(launch_qprep(qraw, S.qstride, R, P.tables, kplanes, keys, L.rgsw32 + q_off * kRgswStride, planes, nq,
+                            parts, st));
+        ++launches;
+    };
+    const int planes_part = sc.matvec_tc ? kPrepPlanes : 0;
+    prep(kPrepKeys | (prep_rgsw ? kPrepRgsw : 0) | (lwe_ready ? 0 : planes_part));
     if (ev) IPB_CK(cudaEventRecord(ev[1], st));
     // Beside: the tensor pass (keys only) on sc.tp_sms SMs from the lane's
-    // second stream while the mat-vec (DB only) runs on the other SMs; the
-    // two persistent kernels take one CTA per SM each, so the split holds.
+    // Horner stream while the mat-vec (DB only) starts on the other SMs; both
+    // are persistent with one CTA per SM, so the mat-vec's remaining CTAs start
+    // as the tensor pass's end.
     const bool beside = sc.matvec_tc && sc.tp_sms > 0 && sc.tp_sms < S.num_sms;
     auto tensor_pass = [&](cudaStream_t ts, int sms) {
         for (size_t c0 = 0; c0 < count; c0 += (size_t)sc.tp_pass) {
             const int n = (int)std::min<size_t>((size_t)sc.tp_pass, count - c0);
             IPB_CK(launch_tensor_pass(P.pre_dt, 0, tp_tiles(G), kplanes + c0 * kTpPlaneBytes, n, nullptr,
-                                      tp_out + c0 * S.pb_qstride, S.pb_qstride, L.d_err, L.tiles + 1, sms, ts));
+                                      tp_out + c0 * S.pb_qstride, S.pb_qstride, L.d_err, L.tiles + 2, sms, ts));
             ++launches;
         }
     };
     if (beside) {
-        IPB_CK(cudaEventRecord(L.fork, st));
-        IPB_CK(cudaStreamWaitEvent(L.aux, L.fork, 0));
-        tensor_pass(L.aux, sc.tp_sms);
-        IPB_CK(cudaEventRecord(L.join, L.aux));
-    }
-    if (lwe_ready && !beside) {
+        IPB_CK(cudaEventRecord(L.hfork, st));
+        IPB_CK(cudaStreamWaitEvent(L.hstream, L.hfork, 0));
+        tensor_pass(L.hstream, sc.tp_sms);
+        IPB_CK(cudaEventRecord(L.hjoin, L.hstream));
+    } else if (lwe_ready) {
         tensor_pass(st, S.num_sms);
+    }
+    if (lwe_ready) {
         IPB_CK(cudaStreamWaitEvent(st, lwe_ready, 0));
+        if (planes_part) prep(planes_part);
     }
     int mv_parts;
     if (sc.matvec_tc) {
-        IPB_CK(launch_qplanes(qraw, S.qstride, R, P.tables, planes, nq, st));
-        ++launches;
         for (size_t c0 = 0; c0 < count; c0 += 32) {
             const int n = (int)std::min<size_t>(32, count - c0);
             IPB_CK(launch_matvec_tc(P.db, R, C, planes + mv_tc_planes_offset(c0, R), n, P.tables,
-                                    mvpart + c0 * S.mv_qstride, S.mv_qstride, L.d_err, L.tiles,
-                                    beside ? S.num_sms - sc.tp_sms : S.num_sms, S.tc_kchunk_rows, st));
+                                    mvpart + c0 * S.mv_qstride, S.mv_qstride, L.d_err, L.tiles, S.num_sms,
+                                    S.tc_kchunk_rows, st));
             ++launches;
         }
         mv_parts = S.tc_kchunks;
@@ -480,7 +503,7 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
         mv_parts = S.mv_chunks;
     }
     if (beside)
-        IPB_CK(cudaStreamWaitEvent(st, L.join, 0));  // stage times: mat-vec = both, tensor pass = 0
+        IPB_CK(cudaStreamWaitEvent(st, L.hjoin, 0));  // stage times: mat-vec = both, tensor pass = 0
     if (ev) IPB_CK(cudaEventRecord(ev[2], st));
     if (!beside && !lwe_ready) tensor_pass(st, S.num_sms);
     if (ev) IPB_CK(cudaEventRecord(ev[3], st));
@@ -605,26 +628,30 @@ static std::vector<size_t> chunk_sizes(size_t G, size_t ipg, int num_sms, size_t
 // faster).
 // lwe_ready / rgsw_ready (optional): the blocking path's copies, on other
 // streams, of the LWE vectors (the mat-vec waits) and of the prepared RGSW
-// parts (the first Horner chunk waits).  qprep_parts as run_db_phase's.
+// parts (the first Horner chunk waits; else they are prepared here).
 static int run_chunked(const Server& S, Lane& L, const Sched& sc, size_t count, cudaStream_t st,
-                       cudaEvent_t lwe_ready = nullptr, cudaEvent_t rgsw_ready = nullptr, int qprep_parts = 3,
+                       cudaEvent_t lwe_ready = nullptr, cudaEvent_t rgsw_ready = nullptr,
                        cudaEvent_t db_done = nullptr) {
     const Params& pp = S.pp;
     const Precomp& P = *S.pre;
     const size_t R = pp.db_rows, C = pp.db_cols, G = pp.n_packed;
     const int nq = (int)count;
     int launches = 0;
-    IPB_CK(launch_qprep_parts(L.qraw, S.qstride, R, P.tables, L.kplanes, L.keys, L.rgsw32, nq, qprep_parts, st));
-    ++launches;
+    auto prep = [&](int parts) {
+        IPB_CK(launch_qprep(L.qraw, S.qstride, R, P.tables, L.kplanes, L.keys, L.rgsw32, L.planes, nq, parts, st));
+        ++launches;
+    };
+    prep(kPrepKeys | (rgsw_ready ? 0 : kPrepRgsw) | (lwe_ready ? 0 : kPrepPlanes));
     for (size_t c0 = 0; c0 < count; c0 += (size_t)sc.tp_pass) {
         const int n = (int)std::min<size_t>((size_t)sc.tp_pass, count - c0);
         IPB_CK(launch_tensor_pass(P.pre_dt, 0, tp_tiles(G), L.kplanes + c0 * kTpPlaneBytes, n, nullptr,
-                                  L.tp_out + c0 * S.pb_qstride, S.pb_qstride, L.d_err, L.tiles + 1, S.num_sms, st));
+                                  L.tp_out + c0 * S.pb_qstride, S.pb_qstride, L.d_err, L.tiles + 2, S.num_sms, st));
         ++launches;
     }
-    if (lwe_ready) IPB_CK(cudaStreamWaitEvent(st, lwe_ready, 0));
-    IPB_CK(launch_qplanes(L.qraw, S.qstride, R, P.tables, L.planes, nq, st));
-    ++launches;
+    if (lwe_ready) {
+        IPB_CK(cudaStreamWaitEvent(st, lwe_ready, 0));
+        prep(kPrepPlanes);
+    }
     // Chunks are ranges [lo, hi) of chain positions, the same in every
     // response ciphertext (ciphertext t's groups t * d_act + [lo, hi)): one
     // mat-vec launch covers the range in all of them.
@@ -688,7 +715,7 @@ void enqueue_horner(const Server& S, const Sched& sc, const uint32_t* packed_b, 
 void enqueue_qprep_slots(const Server& S, Lane& L, size_t s0, size_t count, cudaStream_t st) {
     IPB_CK(launch_qprep(L.qraw + s0 * S.qstride, S.qstride, S.pp.db_rows, S.pre->tables,
                         L.kplanes + s0 * kTpPlaneBytes, L.keys + s0 * kKeyStride, L.rgsw32 + s0 * kRgswStride,
-                        (int)count, st));
+                        nullptr, (int)count, kPrepKeys | kPrepRgsw, st));
 }
 
 void enqueue_scan_segment(const Server& S, Lane& L, uint8_t* kplanes_pos, const std::vector<SlotRun>& runs, int seg,
@@ -701,8 +728,8 @@ void enqueue_scan_segment(const Server& S, Lane& L, uint8_t* kplanes_pos, const 
     for (const SlotRun& r : runs) {
         if (n + r.k > 32 || r.s0 + r.k > L.cap) throw std::invalid_argument("scan segment: 1..32 queries per pass");
         // positions n .. n + k - 1 of this segment's pass: query and key planes
-        IPB_CK(launch_qplanes(L.qraw + r.s0 * S.qstride, S.qstride, R, P.tables, L.planes + mv_tc_planes_offset(n, R),
-                              (int)r.k, st));
+        IPB_CK(launch_qprep(L.qraw + r.s0 * S.qstride, S.qstride, R, P.tables, nullptr, nullptr, nullptr,
+                            L.planes + mv_tc_planes_offset(n, R), (int)r.k, kPrepPlanes, st));
         IPB_CK(cudaMemcpyAsync(kplanes_pos + n * kTpPlaneBytes, L.kplanes + r.s0 * kTpPlaneBytes,
                                r.k * kTpPlaneBytes, cudaMemcpyDeviceToDevice, st));
         for (size_t i = 0; i < r.k; ++i) qmap[n + i] = (uint8_t)(r.s0 + i);
@@ -718,7 +745,7 @@ void enqueue_scan_segment(const Server& S, Lane& L, uint8_t* kplanes_pos, const 
     for (size_t q0 = 0; q0 < n; q0 += (size_t)L.gt_pass) {
         const int k = (int)std::min<size_t>((size_t)L.gt_pass, n - q0);
         IPB_CK(launch_tensor_pass(P.pre_dt, n_tiles * seg, n_tiles, kplanes_pos + q0 * kTpPlaneBytes, k, qmap + q0,
-                                  L.tp_out, S.pb_qstride, L.d_err, L.tiles + 1, S.num_sms, st));
+                                  L.tp_out, S.pb_qstride, L.d_err, L.tiles + 2, S.num_sms, st));
     }
 }
 
@@ -741,7 +768,7 @@ int run_pipeline(const Server& S, Lane& L, const Sched& sc, size_t count, cudaSt
     // Stage timing needs the stages one after the other: it times the
     // unchunked pipeline.
     if (phases == kPhaseAll && !ev && chunked_ok(S, sc, count))
-        return run_chunked(S, L, sc, count, st, nullptr, nullptr, 3, db_done);
+        return run_chunked(S, L, sc, count, st, nullptr, nullptr, db_done);
     if (phases != kPhaseAll || 6 * ns > n_ev) ev = nullptr;
     int launches = 0;
     // Slices run one after the other, each its own pipeline on its lane
@@ -772,36 +799,55 @@ static void run_pipeline(Server* S, size_t count) {
                                                     S->timing ? S->ev.data() : nullptr, kPhaseAll, S->ev.size());
 }
 
-// The blocking answer from host views: the KSK parts are copied first and
-// the query prep and tensor pass (which need only them) start while the
-// LWE vectors and then the RGSW parts cross PCIe on the lane's second
-// stream; the mat-vec waits for the LWE vectors, the Horner chains for the
-// RGSW parts (prepared on that stream).  Schedules that already run the
-// tensor pass on the second stream stage everything first instead.
+// Batches up to this many bytes of queries are copied in one go on the
+// handle's stream (one query of 32768 rows: 0.9 MB, 17 us of PCIe): two more
+// streams and their events cost as much as the overlap would save.
+constexpr size_t kSmallBatchBytes = (size_t)1 << 20;
+
+cudaEvent_t stage_split(const Server& S, const ipir_query_view* qs, size_t count, bool rgsw) {
+    const Lane& L = S.lane;
+    if (count * S.qstride * 8 <= kSmallBatchBytes) {
+        stage_parts(S, qs, count, 0, rgsw ? 5 : 4, S.stream);
+        return nullptr;
+    }
+    IPB_CK(cudaEventRecord(L.fork, S.stream));  // the lane's buffers are free from here on
+    IPB_CK(cudaStreamWaitEvent(L.aux, L.fork, 0));
+    stage_parts(S, qs, count, 2, 2, S.stream);  // KSK parts: needed first
+    stage_parts(S, qs, count, 0, 2, L.aux);     // LWE vectors: needed by the mat-vec
+    IPB_CK(cudaEventRecord(L.join, L.aux));
+    return L.join;
+}
+
+// The blocking answer from host views.  Beyond a small batch the KSK parts
+// are copied first and the query prep and tensor pass (which need only them)
+// start while the LWE vectors and then the RGSW parts cross PCIe on the lane's
+// copy stream; the mat-vec waits for the LWE vectors, the Horner chains for
+// the RGSW parts (prepared on that stream).  With stage timing everything is
+// staged first.
 static void stage_and_run(Server* S, const ipir_query_view* qs, size_t count) {
     IPB_CK(cudaSetDevice(S->device));
     const Sched& sc = sched_for(*S, count);
-    if (sc.tp_sms > 0 || S->timing) {
+    if (S->timing) {
         stage_queries(S, qs, count);
-        S->timed_slices = S->timing ? slices_of(count, sc) : 0;
-        S->launches += (unsigned long long)run_pipeline(*S, S->lane, sc, count, S->stream,
-                                                        S->timing ? S->ev.data() : nullptr, kPhaseAll, S->ev.size());
+        S->timed_slices = slices_of(count, sc);
+        S->launches += (unsigned long long)run_pipeline(*S, S->lane, sc, count, S->stream, S->ev.data(), kPhaseAll,
+                                                        S->ev.size());
         return;
     }
     Lane& L = S->lane;
-    IPB_CK(cudaEventRecord(L.fork, S->stream));  // the lane's buffers are free from here on
-    IPB_CK(cudaStreamWaitEvent(L.aux, L.fork, 0));
-    stage_parts(*S, qs, count, 2, 2, S->stream);  // KSK parts: needed first
-    stage_parts(*S, qs, count, 0, 2, L.aux);      // LWE vectors: needed by the mat-vec
-    IPB_CK(cudaEventRecord(L.join, L.aux));
-    stage_parts(*S, qs, count, 4, 1, L.aux);      // RGSW parts: needed by the Horner chains
-    IPB_CK(launch_qprep_parts(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, L.kplanes, L.keys, L.rgsw32,
-                              (int)count, 2, L.aux));
-    IPB_CK(cudaEventRecord(L.rgsw_ready, L.aux));
+    const cudaEvent_t lwe_ready = stage_split(*S, qs, count, true);
     S->staged = count;
+    if (!lwe_ready) {
+        S->launches += (unsigned long long)run_pipeline(*S, L, sc, count, S->stream, nullptr);
+        return;
+    }
+    stage_parts(*S, qs, count, 4, 1, L.aux);      // RGSW parts: needed by the Horner chains
+    IPB_CK(launch_qprep(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, nullptr, nullptr, L.rgsw32, nullptr,
+                        (int)count, kPrepRgsw, L.aux));
+    IPB_CK(cudaEventRecord(L.rgsw_ready, L.aux));
     S->launches += 1;
     if (chunked_ok(*S, sc, count)) {
-        S->launches += (unsigned long long)run_chunked(*S, L, sc, count, S->stream, L.join, L.rgsw_ready, 1);
+        S->launches += (unsigned long long)run_chunked(*S, L, sc, count, S->stream, lwe_ready, L.rgsw_ready);
         return;
     }
     // The first slice's key side starts before the LWE vectors land; every
@@ -810,7 +856,7 @@ static void stage_and_run(Server* S, const ipir_query_view* qs, size_t count) {
     for (size_t k = 0; k < ns; ++k) {
         const size_t q0 = k * slice, n = std::min(slice, count - q0);
         S->launches += (unsigned long long)run_db_phase(*S, L, sc, q0, n, S->stream, nullptr,
-                                                        k == 0 ? L.join : nullptr, 1);
+                                                        k == 0 ? lwe_ready : nullptr, false);
         if (k == 0) IPB_CK(cudaStreamWaitEvent(S->stream, L.rgsw_ready, 0));
         S->launches += (unsigned long long)run_horner_phase(*S, L, sc, q0, n, S->stream, nullptr);
     }
@@ -1613,8 +1659,9 @@ int ipir_b200_matvec_ex(const uint16_t* db, size_t rows, size_t cols, const uint
             if (!M.T) {
                 M.T = ipb::upload_tables(M.arena, 0);
                 M.err = M.arena.alloc<int>(1);
-                M.tiles = M.arena.alloc<unsigned>(1);
+                M.tiles = M.arena.alloc<unsigned>(2);
                 IPB_CK(cudaMemset(M.err, 0, sizeof(int)));
+                IPB_CK(cudaMemset(M.tiles, 0, 2 * sizeof(unsigned)));
                 IPB_CK(cudaDeviceSynchronize());  // tables visible to any stream
             }
             // exact K-chunks: tensor cores accumulate s32 over <= 32768 rows, the
@@ -1638,7 +1685,8 @@ int ipir_b200_matvec_ex(const uint16_t* db, size_t rows, size_t cols, const uint
                     M.planes = M.arena.alloc<uint8_t>(pbytes);
                     M.planes_cap = pbytes;
                 }
-                IPB_CK(ipb::launch_qplanes(queries, 2 * rows, rows, M.T, M.planes, (int)count, s));
+                IPB_CK(ipb::launch_qprep(queries, 2 * rows, rows, M.T, nullptr, nullptr, nullptr, M.planes, (int)count,
+                                         ipb::kPrepPlanes, s));
             }
             for (size_t q0 = 0; q0 < count; q0 += (size_t)qpp) {
                 const int n = (int)std::min<size_t>((size_t)qpp, count - q0);

@@ -102,8 +102,8 @@ struct Sched {
     int matvec_tc = 1;       // 1: tcgen05 int8 mat-vec, 0: CUDA-core mat-vec
     int tp_pass = 32;        // queries per tensor-pass GEMM (<= the lane's gt_pass)
     int horner_cluster = 1;  // 1: 4-CTA cluster per chain, 2: 8-CTA cluster, 0: one CTA per chain
-    int tp_sms = 0;          // > 0: tensor pass on this many SMs beside the tcgen05 mat-vec on the
-                             // others (the lane's second stream); 0: tensor pass after the mat-vec
+    int tp_sms = 0;          // > 0: tensor pass on this many SMs beside the tcgen05 mat-vec, which starts
+                             // on the others and takes these over as they come free; 0: one after the other
     int slice = 32;          // > 0: a batch larger than this runs as consecutive slices of this many
                              // queries, each its own pipeline (query prep .. Horner) on the lane's slots;
                              // 0: the whole batch in one pipeline
@@ -136,20 +136,22 @@ struct Lane {
     uint64_t* resp = nullptr;
     uint8_t* planes = nullptr;   // query byte planes for the tensor-core mat-vec
     int* d_err = nullptr;        // device error word (pipeline wait timeouts)
-    unsigned* tiles = nullptr;   // work-item counters: [0] mat-vec, [1] tensor pass
+    unsigned* tiles = nullptr;   // work-item counters: [0..1] mat-vec, [2..3] tensor pass
     uint8_t* wire_in = nullptr;  // packed queries
     uint8_t* wire_out = nullptr; // packed or compressed responses
     uint32_t* codec_tmp = nullptr;  // coefficient-form responses for compression
-    cudaStream_t aux = nullptr;     // second stream: the tensor pass beside the mat-vec
+    cudaStream_t aux = nullptr;     // the blocking path's copies
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaEvent_t rgsw_ready = nullptr;  // RGSW parts staged and prepared on aux
-    cudaStream_t hstream = nullptr;    // Horner chunks trailing the DB pass (Sched::hchunks)
-    cudaEvent_t hjoin = nullptr;
+    cudaStream_t hstream = nullptr;    // the tensor pass beside the mat-vec, or Horner chunks trailing the
+                                       // DB pass (Sched::tp_sms, hchunks: one or the other)
+    cudaEvent_t hfork = nullptr, hjoin = nullptr;
     cudaEvent_t hev[kMaxHChunks] = {};  // chunk c's packed ciphertexts are final
     ~Lane() {
         for (auto& e : hev)
             if (e) cudaEventDestroy(e);
         if (hjoin) cudaEventDestroy(hjoin);
+        if (hfork) cudaEventDestroy(hfork);
         if (hstream) cudaStreamDestroy(hstream);
         if (rgsw_ready) cudaEventDestroy(rgsw_ready);
         if (join) cudaEventDestroy(join);
@@ -222,12 +224,17 @@ size_t auto_scan_segments(float ms);
 // The DB-bound phase (query prep, mat-vec, tensor pass, finalize) of lane
 // slots [q_off, q_off + count) on st: packed ciphertext b parts into
 // L.packed_b.  lwe_ready: an event the mat-vec waits for (the key side runs
-// first); qprep_parts: 3 keys and RGSW parts, 1 keys only.  Returns launches.
+// first); prep_rgsw: the RGSW parts are prepared here as well.  Returns launches.
 int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t count, cudaStream_t st,
-                 cudaEvent_t* ev, cudaEvent_t lwe_ready = nullptr, int qprep_parts = 3);
+                 cudaEvent_t* ev, cudaEvent_t lwe_ready = nullptr, bool prep_rgsw = true);
 // H2D of parts [p0, p0 + np) (0, 1: LWE limbs, 2: KSK5, 3: KSK-1, 4: RGSW) of
 // each query into the handle's lane, one copy per contiguous host run.
 void stage_parts(const Server& S, const ipir_query_view* qs, size_t count, int p0, int np, cudaStream_t st);
+// Copies what the mat-vec and the tensor pass read of the queries: the KSK
+// parts on the handle's stream, the LWE vectors on the lane's copy stream.
+// Returns the event of the latter, or null if all of it went to the handle's
+// stream (a small batch, its RGSW parts with it if `rgsw`).
+cudaEvent_t stage_split(const Server& S, const ipir_query_view* qs, size_t count, bool rgsw);
 // Waits for the work enqueued on st, then throws (and clears the word, on
 // st) if a kernel's bounded wait ran out or a kernel stopped early.
 void check_device_error(Lane& L, cudaStream_t st);

@@ -128,12 +128,14 @@ int ipir_b200_shard_pack(ipir_shard* sh, const ipir_query_view* queries, size_t 
         IPB_CK(cudaSetDevice(S->device));
         ipb::Lane& L = S->lane;
         const ipb::Sched& sc = ipb::sched_for(*S, count);
-        ipb::stage_parts(*S, queries, count, 0, 4, S->stream);  // LWE vectors and KSK parts; no RGSW
+        // LWE vectors and KSK parts; no RGSW
+        const cudaEvent_t lwe_ready = ipb::stage_split(*S, queries, count, false);
         const size_t ns = ipb::slices_of(count, sc), slice = sc.slice > 0 ? (size_t)sc.slice : count;
         for (size_t k = 0; k < ns; ++k) {
             const size_t q0 = k * slice;
             S->launches += (unsigned long long)ipb::run_db_phase(*S, L, sc, q0, std::min(slice, count - q0),
-                                                                 S->stream, nullptr, nullptr, 1);
+                                                                 S->stream, nullptr, k == 0 ? lwe_ready : nullptr,
+                                                                 false);
         }
         ipb::check_device_error(L, S->stream);  // nothing is written if a kernel stopped early
         IPB_CK(cudaMemcpyAsync(out_packed_b, L.packed_b, count * S->pb_qstride * 4, cudaMemcpyDeviceToDevice,
@@ -198,8 +200,8 @@ int ipir_b200_horner_answer(ipir_horner* h, const uint32_t* packed_b, const ipir
         IPB_CK(cudaEventRecord(L.fork, static_cast<cudaStream_t>(stream)));
         IPB_CK(cudaStreamWaitEvent(S->stream, L.fork, 0));
         ipb::stage_parts(*S, queries, count, 4, 1, S->stream);  // RGSW parts only
-        IPB_CK(launch_qprep_parts(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, L.kplanes, L.keys, L.rgsw32,
-                                  (int)count, 2, S->stream));
+        IPB_CK(launch_qprep(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, nullptr, nullptr, L.rgsw32, nullptr,
+                            (int)count, ipb::kPrepRgsw, S->stream));
         const size_t ns = ipb::slices_of(count, sc), slice = sc.slice > 0 ? (size_t)sc.slice : count;
         for (size_t k = 0; k < ns; ++k) {
             const size_t q0 = k * slice, n = std::min(slice, count - q0);

@@ -75,6 +75,16 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
+// A persistent kernel's work-item counter c[0] and CTA count c[1] go back to
+// zero with the launch's last CTA (one thread of every CTA calls this once its
+// CTA takes no more items), so no memset precedes a launch.
+__device__ __forceinline__ void release_counter(unsigned* c) {
+    __threadfence();
+    if (atomicAdd(c + 1, 1u) == gridDim.x - 1) {
+        c[0] = 0;
+        c[1] = 0;
+    }
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 

@@ -187,7 +187,7 @@ struct TpParams {
     int acc_stages;
     uint32_t tmem_cols;
     int* err;
-    unsigned* tiles;       // work-item counter, zero at launch
+    unsigned* tiles;       // [0] work-item counter, [1] CTAs done: both zero between launches
     int has_qmap;          // output row of pass query p: qmap[p] (else p)
     uint8_t qmap[32];
     uint32_t c[2][7];      // 256^k mod q_l
@@ -197,8 +197,8 @@ struct TpParams {
                            // the abort path, IPB_TEST_ABORT_AFTER_ITEMS); 0: off
 };
 
-// Persistent, one CTA per SM, work items (MTI consecutive tiles) taken from a
-// per-launch atomic counter by the producer and published to the MMA thread
+// Persistent, one CTA per SM, work items (MTI consecutive tiles) taken from an
+// atomic counter by the producer and published to the MMA thread
 // and the epilogue through a ring of shared slots (-1 ends it), so SMs held
 // by other kernels at launch take fewer items.  Warps: 0 producer (one
 // thread: MTI bulk copies of 16 KB and one key-plane tile per stage), 1 TMEM
@@ -228,6 +228,7 @@ __global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_const
     __shared__ uint64_t ifull[kRing], iempty[kRing];
     __shared__ uint64_t mma_done;  // the MMA issuer's final commit: all its MMAs have completed
 
+    let_next_start();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -245,6 +246,7 @@ __global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    after_previous();
     const uint32_t tmem_base = *tmem_slot;
     const int acc_cols = MTI * P.nb;
 
@@ -380,6 +382,7 @@ __global__ void __launch_bounds__(kTpThreads, 1) tp_tc_kernel(const __grid_const
     }
     tc_fence_before();
     __syncthreads();
+    if (threadIdx.x == 0) release_counter(P.tiles);
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(P.tmem_cols));
@@ -501,9 +504,7 @@ cudaError_t launch_tensor_pass(const uint8_t* Dt, int tile0, int n_tiles, const 
     CUtensorMap mb;
     if (!make_map_b(&mb, kplanes, nq)) return cudaErrorInvalidValue;
     const size_t smem = 1024 + (size_t)P.stages * stage_bytes + (2 * P.stages + 4) * 8 + 16;
-    if ((e = cudaMemsetAsync(tiles, 0, sizeof(unsigned), s))) return e;
-    kernel<<<std::min(P.n_items, sms), kTpThreads, smem, s>>>(mb, P);
-    return cudaGetLastError();
+    return launch_overlapped(kernel, std::min(P.n_items, sms), kTpThreads, smem, s, mb, P);
 }
 
 }  // namespace ipb
