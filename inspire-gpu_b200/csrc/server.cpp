@@ -20,6 +20,7 @@
 
 #include "inspire_b200.h"
 #include "inspire_b200.hpp"
+#include "host_upload.h"
 #include "server_internal.h"
 
 namespace ipb {
@@ -60,7 +61,6 @@ DevTables* upload_tables(DevArena& A, cudaStream_t s) {
     return d;
 }
 
-// gpu_preprocess (reference src/gpu_protocol.cu:535-817) on one stream.
 void alloc_precomp(Precomp& P, cudaStream_t s) {
     const size_t R = P.pp.db_rows, C = P.pp.db_cols, G = P.pp.n_packed;
     DevArena& A = P.arena;
@@ -71,6 +71,31 @@ void alloc_precomp(Precomp& P, cudaStream_t s) {
     P.pre_df = A.alloc<uint32_t>(G * kGroupStrideF);
 }
 
+namespace {
+// The upload's stream and, per staging buffer, when its copy and its encode
+// are done.
+struct CopyStream {
+    cudaStream_t s = nullptr;
+    cudaEvent_t copied[2] = {}, encoded[2] = {};
+    CopyStream() {
+        IPB_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        for (int k = 0; k < 2; ++k) {
+            IPB_CK(cudaEventCreateWithFlags(&copied[k], cudaEventDisableTiming));
+            IPB_CK(cudaEventCreateWithFlags(&encoded[k], cudaEventDisableTiming));
+        }
+    }
+    ~CopyStream() {
+        if (s) cudaStreamSynchronize(s);
+        for (int k = 0; k < 2; ++k) {
+            if (copied[k]) cudaEventDestroy(copied[k]);
+            if (encoded[k]) cudaEventDestroy(encoded[k]);
+        }
+        if (s) cudaStreamDestroy(s);
+    }
+};
+}  // namespace
+
+// gpu_preprocess (reference src/gpu_protocol.cu:535-817).
 // P.pp is the geometry P holds.  For a group shard (global != null), P.pp
 // covers groups [g0, g0 + P.pp.n_packed) of the global database: the encode
 // mixes the D_act column polynomials of each row block across groups, so it
@@ -88,41 +113,39 @@ static void preprocess_into(Precomp& P, const uint16_t* db_host, cudaStream_t s,
     DevArena tmp;
     try {
         // ---- encode (in-place inverse DFT over D_act column polys per row block)
-        if (d_act <= 1) {
+        // Chunks of rows alternate between two staging buffers: one is copied to
+        // the device on a stream of its own while the other is encoded.
+        HostUpload up(db_host, R * Cg * sizeof(uint16_t));
+        if (d_act <= 1 && C == Cg) {
+            up.copy(P.db, db_host, R * C * sizeof(uint16_t), s);
+        } else if (d_act <= 1) {
             IPB_CK(cudaMemcpy2DAsync(P.db, C * sizeof(uint16_t), db_host + col0, Cg * sizeof(uint16_t),
                                      C * sizeof(uint16_t), R, cudaMemcpyHostToDevice, s));
-        } else if (global) {
-            int logd = 0;
-            while (((size_t)1 << logd) < d_act) ++logd;
-            const int nlA = std::min(logd, 4), nlB = logd - nlA;
-            const uint32_t dinv = inv_mod_p((uint32_t)d_act);
-            const size_t row_bytes = Cg * sizeof(uint16_t);
-            const size_t chunk_rows = std::max<size_t>(1, std::min<size_t>(R, (size_t)(256u << 20) / row_bytes));
-            uint16_t* staging = tmp.alloc<uint16_t>(chunk_rows * Cg);
-            uint16_t* enc = tmp.alloc<uint16_t>(chunk_rows * Cg);
-            for (size_t r0 = 0; r0 < R; r0 += chunk_rows) {
-                const size_t nr = std::min(chunk_rows, R - r0);
-                IPB_CK(cudaMemcpyAsync(staging, db_host + r0 * Cg, nr * row_bytes, cudaMemcpyHostToDevice, s));
-                IPB_CK(launch_encode_pass(staging, enc, nr, Cg, d_act, logd, 0, nlA, true, nlB == 0, dinv, s));
-                if (nlB > 0)
-                    IPB_CK(launch_encode_pass(nullptr, enc, nr, Cg, d_act, logd, nlA, nlB, false, true, dinv, s));
-                IPB_CK(cudaMemcpy2DAsync(P.db + r0 * C, C * sizeof(uint16_t), enc + col0, row_bytes,
-                                         C * sizeof(uint16_t), nr, cudaMemcpyDeviceToDevice, s));
-            }
         } else {
             int logd = 0;
             while (((size_t)1 << logd) < d_act) ++logd;
             const int nlA = std::min(logd, 4), nlB = logd - nlA;
             const uint32_t dinv = inv_mod_p((uint32_t)d_act);
-            const size_t row_bytes = C * sizeof(uint16_t);
-            const size_t chunk_rows = std::max<size_t>(1, std::min<size_t>(R, (size_t)(256u << 20) / row_bytes));
-            uint16_t* staging = tmp.alloc<uint16_t>(chunk_rows * C);
-            for (size_t r0 = 0; r0 < R; r0 += chunk_rows) {
+            const size_t row_bytes = Cg * sizeof(uint16_t);
+            const size_t chunk_rows = std::max<size_t>(1, std::min<size_t>(R, (size_t)(64u << 20) / row_bytes));
+            uint16_t* staging[2] = {tmp.alloc<uint16_t>(chunk_rows * Cg), tmp.alloc<uint16_t>(chunk_rows * Cg)};
+            uint16_t* const enc = global ? tmp.alloc<uint16_t>(chunk_rows * Cg) : nullptr;
+            CopyStream cs;
+            size_t k = 0;
+            for (size_t r0 = 0; r0 < R; r0 += chunk_rows, k ^= 1) {
                 const size_t nr = std::min(chunk_rows, R - r0);
-                IPB_CK(cudaMemcpyAsync(staging, db_host + r0 * C, nr * row_bytes, cudaMemcpyHostToDevice, s));
-                IPB_CK(launch_encode_pass(staging, P.db + r0 * C, nr, C, d_act, logd, 0, nlA, true, nlB == 0, dinv, s));
+                uint16_t* const dst = global ? enc : P.db + r0 * C;
+                IPB_CK(cudaStreamWaitEvent(cs.s, cs.encoded[k], 0));
+                up.copy(staging[k], db_host + r0 * Cg, nr * row_bytes, cs.s);
+                IPB_CK(cudaEventRecord(cs.copied[k], cs.s));
+                IPB_CK(cudaStreamWaitEvent(s, cs.copied[k], 0));
+                IPB_CK(launch_encode_pass(staging[k], dst, nr, Cg, d_act, logd, 0, nlA, true, nlB == 0, dinv, s));
+                IPB_CK(cudaEventRecord(cs.encoded[k], s));
                 if (nlB > 0)
-                    IPB_CK(launch_encode_pass(nullptr, P.db + r0 * C, nr, C, d_act, logd, nlA, nlB, false, true, dinv, s));
+                    IPB_CK(launch_encode_pass(nullptr, dst, nr, Cg, d_act, logd, nlA, nlB, false, true, dinv, s));
+                if (global)
+                    IPB_CK(cudaMemcpy2DAsync(P.db + r0 * C, C * sizeof(uint16_t), enc + col0, row_bytes,
+                                             C * sizeof(uint16_t), nr, cudaMemcpyDeviceToDevice, s));
             }
         }
         // ---- CRS polys a~_r = NTT(tau_{2N-1}(expand_seed("rlwe", r)))  (src/gpu_protocol.cu:569-582)
