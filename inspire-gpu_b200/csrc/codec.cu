@@ -37,15 +37,14 @@ __device__ __forceinline__ uint64_t crt_garner(uint32_t v0, uint32_t v1, const D
     return (uint64_t)v1 + (uint64_t)kQ1 * h;
 }
 
-// Query: packed bytes [q][bytes] -> flat u64 [q][2R + 6 d_eff 2 N].
+// Query: values [v0, v1) of packed bytes [q][bytes] -> flat u64 [q][2R + 6 d_eff 2 N].
 __global__ void __launch_bounds__(256) query_unpack_kernel(const uint8_t* __restrict__ in, size_t in_stride,
                                                            size_t in_bytes, uint64_t* __restrict__ out,
-                                                           size_t out_stride, size_t R,
+                                                           size_t out_stride, size_t R, size_t v0, size_t v1,
                                                            const DevTables* __restrict__ T) {
-    const size_t nv = R + (size_t)6 * kDeff * kN;
     const uint8_t* src = in + (size_t)blockIdx.y * in_stride;
     uint64_t* dst = out + (size_t)blockIdx.y * out_stride;
-    for (size_t v = (size_t)blockIdx.x * 256 + threadIdx.x; v < nv; v += (size_t)gridDim.x * 256) {
+    for (size_t v = v0 + (size_t)blockIdx.x * 256 + threadIdx.x; v < v1; v += (size_t)gridDim.x * 256) {
         const size_t bit = v * kWireBits;
         const size_t b0 = bit >> 3;
         const int sh = (int)(bit & 7);
@@ -91,9 +90,11 @@ __global__ void __launch_bounds__(256) response_pack_kernel(const uint64_t* __re
     }
 }
 
-// u64 response -> u32 copy (canonical residues) for the in-place inverse NTT.
-__global__ void __launch_bounds__(256) narrow_kernel(const uint64_t* __restrict__ in, uint32_t* __restrict__ out,
-                                                    size_t n) {
+// u64 responses -> u32 copies (canonical residues) for the in-place inverse NTT.
+__global__ void __launch_bounds__(256) narrow_kernel(const uint64_t* __restrict__ in, size_t in_stride,
+                                                    uint32_t* __restrict__ out, size_t n) {
+    in += (size_t)blockIdx.y * in_stride;
+    out += (size_t)blockIdx.y * n;
     for (size_t k = (size_t)blockIdx.x * 256 + threadIdx.x; k < n; k += (size_t)gridDim.x * 256)
         out[k] = (uint32_t)in[k];
 }
@@ -144,12 +145,14 @@ size_t wire_query_bytes(size_t rows) { return ((rows + (size_t)6 * kDeff * kN) *
 size_t wire_response_bytes(size_t num_cts) { return (num_cts * 2 * kN * kWireBits + 7) / 8; }
 size_t wire_compressed_bytes(size_t num_cts) { return num_cts * 12288; }
 
-cudaError_t launch_query_unpack(const uint8_t* in, size_t in_stride, size_t rows, uint64_t* out, size_t out_stride,
-                                int nq, const DevTables* T, cudaStream_t s) {
-    if (nq <= 0) return cudaSuccess;
-    const size_t nv = rows + (size_t)6 * kDeff * kN;
-    query_unpack_kernel<<<dim3(grid_for(nv), nq), 256, 0, s>>>(in, in_stride, wire_query_bytes(rows), out, out_stride,
-                                                              rows, T);
+size_t wire_query_value_byte(size_t v) { return v * kWireBits / 8; }
+
+cudaError_t launch_query_unpack(const uint8_t* in, size_t in_stride, size_t rows, size_t v0, size_t v1, uint64_t* out,
+                                size_t out_stride, int nq, const DevTables* T, cudaStream_t s) {
+    if (nq <= 0 || v0 >= v1) return cudaSuccess;
+    if (v1 > rows + (size_t)6 * kDeff * kN) return cudaErrorInvalidValue;
+    query_unpack_kernel<<<dim3(grid_for(v1 - v0), nq), 256, 0, s>>>(in, in_stride, wire_query_bytes(rows), out,
+                                                                    out_stride, rows, v0, v1, T);
     return cudaGetLastError();
 }
 
@@ -165,13 +168,11 @@ cudaError_t launch_response_compress(const uint64_t* flat, size_t flat_stride, s
                                      uint8_t* out, size_t out_stride, int nq, const DevTables* T, cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
     const size_t per_q = num_cts * 4 * kN;  // u32 coefficients per query in tmp
-    for (int q = 0; q < nq; ++q) {
-        narrow_kernel<<<grid_for(per_q), 256, 0, s>>>(flat + (size_t)q * flat_stride, tmp + (size_t)q * per_q, per_q);
-        cudaError_t e = cudaGetLastError();
-        if (e) return e;
-    }
+    narrow_kernel<<<dim3(grid_for(per_q), nq), 256, 0, s>>>(flat, flat_stride, tmp, per_q);
+    cudaError_t e = cudaGetLastError();
+    if (e) return e;
     // poly index (q * num_cts + ct) * 4 + ab * 2 + limb: limb = index & 1
-    cudaError_t e = launch_ntt_batch(tmp, (size_t)nq * num_cts * 4, 1, true, T, s);
+    e = launch_ntt_batch(tmp, (size_t)nq * num_cts * 4, 1, true, T, s);
     if (e) return e;
     response_compress_kernel<<<dim3(grid_for(num_cts * kN), nq), 256, 0, s>>>(tmp, per_q, num_cts, out, out_stride,
                                                                                T);

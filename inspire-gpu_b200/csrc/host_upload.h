@@ -3,8 +3,9 @@
 // The driver stages a pageable copy through one thread (about 10 GB/s), which
 // was most of preprocessing: a 1 GB database took 123 ms, 14 of them kernels.
 // Here several threads fill pinned slots and enqueue the copies, so the upload
-// runs nearer the PCIe rate.  Buffers that are already pinned (or not host
-// memory), and small ones, are copied directly.
+// runs nearer the PCIe rate (four threads: 60 ms for that database; two 79,
+// eight 68).  Buffers that are already pinned (or not host memory), and small
+// ones, are copied directly.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -32,7 +33,7 @@ class HostUpload {
         }
         if (a.type != cudaMemoryTypeUnregistered || bytes < kMinBytes) return;
         if (cudaGetDevice(&device_) != cudaSuccess) return;
-        const size_t n = std::max(1u, std::min(8u, std::thread::hardware_concurrency() / 2));
+        const size_t n = std::max(1u, std::min(4u, std::thread::hardware_concurrency() / 2));
         void* p = nullptr;
         if (cudaHostAlloc(&p, n * 2 * kSlot, cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError();
@@ -77,7 +78,7 @@ class HostUpload {
     }
 
   private:
-    static constexpr size_t kSlot = (size_t)512 << 10;
+    static constexpr size_t kSlot = (size_t)1 << 20;
     static constexpr size_t kMinBytes = (size_t)32 << 20;
 
     void work(size_t id) {

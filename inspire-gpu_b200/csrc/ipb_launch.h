@@ -131,9 +131,13 @@ cudaError_t launch_horner_cluster8(const uint32_t* pre_a, const uint32_t* packed
 size_t wire_query_bytes(size_t rows);
 size_t wire_response_bytes(size_t num_cts);
 size_t wire_compressed_bytes(size_t num_cts);
-// nq packed queries (in_stride bytes apart) -> flat u64 queries.
-cudaError_t launch_query_unpack(const uint8_t* in, size_t in_stride, size_t rows, uint64_t* out, size_t out_stride,
-                                int nq, const DevTables* T, cudaStream_t s);
+// Values [v0, v1) of nq packed queries (in_stride bytes apart; R LWE
+// coefficients, then the KSK5, KSK-1 and RGSW polynomials) -> flat u64 queries.
+// Value v starts in byte wire_query_value_byte(v), at its first bit if v is a
+// multiple of 8.
+size_t wire_query_value_byte(size_t v);
+cudaError_t launch_query_unpack(const uint8_t* in, size_t in_stride, size_t rows, size_t v0, size_t v1, uint64_t* out,
+                                size_t out_stride, int nq, const DevTables* T, cudaStream_t s);
 // nq flat u64 responses -> packed responses (out_stride bytes apart).
 cudaError_t launch_response_pack(const uint64_t* flat, size_t flat_stride, size_t num_cts, uint8_t* out,
                                  size_t out_stride, int nq, const DevTables* T, cudaStream_t s);

@@ -10,17 +10,16 @@
 // q's B[i] (K-major rows built by qplanes_kernel).  One
 // tcgen05.mma.kind::i8 chain accumulates D[m'][n] = sum_i A'[m'][i] B[n][i]
 // in s32 TMEM.  With K <= 32768 rows per chunk every D entry is
-// <= 255*255*32768 < 2^31: exact.  The epilogue forms, per limb,
-// sum_k (256^k mod q_l) D[m'][n_k] (< 2^61) in each of the lo and hi byte
-// rows and combines them as (lo + 256 (hi mod q_l)) mod q_l: the exact
-// sum_i db[i][j] b_{q,l}[i] mod q_l.  All arithmetic stays exact, so the
-// result equals the reference's.  Seven planes per query instead of four
+// <= 255*255*32768 < 2^31: exact.  The epilogue forms, per limb, the sum over
+// both byte rows of sum_k (256^(k + byte) mod q_l) D[m'][n_k] (< 2^62) and
+// reduces it: the exact sum_i db[i][j] b_{q,l}[i] mod q_l.  All arithmetic
+// stays exact, so the result equals the reference's.  Seven planes per query instead of four
 // per limb: 12.5 % fewer MMAs and query-plane bytes.
 //
-// CTA roles (256 threads): warp 0 issues TMA loads (DB tile 256 x 64 rows as
+// CTA roles (384 threads): warp 0 issues TMA loads (DB tile 256 x 64 rows as
 // two 128-byte boxes, query planes N x 64), warp 1 allocates TMEM and one
-// thread issues the MMAs, warps 4..7 drain TMEM (tcgen05.ld) and write
-// partial sums.  Stages are recycled through mbarriers; every wait is
+// thread issues the MMAs, warps 4..11 drain TMEM (tcgen05.ld), four each half
+// of the tile, and write partial sums.  Stages are recycled through mbarriers; every wait is
 // bounded and reports a timeout through *err instead of hanging.
 //
 // Work items (m'-tile, K-chunk) are handed out dynamically: the producer
@@ -58,7 +57,7 @@ struct TcParams {
     size_t ld;             // columns per (chunk, limb) row of part
     int nq;                // queries in this pass (<= 32)
     int npad;              // N = 16 ceil(7 nq / 16) (<= 224)
-    uint32_t c[2][kPlanes];  // 256^k mod q_l
+    uint32_t c[2][kPlanes + 1];  // 256^k mod q_l
     int n_mtiles;
     int mt_per_range;      // > 0: the m' tiles cover ranges of this many tiles, range r starting
     int range_stride_m;    // r * range_stride_m m' rows after the first (several column ranges in one
@@ -84,7 +83,10 @@ __device__ __forceinline__ int mtile_m0(const TcParams& P, int mt) {
     return P.mt_per_range ? (mt / P.mt_per_range) * P.range_stride_m + (mt % P.mt_per_range) * kMT : mt * kMT;
 }
 
-__global__ void __launch_bounds__(256, 1) mv_tc_kernel(const __grid_constant__ CUtensorMap map_a,
+constexpr int kMvThreads = 384;
+constexpr int kEpiThreads = 256;
+
+__global__ void __launch_bounds__(kMvThreads, 1) mv_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                                        const __grid_constant__ CUtensorMap map_b, TcParams P) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -108,8 +110,8 @@ __global__ void __launch_bounds__(256, 1) mv_tc_kernel(const __grid_constant__ C
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], 128); }
-        for (int r = 0; r < kRing; ++r) { mbar_init(&ifull[r], 1); mbar_init(&iempty[r], 1 + 128); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], kEpiThreads); }
+        for (int r = 0; r < kRing; ++r) { mbar_init(&ifull[r], 1); mbar_init(&iempty[r], 1 + kEpiThreads); }
         mbar_init(&mma_done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -223,11 +225,25 @@ __global__ void __launch_bounds__(256, 1) mv_tc_kernel(const __grid_constant__ C
         }
     } else if (warp >= 4) {
         // ---------------- epilogue: TMEM -> u64 dot products -> mod q
-        const int wq = warp & 3;
+        // An accumulator set of more than 256 columns (more than 18 queries)
+        // is not double-buffered: the MMAs wait while it is drained, so the
+        // epilogue's length counts.  Two warps per TMEM lane quarter, one half
+        // of the m' tile each; the weights of the lane's byte row (lo bytes in
+        // even lanes, hi in odd) are in registers, and the pair of lanes of a
+        // column meets once per query in 64 bits: the even lane reduces and
+        // writes limb 0, the odd one limb 1.
+        const int wq = warp & 3, mb = (warp - 4) >> 2, hi = lane & 1;
         const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
         int as = 0;
         uint32_t aph = 0;
-        const uint64_t cr0 = P.T->limb[0].cr, cr1 = P.T->limb[1].cr;
+        const uint64_t cr = P.T->limb[hi].cr;
+        const uint32_t ql = hi ? kQ1 : kQ0;
+        uint32_t w0[kPlanes], w1[kPlanes];
+#pragma unroll
+        for (int k = 0; k < kPlanes; ++k) {
+            w0[k] = P.c[0][k + hi];
+            w1[k] = P.c[1][k + hi];
+        }
         for (int it = 0;; ++it) {
             const int r = it % kRing;
             if (!mbar_wait_ab(&ifull[r], (uint32_t)(it / kRing) & 1, P.err, 8, &abort_flag)) { abort_flag = 1; break; }
@@ -238,52 +254,42 @@ __global__ void __launch_bounds__(256, 1) mv_tc_kernel(const __grid_constant__ C
             tc_fence_after();
             const int mt = item % P.n_mtiles, kc = item / P.n_mtiles;
             const int m0 = mtile_m0(P, mt);
-            for (int mb = 0; mb < 2; ++mb) {
-                const size_t j = ((size_t)m0 + mb * 128 + wq * 32 + lane) >> 1;
-                for (int q0 = 0; q0 < P.nq; q0 += 8) {
-                    // queries q0..q0+7: columns 7 q0 .. 7 q0 + 55, seven 8-column
-                    // loads (those at or past N are not loaded: they hold no query)
-                    uint32_t t[kPlanes][8];
+            const size_t col = ((size_t)m0 + mb * 128 + wq * 32 + lane) >> 1;
+            uint32_t* const out = P.part + ((size_t)kc * 2 + hi) * P.ld + col;
+            const uint32_t acc = tmem_base + lane_base + (uint32_t)(as * 2 * P.npad + mb * P.npad);
+            for (int q0 = 0; q0 < P.nq; q0 += 8) {
+                // queries q0..q0+7: columns 7 q0 .. 7 q0 + 55, seven 8-column
+                // loads (those at or past N are not loaded: they hold no query)
+                uint32_t t[kPlanes][8];
 #pragma unroll
-                    for (int c = 0; c < kPlanes; ++c) {
-                        const int col = kPlanes * q0 + 8 * c;
-                        if (col < P.npad) {
-                            tmem_ld8_issue(tmem_base + lane_base + (uint32_t)(as * 2 * P.npad + mb * P.npad + col),
-                                           t[c]);
-                        } else {
+                for (int c = 0; c < kPlanes; ++c) {
+                    const int n = kPlanes * q0 + 8 * c;
+                    if (n < P.npad) {
+                        tmem_ld8_issue(acc + (uint32_t)n, t[c]);
+                    } else {
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) t[c][e] = 0;
-                        }
+                        for (int e = 0; e < 8; ++e) t[c][e] = 0;
                     }
-                    uint32_t v[kPlanes * 8];
+                }
+                uint32_t v[kPlanes * 8];
 #pragma unroll
-                    for (int c = 0; c < kPlanes; ++c) {
-                        tmem_wait8(t[c]);  // one wait for all seven loads; the others are no-ops
+                for (int c = 0; c < kPlanes; ++c) {
+                    tmem_wait8(t[c]);  // one wait for all seven loads; the others are no-ops
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) v[8 * c + e] = t[c][e];
+                    for (int e = 0; e < 8; ++e) v[8 * c + e] = t[c][e];
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    if (q0 + e >= P.nq) break;
+                    uint64_t a0 = 0, a1 = 0;
+#pragma unroll
+                    for (int k = 0; k < kPlanes; ++k) {
+                        a0 += (uint64_t)w0[k] * v[kPlanes * e + k];
+                        a1 += (uint64_t)w1[k] * v[kPlanes * e + k];
                     }
-                    // per limb sum_k (256^k mod q) D[row][7 q + k] (< 2^61); lane
-                    // 2j+1 holds the hi DB byte's sums, lane 2j the lo byte's:
-                    // result = (lo + 256 (hi mod q)) mod q
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        uint64_t a0 = 0, a1 = 0;
-#pragma unroll
-                        for (int k = 0; k < kPlanes; ++k) {
-                            a0 += (uint64_t)P.c[0][k] * v[kPlanes * e + k];
-                            a1 += (uint64_t)P.c[1][k] * v[kPlanes * e + k];
-                        }
-                        const uint32_t h0 = (lane & 1) ? mod_u64(a0, cr0, kQ0) : 0u;
-                        const uint32_t h1 = (lane & 1) ? mod_u64(a1, cr1, kQ1) : 0u;
-                        const uint32_t p0 = __shfl_down_sync(0xffffffffu, h0, 1);
-                        const uint32_t p1 = __shfl_down_sync(0xffffffffu, h1, 1);
-                        if ((lane & 1) == 0 && q0 + e < P.nq) {
-                            const int qo = P.has_qmap ? P.qmap[q0 + e] : q0 + e;
-                            uint32_t* dst = P.part + (size_t)qo * P.part_qstride + (size_t)kc * 2 * P.ld + j;
-                            dst[0] = mod_u64(a0 + ((uint64_t)p0 << 8), cr0, kQ0);
-                            dst[P.ld] = mod_u64(a1 + ((uint64_t)p1 << 8), cr1, kQ1);
-                        }
-                    }
+                    const uint64_t sum = (hi ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hi ? a0 : a1, 1);
+                    const int qo = P.has_qmap ? P.qmap[q0 + e] : q0 + e;
+                    out[(size_t)qo * P.part_qstride] = mod_u64(sum, cr, ql);
                 }
             }
             tc_fence_before();
@@ -427,7 +433,7 @@ cudaError_t launch_matvec_tc_ranges(const uint16_t* db, size_t rows, size_t ld, 
         const uint32_t qs[2] = {kQ0, kQ1};
         for (int l = 0; l < 2; ++l) {
             uint64_t c = 1;
-            for (int k = 0; k < kPlanes; ++k, c = c * 256 % qs[l]) P.c[l][k] = (uint32_t)c;
+            for (int k = 0; k <= kPlanes; ++k, c = c * 256 % qs[l]) P.c[l][k] = (uint32_t)c;
         }
     }
     P.mt_per_range = n_ranges > 1 ? (int)((2 * cols_per_range) / kMT) : 0;
@@ -452,7 +458,7 @@ cudaError_t launch_matvec_tc_ranges(const uint16_t* db, size_t rows, size_t ld, 
     if (e) return e;
     const int items = P.n_mtiles * P.n_kchunks;
     const int grid = std::min(items, std::max(1, num_sms));
-    return launch_overlapped(mv_tc_kernel, grid, 256, smem, s, ma, mb, P);
+    return launch_overlapped(mv_tc_kernel, grid, kMvThreads, smem, s, ma, mb, P);
 }
 
 }  // namespace ipb

@@ -841,6 +841,31 @@ cudaEvent_t stage_split(const Server& S, const ipir_query_view* qs, size_t count
     return L.join;
 }
 
+// The pipeline of a batch whose KSK parts are in place on the handle's stream,
+// whose LWE vectors are from lwe_ready on, and whose RGSW parts the lane's copy
+// stream has brought: these are prepared there.
+static void run_split(Server* S, const Sched& sc, size_t count, cudaEvent_t lwe_ready) {
+    Lane& L = S->lane;
+    IPB_CK(launch_qprep(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, nullptr, nullptr, L.rgsw32, nullptr,
+                        (int)count, kPrepRgsw, L.aux));
+    IPB_CK(cudaEventRecord(L.rgsw_ready, L.aux));
+    S->launches += 1;
+    if (chunked_ok(*S, sc, count)) {
+        S->launches += (unsigned long long)run_chunked(*S, L, sc, count, S->stream, lwe_ready, L.rgsw_ready);
+        return;
+    }
+    // The first slice's key side starts before the LWE vectors land; every
+    // slice's RGSW parts were prepared on the copy stream above.
+    const size_t ns = slices_of(count, sc), slice = sc.slice > 0 ? (size_t)sc.slice : count;
+    for (size_t k = 0; k < ns; ++k) {
+        const size_t q0 = k * slice, n = std::min(slice, count - q0);
+        S->launches += (unsigned long long)run_db_phase(*S, L, sc, q0, n, S->stream, nullptr,
+                                                        k == 0 ? lwe_ready : nullptr, false);
+        if (k == 0) IPB_CK(cudaStreamWaitEvent(S->stream, L.rgsw_ready, 0));
+        S->launches += (unsigned long long)run_horner_phase(*S, L, sc, q0, n, S->stream, nullptr);
+    }
+}
+
 // The blocking answer from host views.  Beyond a small batch the KSK parts
 // are copied first and the query prep and tensor pass (which need only them)
 // start while the LWE vectors and then the RGSW parts cross PCIe on the lane's
@@ -865,24 +890,7 @@ static void stage_and_run(Server* S, const ipir_query_view* qs, size_t count) {
         return;
     }
     stage_parts(*S, qs, count, 4, 1, L.aux);      // RGSW parts: needed by the Horner chains
-    IPB_CK(launch_qprep(L.qraw, S->qstride, S->pp.db_rows, S->pre->tables, nullptr, nullptr, L.rgsw32, nullptr,
-                        (int)count, kPrepRgsw, L.aux));
-    IPB_CK(cudaEventRecord(L.rgsw_ready, L.aux));
-    S->launches += 1;
-    if (chunked_ok(*S, sc, count)) {
-        S->launches += (unsigned long long)run_chunked(*S, L, sc, count, S->stream, lwe_ready, L.rgsw_ready);
-        return;
-    }
-    // The first slice's key side starts before the LWE vectors land; every
-    // slice's RGSW parts were prepared on the second stream above.
-    const size_t ns = slices_of(count, sc), slice = sc.slice > 0 ? (size_t)sc.slice : count;
-    for (size_t k = 0; k < ns; ++k) {
-        const size_t q0 = k * slice, n = std::min(slice, count - q0);
-        S->launches += (unsigned long long)run_db_phase(*S, L, sc, q0, n, S->stream, nullptr,
-                                                        k == 0 ? lwe_ready : nullptr, false);
-        if (k == 0) IPB_CK(cudaStreamWaitEvent(S->stream, L.rgsw_ready, 0));
-        S->launches += (unsigned long long)run_horner_phase(*S, L, sc, q0, n, S->stream, nullptr);
-    }
+    run_split(S, sc, count, lwe_ready);
 }
 
 // A kernel whose pipeline wait ran out of iterations leaves a code in the
@@ -1059,15 +1067,34 @@ std::vector<Sched> autotune(const Server& S, Lane& L, cudaStream_t st) {
 }
 
 // ipir_answer_batch on packed queries: H2D of the packed bytes, unpack on
-// the device, the pipeline, then the response in the requested format.
+// the device, the pipeline, then the response in the requested format.  The
+// parts of a larger batch are copied and unpacked in the order of
+// stage_and_run.
 static void answer_wire(Server* S, const uint8_t* packed, size_t count, int fmt, void* out) {
     IPB_CK(cudaSetDevice(S->device));
     Lane& L = S->lane;
     const Precomp& P = *S->pre;
     cudaStream_t st = S->stream;
-    IPB_CK(cudaMemcpyAsync(L.wire_in, packed, count * S->wire_q, cudaMemcpyHostToDevice, st));
-    IPB_CK(launch_query_unpack(L.wire_in, S->wire_q, S->pp.db_rows, L.qraw, S->qstride, (int)count, P.tables, st));
-    run_pipeline(S, count);
+    const size_t R = S->pp.db_rows, keys_end = R + 2 * kDeff * kN, nv = R + 6 * kDeff * kN;  // all multiples of 8
+    if (count * S->wire_q <= kSmallBatchBytes || S->timing) {
+        IPB_CK(cudaMemcpyAsync(L.wire_in, packed, count * S->wire_q, cudaMemcpyHostToDevice, st));
+        IPB_CK(launch_query_unpack(L.wire_in, S->wire_q, R, 0, nv, L.qraw, S->qstride, (int)count, P.tables, st));
+        run_pipeline(S, count);
+    } else {
+        auto values = [&](size_t v0, size_t v1, cudaStream_t on) {
+            const size_t b0 = wire_query_value_byte(v0), b1 = v1 == nv ? S->wire_q : wire_query_value_byte(v1);
+            IPB_CK(cudaMemcpy2DAsync(L.wire_in + b0, S->wire_q, packed + b0, S->wire_q, b1 - b0, count,
+                                     cudaMemcpyHostToDevice, on));
+            IPB_CK(launch_query_unpack(L.wire_in, S->wire_q, R, v0, v1, L.qraw, S->qstride, (int)count, P.tables, on));
+        };
+        IPB_CK(cudaEventRecord(L.fork, st));
+        IPB_CK(cudaStreamWaitEvent(L.aux, L.fork, 0));
+        values(R, keys_end, st);
+        values(0, R, L.aux);
+        IPB_CK(cudaEventRecord(L.join, L.aux));
+        values(keys_end, nv, L.aux);
+        run_split(S, sched_for(*S, count), count, L.join);
+    }
     const void* src = L.resp;
     size_t bytes = count * S->resp_qstride * 8;
     if (fmt == 1) {
