@@ -67,9 +67,10 @@ cudaError_t launch_mv_chunk_reduce(const uint32_t* part, size_t part_qstride, in
 // 128-row tiles of 32 slots, 128 tiles per group in (group, limb, slot) order
 // (tp_tiles(groups) in all); kplanes: the queries' KSK5 byte planes,
 // kTpPlaneBytes apart; tp_out: [q][g][l][N] u32, out_qstride words per query.
-// A launch covers tiles [tile0, tile0 + n_tiles) for nq <= kTpMaxQueries
-// queries; query p's results go to row qmap[p] of tp_out (p without a map).
-constexpr int kTpMaxQueries = 32;
+// A launch covers tiles [tile0, tile0 + n_tiles) for nq <= kTpMaxPass queries
+// (32 with a map); query p's results go to row qmap[p] of tp_out (p without a map).
+constexpr int kTpMaxQueries = 32;  // per slice of a batch
+constexpr int kTpMaxPass = 64;
 constexpr size_t kTpPlaneBytes = (size_t)2 * 4 * 4096;
 size_t tp_dt_bytes(size_t groups);
 int tp_tiles(size_t groups);

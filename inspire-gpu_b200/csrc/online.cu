@@ -464,7 +464,11 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
     const uint32_t q = L.q, q_oth = T->limb[1 - l].q;
     const uint64_t carry = gp ? kCarry2 : kCarry1;
     const NttScale scale = L.scale_crt;
-    for (int i = threadIdx.x; i < kN; i += 512) { twf[i] = L.fwd[i]; twi[i] = L.inv[i]; }
+    const size_t start = (size_t)ct * d_act;
+    const size_t len = (start + d_act <= groups) ? d_act : groups - start;
+    const long i_first = hr.i_first < 0 ? (long)len - 2 : (long)hr.i_first;
+    const bool steps = i_first >= (long)hr.i_last;  // one group: the response is its packed ciphertext
+    for (int i = threadIdx.x; steps && i < kN; i += 512) { twf[i] = L.fwd[i]; twi[i] = L.inv[i]; }
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int k = 0; k < 2; ++k) { hb_init(&mbx[k]); hb_init(&mbc[k]); }
@@ -473,17 +477,15 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
     after_previous();  // the tables above are constant; what follows was written by this answer's kernels
     const uint32_t rank_limb = (uint32_t)((p << 1) | (1 - l));   // same poly, other limb
     const uint32_t rank_poly = (uint32_t)(((1 - p) << 1) | l);   // other poly, same limb
-    const size_t start = (size_t)ct * d_act;
-    const size_t len = (start + d_act <= groups) ? d_act : groups - start;
     const uint32_t* pbq = packed_b + (size_t)b * pb_qstride;
     auto src_of = [&](size_t i) -> const uint32_t* {
         return p ? pbq + (i * 2 + l) * kN : pre_a + (i * 2 + l) * kN;
     };
     // RGSW rows of this poly for digit gp: to own output (p' = p) and to the other (p' = 1 - p)
     const uint32_t* rg = rgsw32 + (size_t)b * (4 * kDeff * 2 * kN);
-    uint32_t r_self[8], r_oth[8];
-    ld8(rg + (size_t)(((2 * p + p) * kDeff + gp) * 2 + l) * kN + 8 * t, r_self);
-    ld8(rg + (size_t)(((2 * p + (1 - p)) * kDeff + gp) * 2 + l) * kN + 8 * t, r_oth);
+    uint32_t r_self[8] = {}, r_oth[8] = {};
+    if (steps) ld8(rg + (size_t)(((2 * p + p) * kDeff + gp) * 2 + l) * kN + 8 * t, r_self);
+    if (steps) ld8(rg + (size_t)(((2 * p + (1 - p)) * kDeff + gp) * 2 + l) * kN + 8 * t, r_oth);
     // Shoup factors of the fixed RGSW values: each product below is then
     // exact with one high multiply instead of a 64-bit Barrett reduction.
     uint32_t r_self_p[8], r_oth_p[8];
@@ -495,7 +497,6 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
     uint32_t acc[8] = {};
     uint32_t* const st_part = hr.state + (((size_t)b * (gridDim.x >> 2) + ct) * 4 + p * 2 + l) * kN;
     if (gp == 0) ld8((hr.i_first < 0 ? src_of(start + len - 1) : st_part) + 8 * t, acc);
-    const long i_first = hr.i_first < 0 ? (long)len - 2 : (long)hr.i_first;
     cluster_sync_all();  // every CTA runs and its mbarriers are initialised before any remote access
     const uint32_t peer_x = map_peer(xpart, rank_limb);
     const uint32_t peer_c = map_peer(cin, rank_poly);
@@ -608,7 +609,11 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     const uint32_t q_oth = T->limb[1 - l].q;
     const uint64_t carry = j ? kCarry2 : kCarry1;
     const NttScale scale = L.scale_crt;
-    for (int i = threadIdx.x; i < kN; i += 256) { twf[i] = L.fwd[i]; twi[i] = L.inv[i]; }
+    const size_t start = (size_t)ct * d_act;
+    const size_t len = (start + d_act <= groups) ? d_act : groups - start;
+    const long i_first = hr.i_first < 0 ? (long)len - 2 : (long)hr.i_first;
+    const bool steps = i_first >= (long)hr.i_last;  // one group: the response is its packed ciphertext
+    for (int i = threadIdx.x; steps && i < kN; i += 256) { twf[i] = L.fwd[i]; twi[i] = L.inv[i]; }
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int k = 0; k < 2; ++k) { hb_init(&mbx[k]); hb_init(&mbc[k]); }
@@ -619,16 +624,14 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     const uint32_t rank_sib = (uint32_t)((p << 2) | (l << 1) | (1 - j));    // same poly and limb, other digit
     const uint32_t rank_o0 = (uint32_t)(((1 - p) << 2) | (l << 1) | 0);     // other poly, same limb, digit 0
     const uint32_t rank_o1 = (uint32_t)(((1 - p) << 2) | (l << 1) | 1);     //                        digit 1
-    const size_t start = (size_t)ct * d_act;
-    const size_t len = (start + d_act <= groups) ? d_act : groups - start;
     const uint32_t* pbq = packed_b + (size_t)b * pb_qstride;
     auto src_of = [&](size_t i) -> const uint32_t* {
         return p ? pbq + (i * 2 + l) * kN : pre_a + (i * 2 + l) * kN;
     };
     const uint32_t* rg = rgsw32 + (size_t)b * (4 * kDeff * 2 * kN);
-    uint32_t r_self[8], r_oth[8];
-    ld8(rg + (size_t)(((2 * p + p) * kDeff + j) * 2 + l) * kN + 8 * t, r_self);
-    ld8(rg + (size_t)(((2 * p + (1 - p)) * kDeff + j) * 2 + l) * kN + 8 * t, r_oth);
+    uint32_t r_self[8] = {}, r_oth[8] = {};
+    if (steps) ld8(rg + (size_t)(((2 * p + p) * kDeff + j) * 2 + l) * kN + 8 * t, r_self);
+    if (steps) ld8(rg + (size_t)(((2 * p + (1 - p)) * kDeff + j) * 2 + l) * kN + 8 * t, r_oth);
     // Shoup factors of the fixed RGSW values: each product below is then
     // exact with one high multiply instead of a 64-bit Barrett reduction.
     uint32_t r_self_p[8], r_oth_p[8];
@@ -640,7 +643,6 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     uint32_t acc[8];
     uint32_t* const st_part = hr.state + (((size_t)b * (gridDim.x >> 3) + ct) * 4 + p * 2 + l) * kN;
     ld8((hr.i_first < 0 ? src_of(start + len - 1) : st_part) + 8 * t, acc);
-    const long i_first = hr.i_first < 0 ? (long)len - 2 : (long)hr.i_first;
     cluster_sync_all();  // every CTA runs and its mbarriers are initialised before any remote access
     const uint32_t peer_x = map_peer(xc, rank_limb);
     const uint32_t peer_mbx = map_peer(mbx, rank_limb);

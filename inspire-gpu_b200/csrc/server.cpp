@@ -407,9 +407,9 @@ static bool chunked_ok(const Server& S, const Sched& sc, size_t count);
 
 // Defaults per batch size, each line drawn where both sides measured alike
 // (one GPU, medians of interleaved runs):
-//   Horner kernel: 8 CTAs per chain while all clusters run at once (up to 8
+//   Horner kernel: 8 CTAs per chain while all clusters run at once (up to 15
 //     chains, 3.2 us a step), 4 CTAs beyond (4.0 us; 16 chains of 8 CTAs take
-//     5.0 us).
+//     5.1 us).
 //   Horner chain trailing the DB pass in chunks where a chunk's mat-vec lasts
 //     longer than its chain steps (32768 rows: 19 us a group against 4-11) and
 //     the chain is worth the extra launches: 128 groups, 16 GB: 1 query 3.68
@@ -435,7 +435,7 @@ std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
         Sched& sc = out[c];
         sc.tp_pass = gt_pass;
         if (m) sc.matvec_tc = std::strcmp(m, "simt") != 0;
-        sc.horner_cluster = c * S.pp.num_cts <= 8 ? 2 : 1;
+        sc.horner_cluster = c * S.pp.num_cts <= 15 ? 2 : 1;
         if (chain >= 64 && S.pp.db_rows >= 16384 && c <= std::min<size_t>(16, chain / 8)) {
             Sched chunked = sc;
             chunked.horner_cluster = 1;
@@ -459,7 +459,9 @@ std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
 // q_off: the batch's first lane slot (slices of a batch larger than one DB
 // pass run the whole phase on slots [q_off, q_off + count)).
 // prep_rgsw: the RGSW parts are prepared here too.
-int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t count, cudaStream_t st,
+// span: queries from q_off on that are prepared and go through the tensor
+// pass here (tp_span: this slice's, two slices', or none).
+int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t count, size_t span, cudaStream_t st,
                  cudaEvent_t* ev, cudaEvent_t lwe_ready, bool prep_rgsw) {
     const Params& pp = S.pp;
     const Precomp& P = *S.pre;
@@ -474,21 +476,22 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
     uint8_t* const kplanes = L.kplanes + q_off * kTpPlaneBytes;
     uint32_t* const tp_out = L.tp_out + q_off * S.pb_qstride;
     auto prep = [&](int parts) {
-        IPB_CK(launch_qprep(qraw, S.qstride, R, P.tables, kplanes, keys, L.rgsw32 + q_off * kRgswStride, planes, nq,
-                            parts, st));
-        ++launches;
+        IPB_CK(launch_qprep(qraw, S.qstride, R, P.tables, kplanes, keys, L.rgsw32 + q_off * kRgswStride, planes,
+                            (int)span, parts, st));
+        launches += span > 0;
     };
     const int planes_part = sc.matvec_tc ? kPrepPlanes : 0;
+    const size_t tp_pass = span > count ? span : (size_t)sc.tp_pass;
     prep(kPrepKeys | (prep_rgsw ? kPrepRgsw : 0) | (lwe_ready ? 0 : planes_part));
     if (ev) IPB_CK(cudaEventRecord(ev[1], st));
     // Beside: the tensor pass (keys only) on sc.tp_sms SMs from the lane's
     // Horner stream while the mat-vec (DB only) starts on the other SMs; both
     // are persistent with one CTA per SM, so the mat-vec's remaining CTAs start
     // as the tensor pass's end.
-    const bool beside = sc.matvec_tc && sc.tp_sms > 0 && sc.tp_sms < S.num_sms;
+    const bool beside = sc.matvec_tc && sc.tp_sms > 0 && sc.tp_sms < S.num_sms && span > 0;
     auto tensor_pass = [&](cudaStream_t ts, int sms) {
-        for (size_t c0 = 0; c0 < count; c0 += (size_t)sc.tp_pass) {
-            const int n = (int)std::min<size_t>((size_t)sc.tp_pass, count - c0);
+        for (size_t c0 = 0; c0 < span; c0 += tp_pass) {
+            const int n = (int)std::min(tp_pass, span - c0);
             IPB_CK(launch_tensor_pass(P.pre_dt, 0, tp_tiles(G), kplanes + c0 * kTpPlaneBytes, n, nullptr,
                                       tp_out + c0 * S.pb_qstride, S.pb_qstride, L.d_err, L.tiles + 2, sms, ts));
             ++launches;
@@ -795,13 +798,13 @@ int run_pipeline(const Server& S, Lane& L, const Sched& sc, size_t count, cudaSt
     if (phases != kPhaseAll || 6 * ns > n_ev) ev = nullptr;
     int launches = 0;
     // Slices run one after the other, each its own pipeline on its lane
-    // slots: the DB and the tensors are read once per slice either way (one
-    // mat-vec pass serves at most 32 queries), and a slice's Horner chains fit
-    // the SMs in one wave.
+    // slots: one mat-vec pass serves at most 32 queries, and a slice's Horner
+    // chains fit the SMs in one wave.  The tensor pass takes two slices at once.
     if (phases & kPhaseDb)
         for (size_t k = 0; k < ns; ++k) {
             const size_t q0 = k * slice;
-            launches += run_db_phase(S, L, sc, q0, std::min(slice, count - q0), st, ev ? ev + 6 * k : nullptr);
+            launches += run_db_phase(S, L, sc, q0, std::min(slice, count - q0), tp_span(count, sc, k), st,
+                                     ev ? ev + 6 * k : nullptr);
             if ((phases & kPhaseHorner) && ns > 1)
                 launches += run_horner_phase(S, L, sc, q0, std::min(slice, count - q0), st, ev ? ev + 6 * k : nullptr);
         }
@@ -859,7 +862,7 @@ static void run_split(Server* S, const Sched& sc, size_t count, cudaEvent_t lwe_
     const size_t ns = slices_of(count, sc), slice = sc.slice > 0 ? (size_t)sc.slice : count;
     for (size_t k = 0; k < ns; ++k) {
         const size_t q0 = k * slice, n = std::min(slice, count - q0);
-        S->launches += (unsigned long long)run_db_phase(*S, L, sc, q0, n, S->stream, nullptr,
+        S->launches += (unsigned long long)run_db_phase(*S, L, sc, q0, n, tp_span(count, sc, k), S->stream, nullptr,
                                                         k == 0 ? lwe_ready : nullptr, false);
         if (k == 0) IPB_CK(cudaStreamWaitEvent(S->stream, L.rgsw_ready, 0));
         S->launches += (unsigned long long)run_horner_phase(*S, L, sc, q0, n, S->stream, nullptr);

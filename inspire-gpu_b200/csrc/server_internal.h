@@ -9,6 +9,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -100,7 +101,8 @@ struct Precomp {
 // Kernel choices for one batch size.
 struct Sched {
     int matvec_tc = 1;       // 1: tcgen05 int8 mat-vec, 0: CUDA-core mat-vec
-    int tp_pass = 32;        // queries per tensor-pass GEMM (<= the lane's gt_pass)
+    int tp_pass = 32;        // queries per tensor-pass GEMM (<= the lane's gt_pass); whole 32-query slices
+                             // go two to a GEMM
     int horner_cluster = 1;  // 1: 4-CTA cluster per chain, 2: 8-CTA cluster, 0: one CTA per chain
     int tp_sms = 0;          // > 0: tensor pass on this many SMs beside the tcgen05 mat-vec, which starts
                              // on the others and takes these over as they come free; 0: one after the other
@@ -119,6 +121,15 @@ constexpr int kMaxHChunks = 16;
 constexpr size_t kSliceQueries = 32;
 inline size_t slices_of(size_t c, const Sched& sc) {
     return sc.slice > 0 ? (c + (size_t)sc.slice - 1) / (size_t)sc.slice : 1;
+}
+
+// Queries, from slice k of a batch of c on, that slice k's DB phase prepares
+// and runs the tensor pass for: two whole slices at a time read the tensors
+// once, the second one's phase then has none.
+inline size_t tp_span(size_t c, const Sched& sc, size_t k) {
+    const size_t slice = sc.slice > 0 ? (size_t)sc.slice : c, rest = c - k * slice;
+    if (slice != kSliceQueries || (size_t)sc.tp_pass < slice) return std::min(slice, rest);
+    return k % 2 ? 0 : std::min(2 * slice, rest);
 }
 
 // Per-batch device scratch for up to `cap` queries.
@@ -224,8 +235,10 @@ size_t auto_scan_segments(float ms);
 // The DB-bound phase (query prep, mat-vec, tensor pass, finalize) of lane
 // slots [q_off, q_off + count) on st: packed ciphertext b parts into
 // L.packed_b.  lwe_ready: an event the mat-vec waits for (the key side runs
-// first); prep_rgsw: the RGSW parts are prepared here as well.  Returns launches.
-int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t count, cudaStream_t st,
+// first); prep_rgsw: the RGSW parts are prepared here as well.  span: queries
+// from q_off on that are prepared and go through the tensor pass (tp_span).
+// Returns launches.
+int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t count, size_t span, cudaStream_t st,
                  cudaEvent_t* ev, cudaEvent_t lwe_ready = nullptr, bool prep_rgsw = true);
 // H2D of parts [p0, p0 + np) (0, 1: LWE limbs, 2: KSK5, 3: KSK-1, 4: RGSW) of
 // each query into the handle's lane, one copy per contiguous host run.

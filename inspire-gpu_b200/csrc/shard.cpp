@@ -134,7 +134,7 @@ int ipir_b200_shard_pack(ipir_shard* sh, const ipir_query_view* queries, size_t 
         for (size_t k = 0; k < ns; ++k) {
             const size_t q0 = k * slice;
             S->launches += (unsigned long long)ipb::run_db_phase(*S, L, sc, q0, std::min(slice, count - q0),
-                                                                 S->stream, nullptr, k == 0 ? lwe_ready : nullptr,
+                                                                 ipb::tp_span(count, sc, k), S->stream, nullptr, k == 0 ? lwe_ready : nullptr,
                                                                  false);
         }
         ipb::check_device_error(L, S->stream);  // nothing is written if a kernel stopped early

@@ -461,7 +461,7 @@ cudaError_t launch_tensor_pass(const uint8_t* Dt, int tile0, int n_tiles, const 
                                const uint8_t* qmap, uint32_t* tp_out, size_t out_qstride, int* err, unsigned* tiles,
                                int num_sms, cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
-    if (nq > 32 || !tiles || tile0 < 0 || n_tiles <= 0) return cudaErrorInvalidValue;
+    if (nq > kTpMaxPass || (qmap && nq > 32) || !tiles || tile0 < 0 || n_tiles <= 0) return cudaErrorInvalidValue;
     TpParams P{};
     P.dt = Dt;
     P.out = tp_out;
@@ -477,10 +477,13 @@ cudaError_t launch_tensor_pass(const uint8_t* Dt, int tile0, int n_tiles, const 
     // leaves an item per SM.  G = 1 (128 tiles), 32 queries: 20 us with one tile,
     // 25 with two; G = 128, 32 queries: 1255 and 1227 us (four tiles, whose
     // accumulators cannot be double-buffered: 1300); between, within 3 %.
-    const int mti = n_tiles % 2 == 0 && tile0 % 2 == 0 && n_tiles >= 2 * sms ? 2 : 1;
+    // More than 32 queries: one tile, so that its 256 columns stay
+    // double-buffered (G = 128, 64 queries: 1648 us, two tiles 1683, two passes
+    // of 32 queries 2450).
+    const int mti = nq <= 32 && n_tiles % 2 == 0 && tile0 % 2 == 0 && n_tiles >= 2 * sms ? 2 : 1;
     const auto kernel = mti == 2 ? tp_tc_kernel<2> : tp_tc_kernel<1>;
     P.n_items = n_tiles / mti;
-    P.acc_stages = 2;  // at most 2 x 2 x 128 columns
+    P.acc_stages = 2;  // at most 2 x 2 x 128 or 2 x 256 columns
     uint32_t need = (uint32_t)(P.acc_stages * mti * P.nb), tc = 32;
     while (tc < need) tc <<= 1;
     P.tmem_cols = tc;
@@ -504,7 +507,11 @@ cudaError_t launch_tensor_pass(const uint8_t* Dt, int tile0, int n_tiles, const 
     CUtensorMap mb;
     if (!make_map_b(&mb, kplanes, nq)) return cudaErrorInvalidValue;
     const size_t smem = 1024 + (size_t)P.stages * stage_bytes + (2 * P.stages + 4) * 8 + 16;
-    return launch_overlapped(kernel, std::min(P.n_items, sms), kTpThreads, smem, s, mb, P);
+    // The items take `waves` rounds; the SMs that would have none in the last
+    // round are left to the mat-vec (1 group, 128 items, beside on 98 SMs: 64 CTAs
+    // end as soon, 42 -> 38 us for the answer's kernels).
+    const int waves = (P.n_items + sms - 1) / sms;
+    return launch_overlapped(kernel, (P.n_items + waves - 1) / waves, kTpThreads, smem, s, mb, P);
 }
 
 }  // namespace ipb
