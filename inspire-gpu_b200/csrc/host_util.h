@@ -2,6 +2,7 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 
 #include <cuda_runtime.h>
 
@@ -54,8 +55,8 @@ inline cudaError_t allow_max_smem(K* kernel, size_t* max_dynamic = nullptr) {
 // ipb_common.cuh).  Back-to-back kernels of one answer: 2-4 us less each on the
 // small databases, where launch gaps and prologues are most of the time.
 template <class... P, class... A>
-inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                     A&&... args) {
+inline cudaError_t launch_overlapped_if(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                        cudaStream_t s, A&&... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -65,8 +66,13 @@ inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                     A&&... args) {
+    return launch_overlapped_if(true, kernel, grid, block, smem, s, std::forward<A>(args)...);
 }
 
 }  // namespace ipb

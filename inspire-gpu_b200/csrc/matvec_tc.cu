@@ -381,7 +381,8 @@ cudaError_t launch_matvec_tc_range(const uint16_t* db, size_t rows, size_t ld, s
 cudaError_t launch_matvec_tc_ranges(const uint16_t* db, size_t rows, size_t ld, size_t c0, size_t cols_per_range,
                                     int n_ranges, size_t range_stride, const uint8_t* planes, int nq,
                                     const DevTables* T, uint32_t* part, size_t part_qstride, const uint8_t* qmap,
-                                    int* err, unsigned* tiles, int num_sms, int kchunk_rows, cudaStream_t s) {
+                                    int* err, unsigned* tiles, int num_sms, int kchunk_rows, cudaStream_t s,
+                                    bool overlap) {
     if (nq <= 0) return cudaSuccess;
     if (n_ranges < 1 || cols_per_range == 0 || cols_per_range % 128 || c0 % 128 ||
         (n_ranges > 1 && (range_stride < cols_per_range || range_stride % 128)))
@@ -458,7 +459,7 @@ cudaError_t launch_matvec_tc_ranges(const uint16_t* db, size_t rows, size_t ld, 
     if (e) return e;
     const int items = P.n_mtiles * P.n_kchunks;
     const int grid = std::min(items, std::max(1, num_sms));
-    return launch_overlapped(mv_tc_kernel, grid, kMvThreads, smem, s, ma, mb, P);
+    return launch_overlapped_if(overlap, mv_tc_kernel, grid, kMvThreads, smem, s, ma, mb, P);
 }
 
 }  // namespace ipb

@@ -263,6 +263,7 @@ void alloc_lane(const Server& S, Lane& L, size_t cap, int gt_pass) {
     L.wire_in = A.alloc<uint8_t>(cap * S.wire_q);
     L.wire_out = A.alloc<uint8_t>(cap * std::max(S.wire_r, S.wire_c));
     L.codec_tmp = A.alloc<uint32_t>(cap * S.pp.num_cts * 4 * kN);
+    IPB_CK(cudaHostAlloc(reinterpret_cast<void**>(&L.bounce), Lane::kBounceBytes + sizeof(int), cudaHostAllocDefault));
     IPB_CK(cudaStreamCreateWithFlags(&L.aux, cudaStreamNonBlocking));
     IPB_CK(cudaEventCreateWithFlags(&L.fork, cudaEventDisableTiming));
     IPB_CK(cudaEventCreateWithFlags(&L.join, cudaEventDisableTiming));
@@ -412,9 +413,11 @@ static bool chunked_ok(const Server& S, const Sched& sc, size_t count);
 //     5.1 us).
 //   Horner chain trailing the DB pass in chunks where a chunk's mat-vec lasts
 //     longer than its chain steps (32768 rows: 19 us a group against 4-11) and
-//     the chain is worth the extra launches: 128 groups, 16 GB: 1 query 3.68
-//     against 3.92 ms, 8: 3.99 / 4.08, 16: 4.19 / 4.39, 32: 5.42 / 5.40; 32
-//     groups, 4 GB: 1.14 / 1.10; 128 groups on 2048 rows: 1.84 / 1.75.
+//     the chain is worth the extra launches: 128 groups, 16 GB: 1 query 3.69
+//     against 4.07 ms, 8: 4.05 / 4.25, 16: 4.47 / 4.56, 32: 5.42 / 5.40; 32
+//     groups, 4 GB: 1.14 / 1.10; 128 groups on 2048 rows: 1.84 / 1.75.  At most
+//     8 chunks up to 2 queries (2: 3.82, 4 chunks 3.90), 4 beyond (8: 4.05 /
+//     4.30 with 8: the chains of a chunk hold their SMs longer).
 //   Tensor pass beside the mat-vec, on two SMs of three, where the two streams
 //     are short enough for launch ramps and tails to count (up to 8 GB
 //     together): 1 GB 293 -> 281 us at 1 query, 410 -> 390 at 32; 4 GB (6.4 GB
@@ -439,7 +442,7 @@ std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
         if (chain >= 64 && S.pp.db_rows >= 16384 && c <= std::min<size_t>(16, chain / 8)) {
             Sched chunked = sc;
             chunked.horner_cluster = 1;
-            chunked.hchunks = 8;
+            chunked.hchunks = c <= 2 ? 8 : 4;
             if (chunked_ok(S, chunked, c)) sc = chunked;
         }
         if (h) sc.horner_cluster = std::strcmp(h, "cta") == 0 ? 0 : (std::strcmp(h, "cl8") == 0 ? 2 : 1);
@@ -692,9 +695,12 @@ static int run_chunked(const Server& S, Lane& L, const Sched& sc, size_t count, 
     size_t hi = d_act;
     for (size_t c = 0; c < sizes.size(); hi -= sizes[c], ++c) {
         const size_t lo = hi - sizes[c];
+        // Only the first mat-vec starts early: a later one would take every SM
+        // before the Horner clusters of the chunk before it (16 GB, 1 query 3.96
+        // against 3.81 ms).
         IPB_CK(launch_matvec_tc_ranges(P.db, R, C, lo * kN, (hi - lo) * kN, (int)nct, d_act * kN, L.planes, nq,
                                        P.tables, L.mvpart, S.mv_qstride, nullptr, L.d_err, L.tiles, S.num_sms,
-                                       S.tc_kchunk_rows, st));
+                                       S.tc_kchunk_rows, st, c == 0));
         for (size_t t = 0; t < nct; ++t) {
             IPB_CK(launch_finalize_range(L.mvpart, S.mv_qstride, S.tc_kchunks, C, L.tp_out, P.pre_df, L.keys,
                                          kKeyStride, P.tables, L.packed_b, S.pb_qstride, G, t * d_act + lo, hi - lo,
@@ -898,24 +904,41 @@ static void stage_and_run(Server* S, const ipir_query_view* qs, size_t count) {
 
 // A kernel whose pipeline wait ran out of iterations leaves a code in the
 // device error word; report it (the responses are then not valid).
+static void raise_device_error(Lane& L, cudaStream_t st, int e) {
+    if (!e) return;
+    IPB_CK(cudaMemsetAsync(L.d_err, 0, sizeof(int), st));  // ordered before the next batch's kernels
+    IPB_CK(cudaStreamSynchronize(st));
+    throw std::runtime_error("device pipeline wait timed out (code " + std::to_string(e) + ")");
+}
 void check_device_error(Lane& L, cudaStream_t st) {
     int e = 0;
     IPB_CK(cudaMemcpyAsync(&e, L.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     IPB_CK(cudaStreamSynchronize(st));
-    if (e) {
-        IPB_CK(cudaMemsetAsync(L.d_err, 0, sizeof(int), st));  // ordered before the next batch's kernels
-        IPB_CK(cudaStreamSynchronize(st));
-        throw std::runtime_error("device pipeline wait timed out (code " + std::to_string(e) + ")");
-    }
+    raise_device_error(L, st, e);
 }
 
-// The error word is read first, once the batch has run: a batch whose
-// kernels stopped early writes nothing into the caller's buffer.
+// Waits for the batch on st and copies its responses from `src` to the
+// caller's buffer.  A batch whose kernels stopped early writes nothing there:
+// small responses come with the error word through the lane's pinned buffer
+// (one wait; 10 us of a one-query answer), large ones after it has been read.
+static void deliver(Lane& L, cudaStream_t st, const void* src, size_t bytes, void* out) {
+    if (bytes > Lane::kBounceBytes) {
+        check_device_error(L, st);
+        IPB_CK(cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, st));
+        IPB_CK(cudaStreamSynchronize(st));
+        return;
+    }
+    int* const e = reinterpret_cast<int*>(L.bounce + Lane::kBounceBytes);
+    IPB_CK(cudaMemcpyAsync(e, L.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    IPB_CK(cudaMemcpyAsync(L.bounce, src, bytes, cudaMemcpyDeviceToHost, st));
+    IPB_CK(cudaStreamSynchronize(st));
+    raise_device_error(L, st, *e);
+    std::memcpy(out, L.bounce, bytes);
+}
+
 static void fetch(Server* S, size_t count, uint64_t* out) {
     IPB_CK(cudaSetDevice(S->device));
-    check_device_error(S->lane, S->stream);
-    IPB_CK(cudaMemcpyAsync(out, S->lane.resp, count * S->resp_qstride * 8, cudaMemcpyDeviceToHost, S->stream));
-    IPB_CK(cudaStreamSynchronize(S->stream));
+    deliver(S->lane, S->stream, S->lane.resp, count * S->resp_qstride * 8, out);
     if (S->timing && S->timed_slices)  // stage times summed over the batch's slices
         for (int i = 0; i < 5; ++i) {
             S->stage_ms[i] = 0.f;
@@ -1111,9 +1134,7 @@ static void answer_wire(Server* S, const uint8_t* packed, size_t count, int fmt,
         src = L.wire_out;
         bytes = count * S->wire_c;
     }
-    check_device_error(L, st);  // nothing is written if a kernel stopped early
-    IPB_CK(cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, st));
-    IPB_CK(cudaStreamSynchronize(st));
+    deliver(L, st, src, bytes, out);
 }
 
 static int validate_batch(const Server* S, const ipir_query_view* qs, size_t count, const void* out) {

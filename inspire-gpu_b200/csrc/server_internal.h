@@ -151,6 +151,8 @@ struct Lane {
     uint8_t* wire_in = nullptr;  // packed queries
     uint8_t* wire_out = nullptr; // packed or compressed responses
     uint32_t* codec_tmp = nullptr;  // coefficient-form responses for compression
+    static constexpr size_t kBounceBytes = (size_t)256 << 10;
+    uint8_t* bounce = nullptr;      // pinned: a small batch's responses, then the error word
     cudaStream_t aux = nullptr;     // the blocking path's copies
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaEvent_t rgsw_ready = nullptr;  // RGSW parts staged and prepared on aux
@@ -168,6 +170,7 @@ struct Lane {
         if (join) cudaEventDestroy(join);
         if (fork) cudaEventDestroy(fork);
         if (aux) cudaStreamDestroy(aux);
+        if (bounce) cudaFreeHost(bounce);
         arena.free_all();
     }
 };
