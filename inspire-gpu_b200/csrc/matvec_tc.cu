@@ -72,7 +72,7 @@ struct TcParams {
     const DevTables* T;
     int has_qmap;          // output row of pass query q: qmap[q] (else q)
     uint8_t qmap[32];
-    int abort_after;       // > 0: the MMA issuer stops after this many items and reports code 99 (a test of
+    int abort_after;       // > 0: the MMA issuer stops after this many m' tiles and reports code 99 (a test of
                            // the abort path, IPB_TEST_ABORT_AFTER_ITEMS); 0: off
 };
 
@@ -86,14 +86,23 @@ __device__ __forceinline__ int mtile_m0(const TcParams& P, int mt) {
 constexpr int kMvThreads = 384;
 constexpr int kEpiThreads = 256;
 
+// MT: m' tiles per work item, 1 or 2 (two adjacent ones, 512 bytes of a row,
+// that share a stage's query planes; mv_tiles has the rule).
+// Bound by HBM up to about 8 queries and by power beyond: the same launch takes
+// 3.05 ms alone and 3.9 ms back to back at 32 queries over 16 GB.  Two tiles
+// halve the planes' way from L2 through shared memory: back to back over 16 GB
+// 2.78 -> 2.59 ms at 8 queries, 3.17 -> 2.93 at 16; over 4 GB, where fewer,
+// longer items also leave less of a tail, 0.69 -> 0.64 at 1 and 0.79 -> 0.75 at
+// 16.
+template <int MT>
 __global__ void __launch_bounds__(kMvThreads, 1) mv_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                                        const __grid_constant__ CUtensorMap map_b, TcParams P) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int S = P.stages;
-    const uint32_t a_bytes = kKT * 128;              // one 128-byte m' box x kKT rows
+    constexpr uint32_t a_bytes = kKT * 128;          // one 128-byte m' box x kKT rows
     const uint32_t b_bytes = (uint32_t)P.npad * kKT;
-    const uint32_t stage_bytes = 2 * a_bytes + b_bytes;
+    const uint32_t stage_bytes = 2 * MT * a_bytes + b_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)S * stage_bytes);
     uint64_t* full = bars;
     uint64_t* empty = bars + S;
@@ -125,7 +134,7 @@ __global__ void __launch_bounds__(kMvThreads, 1) mv_tc_kernel(const __grid_const
     tc_fence_after();
     after_previous();
     const uint32_t tmem_base = *tmem_slot;
-    const int n_items = P.n_mtiles * P.n_kchunks;
+    const int n_mitems = P.n_mtiles / MT, n_items = n_mitems * P.n_kchunks;
     const int ktiles = P.kchunk_rows / kKT;
 
     if (warp == 0) {
@@ -146,16 +155,17 @@ __global__ void __launch_bounds__(kMvThreads, 1) mv_tc_kernel(const __grid_const
                 item_ring[r] = item;
                 mbar_arrive(&ifull[r]);
                 if (item < 0) break;
-                const int mt = item % P.n_mtiles, kc = item / P.n_mtiles;
+                const int mt = item % n_mitems * MT, kc = item / n_mitems;
                 const int m0 = mtile_m0(P, mt);
                 for (int kt = 0; kt < ktiles; ++kt) {
                     if (!mbar_wait_ab(&empty[s], ph ^ 1, P.err, 1, &abort_flag)) { abort_flag = 1; break; }
                     uint8_t* st = smem + (size_t)s * stage_bytes;
                     mbar_expect_tx(&full[s], stage_bytes);
                     const int k0 = kc * P.kchunk_rows + kt * kKT;
-                    tma_load_2d(st, &map_a, &full[s], m0, k0);
-                    tma_load_2d(st + a_bytes, &map_a, &full[s], m0 + 128, k0);
-                    tma_load_2d(st + 2 * a_bytes, &map_b, &full[s], k0, 0);
+#pragma unroll
+                    for (int h = 0; h < 2 * MT; ++h)
+                        tma_load_2d(st + h * a_bytes, &map_a, &full[s], m0 + 128 * h, k0);
+                    tma_load_2d(st + 2 * MT * a_bytes, &map_b, &full[s], k0, 0);
                     ++issued;
                     if (++s == S) { s = 0; ph ^= 1; }
                 }
@@ -172,7 +182,7 @@ __global__ void __launch_bounds__(kMvThreads, 1) mv_tc_kernel(const __grid_const
     } else if (warp == 1) {
         // ---------------- MMA issuer
         if (lane == 0) {
-            const uint32_t idesc = idesc_i8(P.npad);
+            const uint32_t idesc = idesc_i8(P.npad), desc0 = smem_desc_lo(smem, 0);
             int s = 0, as = 0;
             uint32_t ph = 0, aph = 0;
             bool it_mma = false;  // any MMA issued
@@ -185,29 +195,45 @@ __global__ void __launch_bounds__(kMvThreads, 1) mv_tc_kernel(const __grid_const
                 const int item = item_ring[r];
                 mbar_arrive(&iempty[r]);
                 if (item < 0 || abort_flag) break;
-                if (P.abort_after > 0 && it >= P.abort_after) {  // test hook: the designed early stop
+                if (P.abort_after > 0 && it * MT >= P.abort_after) {  // test hook: the designed early stop
                     atomicCAS(P.err, 0, 99);
                     abort_flag = 1;
                     break;
                 }
                 if (!mbar_wait_ab(&tempty[as], aph ^ 1, P.err, 3, &abort_flag)) { abort_flag = 1; break; }
                 tc_fence_after();
-                const uint32_t d0 = tmem_base + (uint32_t)(as * 2 * P.npad);
+                const uint32_t d0 = tmem_base + (uint32_t)(as * 2 * MT * P.npad);
                 for (int kt = 0; kt < ktiles; ++kt) {
                     if (!mbar_wait_ab(&full[s], ph, P.err, 4, &abort_flag)) { abort_flag = 1; break; }
                     tc_fence_after();
-                    const uint8_t* st = smem + (size_t)s * stage_bytes;
+                    // A: MN-major, rows of 128 bytes, 8-row swizzle atoms (SBO 1024 B);
+                    // K advances 32 rows = 4096 bytes per MMA.
+                    // B: K-major, 64-byte rows (SWIZZLE_64B), 8-row groups 512 B apart; K advances 32 bytes.
+                    if (MT == 1) {
+                        // Whole descriptors, which takes the thread longer: at 32 queries
+                        // and a burst of launches 1.55 ms over 8 GB against 1.55-1.89 with
+                        // the MMAs issued at once.
+                        const uint8_t* st = smem + (size_t)s * stage_bytes;
 #pragma unroll
-                    for (int kk = 0; kk < kKT / 32; ++kk) {
-                        // A: MN-major, rows of 128 bytes, 8-row swizzle atoms (SBO 1024 B);
-                        // K advances 32 rows = 4096 bytes per MMA.
-                        const uint64_t a0 = smem_desc(st + kk * 4096, 0, 1024);
-                        const uint64_t a1 = smem_desc(st + a_bytes + kk * 4096, 0, 1024);
-                        // B: K-major, 64-byte rows (SWIZZLE_64B), 8-row groups 512 B apart; K advances 32 bytes.
-                        const uint64_t b = smem_desc_sw64(st + 2 * a_bytes + kk * 32, 512);
-                        const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
-                        mma_i8(d0, a0, b, idesc, acc);
-                        mma_i8(d0 + (uint32_t)P.npad, a1, b, idesc, acc);
+                        for (int kk = 0; kk < kKT / 32; ++kk) {
+                            const uint64_t a0 = smem_desc(st + kk * 4096, 0, 1024);
+                            const uint64_t a1 = smem_desc(st + a_bytes + kk * 4096, 0, 1024);
+                            const uint64_t b = smem_desc_sw64(st + 2 * a_bytes + kk * 32, 512);
+                            const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
+                            mma_i8(d0, a0, b, idesc, acc);
+                            mma_i8(d0 + (uint32_t)P.npad, a1, b, idesc, acc);
+                        }
+                    } else {
+                        // A descriptor is one 32-bit add (the address field of its low word).
+                        const uint32_t ad = desc0 + (uint32_t)s * (stage_bytes >> 4);
+                        const uint32_t bd = ad + (2 * MT * a_bytes >> 4) + (1u << 16);
+#pragma unroll
+                        for (int kk = 0; kk < kKT / 32; ++kk)
+#pragma unroll
+                            for (int h = 0; h < 2 * MT; ++h)
+                                mma_i8_lo(d0 + (uint32_t)(h * P.npad), ad + h * (a_bytes >> 4) + kk * 256, bd + kk * 2,
+                                          smem_desc_hi_sw128(1024), smem_desc_hi_sw64(512), idesc,
+                                          (kt > 0 || kk > 0) ? 1u : 0u);
                     }
                     it_mma = true;
                     mma_commit(&empty[s]);
@@ -225,10 +251,10 @@ __global__ void __launch_bounds__(kMvThreads, 1) mv_tc_kernel(const __grid_const
         }
     } else if (warp >= 4) {
         // ---------------- epilogue: TMEM -> u64 dot products -> mod q
-        // An accumulator set of more than 256 columns (more than 18 queries)
-        // is not double-buffered: the MMAs wait while it is drained, so the
+        // An accumulator set of more than 256 columns (more than 18 queries, or
+        // 9 with two tiles) is not double-buffered: the MMAs wait while it is drained, so the
         // epilogue's length counts.  Two warps per TMEM lane quarter, one half
-        // of the m' tile each; the weights of the lane's byte row (lo bytes in
+        // of each m' tile each; the weights of the lane's byte row (lo bytes in
         // even lanes, hi in odd) are in registers, and the pair of lanes of a
         // column meets once per query in 64 bits: the even lane reduces and
         // writes limb 0, the odd one limb 1.
@@ -252,44 +278,47 @@ __global__ void __launch_bounds__(kMvThreads, 1) mv_tc_kernel(const __grid_const
             if (item < 0) break;
             if (!mbar_wait_ab(&tfull[as], aph, P.err, 5, &abort_flag)) { abort_flag = 1; break; }
             tc_fence_after();
-            const int mt = item % P.n_mtiles, kc = item / P.n_mtiles;
+            const int mt = item % n_mitems * MT, kc = item / n_mitems;
             const int m0 = mtile_m0(P, mt);
-            const size_t col = ((size_t)m0 + mb * 128 + wq * 32 + lane) >> 1;
-            uint32_t* const out = P.part + ((size_t)kc * 2 + hi) * P.ld + col;
-            const uint32_t acc = tmem_base + lane_base + (uint32_t)(as * 2 * P.npad + mb * P.npad);
-            for (int q0 = 0; q0 < P.nq; q0 += 8) {
-                // queries q0..q0+7: columns 7 q0 .. 7 q0 + 55, seven 8-column
-                // loads (those at or past N are not loaded: they hold no query)
-                uint32_t t[kPlanes][8];
 #pragma unroll
-                for (int c = 0; c < kPlanes; ++c) {
-                    const int n = kPlanes * q0 + 8 * c;
-                    if (n < P.npad) {
-                        tmem_ld8_issue(acc + (uint32_t)n, t[c]);
-                    } else {
+            for (int hb = mb; hb < 2 * MT; hb += 2) {  // 128-row halves of the item
+                const size_t col = ((size_t)m0 + hb * 128 + wq * 32 + lane) >> 1;
+                uint32_t* const out = P.part + ((size_t)kc * 2 + hi) * P.ld + col;
+                const uint32_t acc = tmem_base + lane_base + (uint32_t)(as * 2 * MT * P.npad + hb * P.npad);
+                for (int q0 = 0; q0 < P.nq; q0 += 8) {
+                    // queries q0..q0+7: columns 7 q0 .. 7 q0 + 55, seven 8-column
+                    // loads (those at or past N are not loaded: they hold no query)
+                    uint32_t t[kPlanes][8];
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) t[c][e] = 0;
+                    for (int c = 0; c < kPlanes; ++c) {
+                        const int n = kPlanes * q0 + 8 * c;
+                        if (n < P.npad) {
+                            tmem_ld8_issue(acc + (uint32_t)n, t[c]);
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) t[c][e] = 0;
+                        }
                     }
-                }
-                uint32_t v[kPlanes * 8];
+                    uint32_t v[kPlanes * 8];
 #pragma unroll
-                for (int c = 0; c < kPlanes; ++c) {
-                    tmem_wait8(t[c]);  // one wait for all seven loads; the others are no-ops
+                    for (int c = 0; c < kPlanes; ++c) {
+                        tmem_wait8(t[c]);  // one wait for all seven loads; the others are no-ops
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[8 * c + e] = t[c][e];
-                }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    if (q0 + e >= P.nq) break;
-                    uint64_t a0 = 0, a1 = 0;
-#pragma unroll
-                    for (int k = 0; k < kPlanes; ++k) {
-                        a0 += (uint64_t)w0[k] * v[kPlanes * e + k];
-                        a1 += (uint64_t)w1[k] * v[kPlanes * e + k];
+                        for (int e = 0; e < 8; ++e) v[8 * c + e] = t[c][e];
                     }
-                    const uint64_t sum = (hi ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hi ? a0 : a1, 1);
-                    const int qo = P.has_qmap ? P.qmap[q0 + e] : q0 + e;
-                    out[(size_t)qo * P.part_qstride] = mod_u64(sum, cr, ql);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        if (q0 + e >= P.nq) break;
+                        uint64_t a0 = 0, a1 = 0;
+#pragma unroll
+                        for (int k = 0; k < kPlanes; ++k) {
+                            a0 += (uint64_t)w0[k] * v[kPlanes * e + k];
+                            a1 += (uint64_t)w1[k] * v[kPlanes * e + k];
+                        }
+                        const uint64_t sum = (hi ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hi ? a0 : a1, 1);
+                        const int qo = P.has_qmap ? P.qmap[q0 + e] : q0 + e;
+                        out[(size_t)qo * P.part_qstride] = mod_u64(sum, cr, ql);
+                    }
                 }
             }
             tc_fence_before();
@@ -350,16 +379,37 @@ cudaError_t launch_mv_chunk_reduce(const uint32_t* part, size_t part_qstride, in
     return cudaGetLastError();
 }
 
-// nq <= 32 queries whose planes start at `planes` (rows bytes per plane row).
-int matvec_tc_item_cols() { return kMT / 2; }
-
-int matvec_tc_kchunk_rows(size_t rows, size_t cols, int num_sms) {
-    // Rows per exact s32 accumulation: at most 32768, halved while the
-    // (m'-tile, chunk) work items would leave SMs idle.
-    size_t kc = rows < (size_t)kKChunk ? rows : (size_t)kKChunk;
-    const size_t mtiles = (2 * cols) / kMT;
-    while (mtiles * (rows / kc) < (size_t)(2 * num_sms) && kc > 1024 && kc % 2 == 0) kc /= 2;
-    return (int)kc;
+// Tiles per work item for a pass of nq queries over a DB of ld columns per
+// row.  Two while their accumulators fit TMEM (18 queries), if the DB is small
+// enough for the tail of its few items to count or the batch large enough for
+// the planes to (up to 6 GB, or from 6 queries: over 16 GB 1 query takes 2.41 ms
+// with one tile and 2.48 with two, 4: 2.50 / 2.57, 8: 2.78 / 2.59), and if the
+// accumulators are double-buffered or an item long enough for that not to
+// matter (16 queries, 640 rows an item: 31 us with one tile, 36 with two; 2048
+// rows 214 / 217; 8192 rows 214 / 196).
+static int mv_tiles(int nq, size_t rows, size_t ld, int kchunk_rows) {
+    const int npad = (kPlanes * nq + 15) / 16 * 16;
+    if (4 * npad > 512 || (8 * npad > 512 && kchunk_rows < 4096)) return 1;
+    return 2.0 * (double)rows * (double)ld <= 6e9 || nq >= 6 ? 2 : 1;
+}
+// Rows per exact s32 accumulation: at most 32768, halved while there are
+// fewer than two work items per SM.
+int matvec_tc_kchunk_rows(size_t rows, size_t cols, int num_sms, int nq) {
+    auto chunk = [&](size_t tiles_per_item) {
+        size_t kc = rows < (size_t)kKChunk ? rows : (size_t)kKChunk;
+        const size_t mtiles = (2 * cols) / kMT;
+        while (mtiles * (rows / kc) < tiles_per_item * (size_t)(2 * num_sms) && kc > 1024 && kc % 2 == 0) kc /= 2;
+        return (int)kc;
+    };
+    // With two tiles per item the chunks are halved once more where that leaves
+    // the pass on two tiles (21 groups, 8 queries: 768 -> 708 us, one tile 730).
+    const int one = chunk(1);
+    if (mv_tiles(nq, rows, cols, one) == 1) return one;
+    const int two = chunk(2);
+    return mv_tiles(nq, rows, cols, two) == 2 ? two : one;
+}
+int matvec_tc_item_cols(int nq, size_t rows, size_t ld, int kchunk_rows) {
+    return kMT / 2 * mv_tiles(nq, rows, ld, kchunk_rows);
 }
 
 cudaError_t launch_matvec_tc(const uint16_t* db, size_t rows, size_t cols, const uint8_t* planes, int nq,
@@ -442,24 +492,26 @@ cudaError_t launch_matvec_tc_ranges(const uint16_t* db, size_t rows, size_t ld, 
     P.n_mtiles = n_ranges > 1 ? n_ranges * P.mt_per_range : (int)((2 * cols) / kMT);
     P.kchunk_rows = kchunk;
     P.n_kchunks = (int)(rows / kchunk);
-    P.acc_stages = (4 * npad <= 512) ? 2 : 1;
-    uint32_t need = (uint32_t)(P.acc_stages * 2 * npad);
+    const int mt = P.n_mtiles % 2 == 0 && P.mt_per_range % 2 == 0 ? mv_tiles(nq, rows, ld, kchunk) : 1;
+    P.acc_stages = (4 * mt * npad <= 512) ? 2 : 1;
+    uint32_t need = (uint32_t)(P.acc_stages * 2 * mt * npad);
     uint32_t tc = 32;
     while (tc < need) tc <<= 1;
     P.tmem_cols = tc;
     P.err = err;
     P.tiles = tiles;
     P.T = T;
-    const size_t stage_bytes = 2 * (size_t)kKT * 128 + (size_t)npad * kKT;
+    const size_t stage_bytes = 2 * mt * (size_t)kKT * 128 + (size_t)npad * kKT;
     const size_t budget = 200 * 1024;
     P.stages = (int)std::min<size_t>(8, budget / stage_bytes);
     if (P.stages < 2) return cudaErrorInvalidValue;
     const size_t smem = 1024 + (size_t)P.stages * stage_bytes + (2 * P.stages + 4) * 8 + 16;
-    cudaError_t e = allow_max_smem(mv_tc_kernel);
+    const auto kernel = mt == 2 ? mv_tc_kernel<2> : mv_tc_kernel<1>;
+    cudaError_t e = allow_max_smem(kernel);
     if (e) return e;
-    const int items = P.n_mtiles * P.n_kchunks;
+    const int items = P.n_mtiles / mt * P.n_kchunks;
     const int grid = std::min(items, std::max(1, num_sms));
-    return launch_overlapped_if(overlap, mv_tc_kernel, grid, kMvThreads, smem, s, ma, mb, P);
+    return launch_overlapped_if(overlap, kernel, grid, kMvThreads, smem, s, ma, mb, P);
 }
 
 }  // namespace ipb
@@ -470,7 +522,7 @@ cudaError_t launch_matvec_tc_ranges(const uint16_t* db, size_t rows, size_t ld, 
 extern "C" int ipir_b200_kernel_binary_version(int* out) {
     if (!out) return 1;
     cudaFuncAttributes a{};
-    cudaError_t e = cudaFuncGetAttributes(&a, ipb::mv_tc_kernel);
+    cudaError_t e = cudaFuncGetAttributes(&a, ipb::mv_tc_kernel<1>);
     if (e != cudaSuccess) {
         ipb::set_last_error(cudaGetErrorString(e));
         return 4;

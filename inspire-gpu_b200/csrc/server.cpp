@@ -230,6 +230,11 @@ Server::~Server() {
     if (own_stream) cudaStreamDestroy(own_stream);
 }
 
+// Rows per K chunk of the tensor-core mat-vec for a batch of `count` queries.
+static int kchunk_rows(const Server& S, size_t count) {
+    return matvec_tc_kchunk_rows(S.pp.db_rows, S.pp.db_cols, S.num_sms, (int)std::min(count, kSliceQueries));
+}
+
 static int pick_pow2_chunks(size_t target, size_t maxv) {
     size_t c = 1;
     while (c < target && c * 2 <= maxv) c *= 2;
@@ -300,9 +305,11 @@ Server* make_server(const Params& pp, std::shared_ptr<Precomp> pre, size_t max_b
     // limbs x rows x 4 B) within 128 KB of shared memory.
     while (R / (size_t)S->mv_chunks > 4096) S->mv_chunks *= 2;
     IPB_CK(cudaDeviceGetAttribute(&S->num_sms, cudaDevAttrMultiProcessorCount, S->device));
-    S->tc_kchunk_rows = matvec_tc_kchunk_rows(R, C, S->num_sms);
+    S->tc_kchunk_rows = matvec_tc_kchunk_rows(R, C, S->num_sms, (int)kSliceQueries);
     S->tc_kchunks = (int)(R / (size_t)S->tc_kchunk_rows);
-    S->mv_qstride = (size_t)std::max(S->mv_chunks, S->tc_kchunks) * 2 * C;
+    size_t most_chunks = (size_t)S->mv_chunks;
+    for (size_t n = 1; n <= kSliceQueries; ++n) most_chunks = std::max(most_chunks, R / (size_t)kchunk_rows(*S, n));
+    S->mv_qstride = most_chunks * 2 * C;
     S->pb_qstride = G * 2 * kN;
     S->resp_qstride = pp.num_cts * 4 * kN;
     S->wire_q = wire_query_bytes(R);
@@ -514,14 +521,15 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
     }
     int mv_parts;
     if (sc.matvec_tc) {
+        const int kchunk = kchunk_rows(S, count);
         for (size_t c0 = 0; c0 < count; c0 += 32) {
             const int n = (int)std::min<size_t>(32, count - c0);
             IPB_CK(launch_matvec_tc(P.db, R, C, planes + mv_tc_planes_offset(c0, R), n, P.tables,
                                     mvpart + c0 * S.mv_qstride, S.mv_qstride, L.d_err, L.tiles, S.num_sms,
-                                    S.tc_kchunk_rows, st));
+                                    kchunk, st));
             ++launches;
         }
-        mv_parts = S.tc_kchunks;
+        mv_parts = (int)(R / (size_t)kchunk);
     } else {
         for (size_t c0 = 0; c0 < count; c0 += 4) {
             const int n = (int)std::min<size_t>(4, count - c0);
@@ -685,7 +693,8 @@ static int run_chunked(const Server& S, Lane& L, const Sched& sc, size_t count, 
     // response ciphertext (ciphertext t's groups t * d_act + [lo, hi)): one
     // mat-vec launch covers the range in all of them.
     const size_t nct = pp.num_cts, d_act = std::min(pp.D, G);
-    const size_t ipg = (kN / (size_t)matvec_tc_item_cols()) * (size_t)S.tc_kchunks * nct;
+    const int kchunk = kchunk_rows(S, count), kchunks = (int)(R / (size_t)kchunk);
+    const size_t ipg = (kN / (size_t)matvec_tc_item_cols(nq, R, C, kchunk)) * (size_t)kchunks * nct;
     const std::vector<size_t> sizes =
         chunk_sizes(d_act, ipg, S.num_sms, std::min<size_t>((size_t)sc.hchunks, kMaxHChunks));
     IPB_CK(cudaEventRecord(L.hjoin, st));               // the Horner stream starts after this batch's prep
@@ -700,9 +709,9 @@ static int run_chunked(const Server& S, Lane& L, const Sched& sc, size_t count, 
         // against 3.81 ms).
         IPB_CK(launch_matvec_tc_ranges(P.db, R, C, lo * kN, (hi - lo) * kN, (int)nct, d_act * kN, L.planes, nq,
                                        P.tables, L.mvpart, S.mv_qstride, nullptr, L.d_err, L.tiles, S.num_sms,
-                                       S.tc_kchunk_rows, st, c == 0));
+                                       kchunk, st, c == 0));
         for (size_t t = 0; t < nct; ++t) {
-            IPB_CK(launch_finalize_range(L.mvpart, S.mv_qstride, S.tc_kchunks, C, L.tp_out, P.pre_df, L.keys,
+            IPB_CK(launch_finalize_range(L.mvpart, S.mv_qstride, kchunks, C, L.tp_out, P.pre_df, L.keys,
                                          kKeyStride, P.tables, L.packed_b, S.pb_qstride, G, t * d_act + lo, hi - lo,
                                          nq, st));
             ++launches;
@@ -1745,7 +1754,8 @@ int ipir_b200_matvec_ex(const uint16_t* db, size_t rows, size_t cols, const uint
                 kchunk = std::min<size_t>(rows, 4096);
                 while (kchunk > 1024 && (cols / 2048) * (rows / kchunk) < (size_t)(4 * sms)) kchunk /= 2;
             } else {
-                kchunk = o.kchunk_rows ? (size_t)o.kchunk_rows : (size_t)ipb::matvec_tc_kchunk_rows(rows, cols, sms);
+                kchunk = o.kchunk_rows ? (size_t)o.kchunk_rows : (size_t)ipb::matvec_tc_kchunk_rows(
+                                             rows, cols, sms, (int)std::min<size_t>(count, (size_t)qpp));
             }
             const int chunks = (int)(rows / kchunk);
             const size_t pq = (size_t)chunks * 2 * cols;  // partials of one query

@@ -188,7 +188,7 @@ struct Server {
     size_t wire_q = 0, wire_r = 0, wire_c = 0;  // bytes per query: packed query, packed / compressed response
     int mv_chunks = 1;
     int num_sms = 148;
-    int tc_kchunk_rows = 0, tc_kchunks = 1;
+    int tc_kchunk_rows = 0, tc_kchunks = 1;  // of the cyclic scan, whose passes vary in size; a batch has its own
     // sched[c] for batch size c (index 0 unused); env overrides applied at setup
     std::vector<Sched> sched;
     bool tuned = false;

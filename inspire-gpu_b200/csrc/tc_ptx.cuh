@@ -133,6 +133,9 @@ __device__ __forceinline__ uint32_t smem_desc_lo(const void* p, uint32_t lbo_byt
 __host__ __device__ constexpr uint32_t smem_desc_hi_sw128(uint32_t sbo_bytes) {
     return (sbo_bytes >> 4) | 1u << 14 | 2u << 29;
 }
+__host__ __device__ constexpr uint32_t smem_desc_hi_sw64(uint32_t sbo_bytes) {
+    return (sbo_bytes >> 4) | 1u << 14 | 4u << 29;
+}
 __device__ __forceinline__ void mma_i8_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t a_hi, uint32_t b_hi,
                                           uint32_t idesc, uint32_t acc) {
     asm volatile(
