@@ -4,8 +4,9 @@
 // was most of preprocessing: a 1 GB database took 123 ms, 14 of them kernels.
 // Here several threads fill pinned slots and enqueue the copies, so the upload
 // runs nearer the PCIe rate (four threads: 60 ms for that database; two 79,
-// eight 68).  Buffers that are already pinned (or not host memory), and small
-// ones, are copied directly.
+// eight 68).  Buffers that are already pinned (or not host memory) are copied
+// directly, and so are those below 128 MB (64 MB: 30 ms of preprocessing either
+// way).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -13,6 +14,7 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <system_error>
 #include <thread>
@@ -34,12 +36,8 @@ class HostUpload {
         if (a.type != cudaMemoryTypeUnregistered || bytes < kMinBytes) return;
         if (cudaGetDevice(&device_) != cudaSuccess) return;
         const size_t n = std::max(1u, std::min(4u, std::thread::hardware_concurrency() / 2));
-        void* p = nullptr;
-        if (cudaHostAlloc(&p, n * 2 * kSlot, cudaHostAllocDefault) != cudaSuccess) {
-            cudaGetLastError();
-            return;
-        }
-        pinned_ = static_cast<uint8_t*>(p);
+        pinned_ = std::make_unique<PinnedPages>(n * 2 * kSlot);
+        if (!pinned_->p) return;
         try {
             workers_.reserve(n);
             for (size_t i = 0; i < n; ++i) workers_.emplace_back([this, i] { work(i); });
@@ -53,7 +51,6 @@ class HostUpload {
         }
         cv_.notify_all();
         for (auto& t : workers_) t.join();  // each waits for its own copies
-        if (pinned_) cudaFreeHost(pinned_);
     }
     HostUpload(const HostUpload&) = delete;
     HostUpload& operator=(const HostUpload&) = delete;
@@ -79,7 +76,7 @@ class HostUpload {
 
   private:
     static constexpr size_t kSlot = (size_t)1 << 20;
-    static constexpr size_t kMinBytes = (size_t)32 << 20;
+    static constexpr size_t kMinBytes = (size_t)128 << 20;
 
     void work(size_t id) {
         cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -96,7 +93,7 @@ class HostUpload {
             const uint8_t* const src = src_ + off;
             const cudaStream_t s = stream_;
             lk.unlock();
-            uint8_t* const buf = pinned_ + (2 * id + k) * kSlot;
+            uint8_t* const buf = pinned_->p + (2 * id + k) * kSlot;
             if (e == cudaSuccess) e = cudaEventSynchronize(ev[k]);  // this slot's last copy has left it
             if (e == cudaSuccess) {
                 std::memcpy(buf, src, n);
@@ -117,7 +114,7 @@ class HostUpload {
     }
 
     int device_ = 0;
-    uint8_t* pinned_ = nullptr;
+    std::unique_ptr<PinnedPages> pinned_;
     std::vector<std::thread> workers_;
     std::mutex mu_;
     std::condition_variable cv_, done_;

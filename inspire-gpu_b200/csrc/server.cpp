@@ -64,6 +64,8 @@ DevTables* upload_tables(DevArena& A, cudaStream_t s) {
 void alloc_precomp(Precomp& P, cudaStream_t s) {
     const size_t R = P.pp.db_rows, C = P.pp.db_cols, G = P.pp.n_packed;
     DevArena& A = P.arena;
+    // The database and the tensors on their own, the rest in one allocation.
+    A.reserve(sizeof(DevTables) + G * (kGroupStrideA + kGroupStrideF) * sizeof(uint32_t), 3);
     P.tables = upload_tables(A, s);
     P.db = A.alloc<uint16_t>(R * C);
     P.pre_a = A.alloc<uint32_t>(G * kGroupStrideA);
@@ -149,7 +151,7 @@ static void preprocess_into(Precomp& P, const uint16_t* db_host, cudaStream_t s,
             }
         }
         // ---- CRS polys a~_r = NTT(tau_{2N-1}(expand_seed("rlwe", r)))  (src/gpu_protocol.cu:569-582)
-        const size_t n_r = R / kN;
+        const size_t n_r = R / kN, h_k_words = 2 * 2 * kDeff * kN;
         std::vector<uint32_t> h_crs(n_r * 2 * kN);
         {
             std::vector<uint32_t> a(2 * kN);
@@ -164,12 +166,16 @@ static void preprocess_into(Precomp& P, const uint16_t* db_host, cudaStream_t s,
                 }
             }
         }
+        const size_t ap_gstride = (size_t)kHalf * 2 * 2 * kN;
+        const size_t wave = std::min<size_t>(G, 64);
+        tmp.reserve((n_r * 2 * kN + h_k_words + 2 * 2 * (size_t)kN * kN +
+                     wave * (ap_gstride + 2 * 2 * kN + 2 * kGroupStrideD)) * sizeof(uint32_t), 8);
         uint32_t* crs = tmp.alloc<uint32_t>(n_r * 2 * kN);
         IPB_CK(cudaMemcpyAsync(crs, h_crs.data(), h_crs.size() * 4, cudaMemcpyHostToDevice, s));
         IPB_CK(launch_ntt_batch(crs, 2 * n_r, 1, false, P.tables, s));
         // ---- ExpandKSK_a sources: K5[j] = expand_seed("ksk", 5*100+j+1), Kn1[j] with (2N-1)*100+j+1
         //      layout [key][limb][digit][N], NTT form (src/gpu_protocol.cu:364-474)
-        std::vector<uint32_t> h_k(2 * 2 * kDeff * kN);
+        std::vector<uint32_t> h_k(h_k_words);
         {
             std::vector<uint32_t> a(2 * kN);
             for (int key = 0; key < 2; ++key)
@@ -189,8 +195,6 @@ static void preprocess_into(Precomp& P, const uint16_t* db_host, cudaStream_t s,
         // ---- per group: a-side -> column NTTs -> ring-embed gather; CollapseA in waves
         uint32_t* V = tmp.alloc<uint32_t>((size_t)2 * kN * kN);
         uint32_t* Tm = tmp.alloc<uint32_t>((size_t)2 * kN * kN);
-        const size_t ap_gstride = (size_t)kHalf * 2 * 2 * kN;
-        const size_t wave = std::min<size_t>(G, 64);
         uint32_t* a_post = tmp.alloc<uint32_t>(wave * ap_gstride);
         uint32_t* ends = tmp.alloc<uint32_t>(wave * 2 * 2 * kN);
         uint32_t* dp_w = tmp.alloc<uint32_t>(wave * kGroupStrideD);  // D in the reference layout, one wave
@@ -252,6 +256,7 @@ size_t lane_bytes(const Server& S, size_t cap) {
 void alloc_lane(const Server& S, Lane& L, size_t cap, int gt_pass) {
     const size_t R = S.pp.db_rows, G = S.pp.n_packed;
     DevArena& A = L.arena;
+    A.reserve(lane_bytes(S, cap), 14);
     L.cap = cap;
     L.gt_pass = gt_pass;
     L.qraw = A.alloc<uint64_t>(cap * S.qstride);
@@ -268,7 +273,6 @@ void alloc_lane(const Server& S, Lane& L, size_t cap, int gt_pass) {
     L.wire_in = A.alloc<uint8_t>(cap * S.wire_q);
     L.wire_out = A.alloc<uint8_t>(cap * std::max(S.wire_r, S.wire_c));
     L.codec_tmp = A.alloc<uint32_t>(cap * S.pp.num_cts * 4 * kN);
-    IPB_CK(cudaHostAlloc(reinterpret_cast<void**>(&L.bounce), Lane::kBounceBytes + sizeof(int), cudaHostAllocDefault));
     IPB_CK(cudaStreamCreateWithFlags(&L.aux, cudaStreamNonBlocking));
     IPB_CK(cudaEventCreateWithFlags(&L.fork, cudaEventDisableTiming));
     IPB_CK(cudaEventCreateWithFlags(&L.join, cudaEventDisableTiming));
@@ -318,6 +322,7 @@ Server* make_server(const Params& pp, std::shared_ptr<Precomp> pre, size_t max_b
     const int gt_pass = lane_gt_pass(max_batch);
     S->sched = default_sched(*S, max_batch, gt_pass);
     alloc_lane(*S, S->lane, max_batch, gt_pass);
+    S->lane.bounce = std::make_unique<PinnedPages>(Lane::kBounceBytes + sizeof(int));
     S->ev.assign(6 * ((max_batch + kSliceQueries - 1) / kSliceQueries), nullptr);
     for (auto& e : S->ev) IPB_CK(cudaEventCreate(&e));
     pre->adopted = true;
@@ -931,18 +936,19 @@ void check_device_error(Lane& L, cudaStream_t st) {
 // small responses come with the error word through the lane's pinned buffer
 // (one wait; 10 us of a one-query answer), large ones after it has been read.
 static void deliver(Lane& L, cudaStream_t st, const void* src, size_t bytes, void* out) {
-    if (bytes > Lane::kBounceBytes) {
+    if (bytes > Lane::kBounceBytes || !L.bounce || !L.bounce->p) {
         check_device_error(L, st);
         IPB_CK(cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, st));
         IPB_CK(cudaStreamSynchronize(st));
         return;
     }
-    int* const e = reinterpret_cast<int*>(L.bounce + Lane::kBounceBytes);
+    uint8_t* const bounce = L.bounce->p;
+    int* const e = reinterpret_cast<int*>(bounce + Lane::kBounceBytes);
     IPB_CK(cudaMemcpyAsync(e, L.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    IPB_CK(cudaMemcpyAsync(L.bounce, src, bytes, cudaMemcpyDeviceToHost, st));
+    IPB_CK(cudaMemcpyAsync(bounce, src, bytes, cudaMemcpyDeviceToHost, st));
     IPB_CK(cudaStreamSynchronize(st));
     raise_device_error(L, st, *e);
-    std::memcpy(out, L.bounce, bytes);
+    std::memcpy(out, bounce, bytes);
 }
 
 static void fetch(Server* S, size_t count, uint64_t* out) {

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdlib>
+#include <cstring>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -49,16 +51,39 @@ struct DeviceRestore {
     DeviceRestore& operator=(const DeviceRestore&) = delete;
 };
 
-// Device allocations freed together.
+// Device allocations freed together.  reserve() makes one allocation that
+// later ones are carved from (a cudaMalloc and its cudaFree take 0.6 ms here,
+// and a server has two dozen buffers); what does not fit, or was not reserved,
+// gets its own.
 struct DevArena {
     std::vector<void*> ptrs;
     size_t bytes = 0;
+    uint8_t* slab = nullptr;
+    size_t slab_left = 0;
+    // Room for allocations of `total` bytes in all, `count` of them.
+    void reserve(size_t total, size_t count) {
+        void* p = nullptr;
+        const size_t b = total + count * kAlign;
+        if (cudaMalloc(&p, b) != cudaSuccess) {
+            cudaGetLastError();  // no block of that size: one allocation each
+            return;
+        }
+        ptrs.push_back(p);
+        slab = static_cast<uint8_t*>(p);
+        slab_left = b;
+    }
     template <class T>
     T* alloc(size_t count) {
         void* p = nullptr;
-        const size_t b = count * sizeof(T);
-        IPB_CK(cudaMalloc(&p, b ? b : 16));
-        ptrs.push_back(p);
+        const size_t b = count * sizeof(T), padded = (b + kAlign - 1) / kAlign * kAlign;
+        if (padded <= slab_left && padded > 0) {
+            p = slab;
+            slab += padded;
+            slab_left -= padded;
+        } else {
+            IPB_CK(cudaMalloc(&p, b ? b : 16));
+            ptrs.push_back(p);
+        }
         bytes += b;
         return static_cast<T*>(p);
     }
@@ -66,7 +91,37 @@ struct DevArena {
         for (void* p : ptrs) cudaFree(p);
         ptrs.clear();
         bytes = 0;
+        slab = nullptr;
+        slab_left = 0;
     }
+
+  private:
+    static constexpr size_t kAlign = 256;
+};
+
+// Pinned host memory: ordinary pages, registered (0.3 ms for 256 KB; a
+// cudaHostAlloc takes 1.4-3 ms here).  Null where that fails.
+struct PinnedPages {
+    uint8_t* p = nullptr;
+    explicit PinnedPages(size_t n) {
+        n = (n + 4095) / 4096 * 4096;
+        void* m = std::aligned_alloc(4096, n);
+        if (!m) return;
+        std::memset(m, 0, n);
+        if (cudaHostRegister(m, n, cudaHostRegisterDefault) != cudaSuccess) {
+            cudaGetLastError();
+            std::free(m);
+            return;
+        }
+        p = static_cast<uint8_t*>(m);
+    }
+    ~PinnedPages() {
+        if (!p) return;
+        cudaHostUnregister(p);
+        std::free(p);
+    }
+    PinnedPages(const PinnedPages&) = delete;
+    PinnedPages& operator=(const PinnedPages&) = delete;
 };
 
 constexpr size_t kGroupStrideD = (size_t)2 * kSteps * kDeff * kN;  // u32 per group, D_plus / D_minus
@@ -152,7 +207,7 @@ struct Lane {
     uint8_t* wire_out = nullptr; // packed or compressed responses
     uint32_t* codec_tmp = nullptr;  // coefficient-form responses for compression
     static constexpr size_t kBounceBytes = (size_t)256 << 10;
-    uint8_t* bounce = nullptr;      // pinned: a small batch's responses, then the error word
+    std::unique_ptr<PinnedPages> bounce;  // a small batch's responses, then the error word (blocking calls only)
     cudaStream_t aux = nullptr;     // the blocking path's copies
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaEvent_t rgsw_ready = nullptr;  // RGSW parts staged and prepared on aux
@@ -170,7 +225,6 @@ struct Lane {
         if (join) cudaEventDestroy(join);
         if (fork) cudaEventDestroy(fork);
         if (aux) cudaStreamDestroy(aux);
-        if (bounce) cudaFreeHost(bounce);
         arena.free_all();
     }
 };
