@@ -248,19 +248,22 @@ int ipir_b200_fill_db_device(uint16_t* out, size_t count, uint64_t seed, void* s
  * (matvec_tc = 1) or the CUDA cores (0); queries per tensor-pass GEMM
  * (tp_pass); Horner on a 4-CTA cluster per chain (horner_cluster = 1), an
  * 8-CTA cluster (2) or one CTA per chain (0); tp_sms > 0 runs the tensor
- * pass on that many SMs at the same time as the tensor-core mat-vec on the
- * others (the two read disjoint data: the tensor pass is DRAM-bound, the
- * batched mat-vec tensor-core-bound), 0 runs them one after the other;
- * slice = 32 runs a batch of more than 32 queries as consecutive 32-query
- * pipelines (query prep to Horner), 0 as one pipeline; hchunks = 2..16
- * runs the tensor pass first and then the mat-vec and finalize in at most
- * that many group chunks (whole waves of mat-vec work) from the top group
- * down, each chunk's Horner steps on a second stream as soon as its packed
- * ciphertexts are final (databases whose response ciphertexts all chain
- * the same number of groups L = min(D, G), cluster Horner kernels, batches
- * of at most 32; the blocking and staged paths and the serving loop's lane
- * batches), 0 off; the default schedule uses 8 on such databases with
- * L >= 32 for batches of at most min(16, L / 16) queries.  Every schedule gives the same responses. */
+ * pass on that many SMs while the tensor-core mat-vec starts on the others
+ * (it takes those SMs over as the tensor pass ends; the two read disjoint
+ * data), 0 runs them one after the other; slice = 32 runs a batch of more
+ * than 32 queries as consecutive 32-query pipelines (query prep to Horner;
+ * the prep and tensor pass of two slices run as one), 0 as one pipeline;
+ * hchunks = 2..16 runs the tensor pass first and then the mat-vec and
+ * finalize in at most that many group chunks (whole waves of mat-vec work)
+ * from the top group down, each chunk's Horner steps on a second stream as
+ * soon as its packed ciphertexts are final (databases whose response
+ * ciphertexts all chain the same number of groups L = min(D, G), cluster
+ * Horner kernels, batches of at most 32; the blocking and staged paths and
+ * the serving loop's lane batches), 0 off.  Defaults: horner_cluster 2 up to
+ * 15 chains, else 1; hchunks 8 (4 above two queries) with horner_cluster 1 on
+ * databases of at least 16384 rows with L >= 64, for batches of at most
+ * min(16, L / 8) queries; otherwise tp_sms two thirds of the SMs where the
+ * database and its tensors take at most 8 GB.  Every schedule gives the same responses. */
 typedef struct {
     int matvec_tc;
     int tp_pass;

@@ -969,12 +969,14 @@ static void fetch(Server* S, size_t count, uint64_t* out) {
 // For batch sizes 1, 2, 4, ... up to the lane's capacity (and the capacity
 // itself) time every candidate schedule end to end on the device -- mat-vec
 // kernel (tcgen05 / CUDA-core; the CUDA-core kernel streams the DB once per
-// 4 queries, so it is tried up to 8), queries per tensor-pass GEMM (the
-// key-table capacity and its half: fewer queries per pass re-read the
-// tensors but double-buffer the accumulators), Horner kernel (4-CTA
-// cluster, 8-CTA cluster, single CTA) -- and keep the fastest; then, for the
-// tensor-core mat-vec, the number of SMs (1/18 .. 8/18 of them) that run the
-// tensor pass at the same time as the mat-vec, if that is faster still.
+// 4 queries, so it is tried up to 8), queries per tensor-pass GEMM (the most
+// one launch takes and half of that: smaller passes re-read the tensors),
+// Horner kernel (4-CTA cluster, 8-CTA cluster, single CTA) -- and keep the
+// fastest; then, for the tensor-core mat-vec, the number of SMs (1/18 .. 8/18
+// of them) that run the tensor pass at the same time as the mat-vec, if that
+// is faster still; then the chain in chunks; and the size's default schedule
+// where it still beats that (its splits and chunk counts are not all among the
+// candidates).
 // Batches larger than 32 queries also try one pipeline for the whole batch
 // against consecutive 32-query slices.  Sizes between two measured ones use
 // the smaller's.
@@ -987,6 +989,7 @@ std::vector<Sched> autotune(const Server& S, Lane& L, cudaStream_t st) {
     IPB_CK(cudaEventCreate(&e0));
     IPB_CK(cudaEventCreate(&e1));
     std::vector<std::pair<size_t, Sched>> best;
+    const std::vector<Sched> defaults = default_sched(S, L.cap, L.gt_pass);
     try {
         for (size_t b : sizes) {
             std::vector<Sched> cands;
@@ -1078,6 +1081,15 @@ std::vector<Sched> autotune(const Server& S, Lane& L, cudaStream_t st) {
                     const size_t i = (size_t)(std::min_element(t.begin(), t.end()) - t.begin());
                     if (t[i] < a * 0.98f) pick = chs[i];
                 }
+            }
+            {
+                const Sched& def = defaults[b];
+                float a = 1e30f, d = 1e30f;
+                for (int r = 0; r < 3; ++r) {
+                    a = std::min(a, time_of(pick));
+                    d = std::min(d, time_of(def));
+                }
+                if (d < a * 0.99f) pick = def;
             }
             best.emplace_back(b, pick);
         }
