@@ -35,11 +35,7 @@ cudaError_t launch_matvec(const uint16_t* db, size_t rows, size_t cols, int chun
 // receives a nonzero code if a pipeline wait times out.
 size_t mv_tc_planes_bytes(size_t rows, int max_queries);
 size_t mv_tc_planes_offset(size_t first_query, size_t rows);
-// Rows per K chunk for a pass of nq queries.
-int matvec_tc_kchunk_rows(size_t rows, size_t cols, int num_sms, int nq);
-// DB columns per mat-vec work item of a pass of nq queries over a DB of ld
-// columns per row.
-int matvec_tc_item_cols(int nq, size_t rows, size_t ld, int kchunk_rows);
+// (K chunks and columns per work item: matvec_rules.h.)
 // tiles: two device words, zero between launches, that the kernel's CTAs draw
 // work items from (one pair per concurrently running launch).
 cudaError_t launch_matvec_tc(const uint16_t* db, size_t rows, size_t cols, const uint8_t* planes, int nq,

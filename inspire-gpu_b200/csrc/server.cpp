@@ -21,6 +21,7 @@
 #include "inspire_b200.h"
 #include "inspire_b200.hpp"
 #include "host_upload.h"
+#include "matvec_rules.h"
 #include "server_internal.h"
 
 namespace ipb {

@@ -33,3 +33,25 @@ def test_matvec_item_shapes(rows, cols, kchunk, count):
         hi = (q[:, l] >> 14).astype(np.float64) @ f
         want = (lo.astype(np.int64) + (hi.astype(np.int64) % m << 14)) % m
         assert (out[:, l].cpu().numpy() == want).all(), l
+
+
+@pytest.mark.parametrize("rows,cols", [(17408, 3072), (31744, 2432), (17408, 1024)])
+@pytest.mark.parametrize("count", [1, 9])
+def test_default_chunks_of_odd_row_counts(rows, cols, count):
+    """Rows an odd multiple of 1024 above 16384 with few columns: the default
+    K chunk is halved until the halves are no longer whole stages."""
+    import inspire_b200 as ib
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(rows + cols + count)
+    db = torch.randint(0, 65536, (rows, cols), device="cuda", generator=g, dtype=torch.int32)
+    db16 = db.to(torch.int16)
+    q = torch.stack([torch.randint(0, m, (count, rows), device="cuda", generator=g) for m in QS], 1).contiguous()
+    out = torch.zeros((count, 2, cols), dtype=torch.int32, device="cuda")
+    ib.matvec(db16.data_ptr(), rows, cols, q.data_ptr(), count, out.data_ptr(),
+              torch.cuda.current_stream().cuda_stream)
+    f = db.to(torch.float64)  # 16-bit entries, 14-bit halves, < 2^15 rows: sums below 2^45, exact
+    for l, m in enumerate(QS):
+        lo = (q[:, l] & 0x3FFF).to(torch.float64) @ f
+        hi = (q[:, l] >> 14).to(torch.float64) @ f
+        want = (lo.to(torch.int64) + (hi.to(torch.int64) % m << 14)) % m
+        assert (out[:, l] == want).all(), l
