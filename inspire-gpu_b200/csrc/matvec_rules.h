@@ -28,33 +28,43 @@ inline bool mv_kchunk_ok(size_t rows, int kchunk_rows) {
 // with one tile and 2.48 with two, 4: 2.50 / 2.57, 8: 2.78 / 2.59), and if the
 // accumulators are double-buffered or an item long enough for that not to
 // matter (16 queries, 640 rows an item: 31 us with one tile, 36 with two; 2048
-// rows 214 / 217; 8192 rows 214 / 196).
-inline int mv_tiles(int nq, size_t rows, size_t ld, int kchunk_rows) {
+// rows 214 / 217; 8192 rows 214 / 196).  pairs: the launch's tiles pair up
+// (an even number of them in every column range).
+inline int mv_tiles(int nq, size_t rows, size_t ld, int kchunk_rows, bool pairs) {
     const int npad = (kPlanes * nq + 15) / 16 * 16;
-    if (4 * npad > 512 || (8 * npad > 512 && kchunk_rows < 4096)) return 1;
+    if (!pairs || 4 * npad > 512 || (8 * npad > 512 && kchunk_rows < 4096)) return 1;
     return 2.0 * (double)rows * (double)ld <= 6e9 || nq >= 6 ? 2 : 1;
 }
 // Rows per exact s32 accumulation: at most 32768, halved while there are
 // fewer than two work items per SM and the half is whole stages (17408 rows
 // end at 1088).
 inline int matvec_tc_kchunk_rows(size_t rows, size_t cols, int num_sms, int nq) {
+    const size_t mtiles = (2 * cols) / kMT, sms = (size_t)num_sms;
+    const bool pairs = mtiles % 2 == 0;
     auto chunk = [&](size_t tiles_per_item) {
         size_t kc = rows < (size_t)kKChunk ? rows : (size_t)kKChunk;
-        const size_t mtiles = (2 * cols) / kMT;
-        while (mtiles * (rows / kc) < tiles_per_item * (size_t)(2 * num_sms) && kc > 1024 && kc % (2 * kKT) == 0)
-            kc /= 2;
+        while (mtiles * (rows / kc) < tiles_per_item * 2 * sms && kc > 1024 && kc % (2 * kKT) == 0) kc /= 2;
         return (int)kc;
     };
-    // With two tiles per item the chunks are halved once more where that leaves
-    // the pass on two tiles (21 groups, 8 queries: 768 -> 708 us, one tile 730).
     const int one = chunk(1);
-    if (mv_tiles(nq, rows, cols, one) == 1) return one;
+    if (mv_tiles(nq, rows, cols, one, true) == 1) return one;
     const int two = chunk(2);
-    return mv_tiles(nq, rows, cols, two) == 2 ? two : one;
+    // Tiles that do not pair up: the chunks are halved once more where the last
+    // wave of items is fuller then (1 query: 32768 x 38528, 301 items in three
+    // waves to 602 in five, 470 -> 411 us; 8192 x 20608, 322 to 644, 72 -> 65), not
+    // where only the second chunk's sum is added (4096 x 49024, 383 in three to
+    // 766 in six: 70 -> 77).
+    if (!pairs) {
+        const size_t n = mtiles * (rows / (size_t)one);
+        if (2 * ((n + sms - 1) / sms) <= (2 * n + sms - 1) / sms) return one;
+    }
+    // Pairs: once more where that leaves the pass on two tiles per item (21
+    // groups, 8 queries: 768 -> 708 us, one tile 730).
+    return mv_tiles(nq, rows, cols, two, true) == 2 ? two : one;
 }
-// DB columns per work item of a pass of nq queries.
-inline int matvec_tc_item_cols(int nq, size_t rows, size_t ld, int kchunk_rows) {
-    return kMT / 2 * mv_tiles(nq, rows, ld, kchunk_rows);
+// DB columns per work item of a pass of nq queries over ranges of cols columns.
+inline int matvec_tc_item_cols(int nq, size_t rows, size_t ld, size_t cols, int kchunk_rows) {
+    return kMT / 2 * mv_tiles(nq, rows, ld, kchunk_rows, (2 * cols) / kMT % 2 == 0);
 }
 
 }  // namespace ipb

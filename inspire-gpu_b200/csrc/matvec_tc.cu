@@ -451,7 +451,7 @@ cudaError_t launch_matvec_tc_ranges(const uint16_t* db, size_t rows, size_t ld, 
     P.n_mtiles = n_ranges > 1 ? n_ranges * P.mt_per_range : (int)((2 * cols) / kMT);
     P.kchunk_rows = kchunk;
     P.n_kchunks = (int)(rows / kchunk);
-    const int mt = P.n_mtiles % 2 == 0 && P.mt_per_range % 2 == 0 ? mv_tiles(nq, rows, ld, kchunk) : 1;
+    const int mt = mv_tiles(nq, rows, ld, kchunk, P.n_mtiles % 2 == 0 && P.mt_per_range % 2 == 0);
     P.acc_stages = (4 * mt * npad <= 512) ? 2 : 1;
     uint32_t need = (uint32_t)(P.acc_stages * 2 * mt * npad);
     uint32_t tc = 32;

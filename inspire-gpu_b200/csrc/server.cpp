@@ -700,7 +700,7 @@ static int run_chunked(const Server& S, Lane& L, const Sched& sc, size_t count, 
     // mat-vec launch covers the range in all of them.
     const size_t nct = pp.num_cts, d_act = std::min(pp.D, G);
     const int kchunk = kchunk_rows(S, count), kchunks = (int)(R / (size_t)kchunk);
-    const size_t ipg = (kN / (size_t)matvec_tc_item_cols(nq, R, C, kchunk)) * (size_t)kchunks * nct;
+    const size_t ipg = (kN / (size_t)matvec_tc_item_cols(nq, R, C, kN, kchunk)) * (size_t)kchunks * nct;
     const std::vector<size_t> sizes =
         chunk_sizes(d_act, ipg, S.num_sms, std::min<size_t>((size_t)sc.hchunks, kMaxHChunks));
     IPB_CK(cudaEventRecord(L.hjoin, st));               // the Horner stream starts after this batch's prep

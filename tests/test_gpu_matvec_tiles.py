@@ -35,11 +35,12 @@ def test_matvec_item_shapes(rows, cols, kchunk, count):
         assert (out[:, l].cpu().numpy() == want).all(), l
 
 
-@pytest.mark.parametrize("rows,cols", [(17408, 3072), (31744, 2432), (17408, 1024)])
+@pytest.mark.parametrize("rows,cols", [(17408, 3072), (31744, 2432), (17408, 1024), (32768, 38528), (4096, 49024)])
 @pytest.mark.parametrize("count", [1, 9])
-def test_default_chunks_of_odd_row_counts(rows, cols, count):
+def test_default_chunks(rows, cols, count):
     """Rows an odd multiple of 1024 above 16384 with few columns: the default
-    K chunk is halved until the halves are no longer whole stages."""
+    K chunk is halved until the halves are no longer whole stages; and an odd
+    number of tiles, halved once more and not."""
     import inspire_b200 as ib
     import torch
     g = torch.Generator(device="cuda").manual_seed(rows + cols + count)

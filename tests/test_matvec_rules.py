@@ -1,5 +1,6 @@
 """The mat-vec's own choice of K chunks (csrc/matvec_rules.h) over the shapes
-its entry points accept: every choice meets the launch's conditions."""
+its entry points accept: every choice meets the launch's conditions, and
+tiles that do not pair up are not split for pairs."""
 import os
 import shutil
 import subprocess
@@ -44,3 +45,12 @@ def _sweep(tmp_path, check):
 
 def test_every_default_chunk_is_accepted_by_the_launch(tmp_path):
     _sweep(tmp_path, "mv_kchunk_ok(rows, kc)")
+
+
+def test_odd_tile_counts_split_for_the_last_wave_only(tmp_path):
+    """An odd number of 128-column tiles runs one tile per item.  A chunk whose
+    double already gives two items per SM is there only because the items'
+    last wave is fuller."""
+    _sweep(tmp_path, "cols / 128 % 2 == 0 || 2 * kc > kKChunk || rows % (2 * (size_t)kc) || "
+                     "cols / 128 * (rows / (2 * kc)) < 2 * (size_t)sms || "
+                     "2 * ((cols / 128 * (rows / (2 * kc)) + sms - 1) / sms) > (cols / 128 * (rows / kc) + sms - 1) / sms")
