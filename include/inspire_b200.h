@@ -117,7 +117,8 @@ int ipir_b200_sync(ipir_server* srv);
 
 /* Stage timers (CUDA events on the handle's stream), off by default.
  * stage_times writes up to n floats (ms) of the last run:
- * [qprep, matvec, collapse, finalize, horner]. */
+ * [qprep, matvec, collapse, finalize, horner].  While they are on, the stages
+ * run one after the other (schedule fields tp_sms and hchunks do not apply). */
 int ipir_b200_enable_stage_timing(ipir_server* srv, int on);
 int ipir_b200_stage_times(const ipir_server* srv, float* ms_out, size_t n);
 

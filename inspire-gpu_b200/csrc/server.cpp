@@ -503,8 +503,8 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
     // Beside: the tensor pass (keys only) on sc.tp_sms SMs from the lane's
     // Horner stream while the mat-vec (DB only) starts on the other SMs; both
     // are persistent with one CTA per SM, so the mat-vec's remaining CTAs start
-    // as the tensor pass's end.
-    const bool beside = sc.matvec_tc && sc.tp_sms > 0 && sc.tp_sms < S.num_sms && span > 0;
+    // as the tensor pass's end.  Stage timing needs them one after the other.
+    const bool beside = !ev && sc.matvec_tc && sc.tp_sms > 0 && sc.tp_sms < S.num_sms && span > 0;
     auto tensor_pass = [&](cudaStream_t ts, int sms) {
         for (size_t c0 = 0; c0 < span; c0 += tp_pass) {
             const int n = (int)std::min(tp_pass, span - c0);
@@ -545,8 +545,7 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
         }
         mv_parts = S.mv_chunks;
     }
-    if (beside)
-        IPB_CK(cudaStreamWaitEvent(st, L.hjoin, 0));  // stage times: mat-vec = both, tensor pass = 0
+    if (beside) IPB_CK(cudaStreamWaitEvent(st, L.hjoin, 0));
     if (ev) IPB_CK(cudaEventRecord(ev[2], st));
     if (!beside && !lwe_ready) tensor_pass(st, S.num_sms);
     if (ev) IPB_CK(cudaEventRecord(ev[3], st));
@@ -813,7 +812,7 @@ int run_pipeline(const Server& S, Lane& L, const Sched& sc, size_t count, cudaSt
         throw std::invalid_argument("run_pipeline: batch exceeds the lane or its tensor-pass buffer");
     const size_t ns = slices_of(count, sc), slice = sc.slice > 0 ? (size_t)sc.slice : count;
     // Stage timing needs the stages one after the other: it times the
-    // unchunked pipeline.
+    // unchunked pipeline, the tensor pass after the mat-vec.
     if (phases == kPhaseAll && !ev && chunked_ok(S, sc, count))
         return run_chunked(S, L, sc, count, st, nullptr, nullptr, db_done);
     if (phases != kPhaseAll || 6 * ns > n_ev) ev = nullptr;
