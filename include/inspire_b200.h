@@ -281,7 +281,10 @@ int ipir_b200_autotune(ipir_server* srv);
 /* The schedule the handle uses for `count` queries. */
 int ipir_b200_get_schedule(const ipir_server* srv, size_t count, ipir_serve_schedule* out);
 /* Pin the schedule the handle uses for `count` queries (tp_pass at most
- * min(max_batch, 32)): 0, 1 null argument, 2 out of range. */
+ * min(max_batch, 32)): 0, 1 null argument, 2 out of range.  tp_sms > 0 excludes
+ * chunks (hchunks is then ignored) and the CUDA-core mat-vec (refused); only
+ * the default tp_sms, as get_schedule reports it, gives way to either and is
+ * stored as 0. */
 int ipir_b200_set_schedule(ipir_server* srv, size_t count, const ipir_serve_schedule* sc);
 /* Kernels launched by the handle's answer pipeline since create. */
 int ipir_b200_launch_count(const ipir_server* srv, unsigned long long* out);

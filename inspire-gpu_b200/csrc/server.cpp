@@ -419,6 +419,14 @@ int lane_gt_pass(size_t cap) { return (int)std::min<size_t>(cap, (size_t)kTpMaxQ
 
 static bool chunked_ok(const Server& S, const Sched& sc, size_t count);
 
+// SMs for the tensor pass beside the mat-vec where nothing else is asked for
+// (default_sched has the measurements).
+static int default_tp_sms(const Server& S) {
+    const double stream_bytes =
+        2.0 * (double)S.pp.db_rows * (double)S.pp.db_cols + (double)tp_dt_bytes(S.pp.n_packed);
+    return stream_bytes <= 8e9 ? S.num_sms * 2 / 3 : 0;
+}
+
 // Defaults per batch size, each line drawn where both sides measured alike
 // (one GPU, medians of interleaved runs):
 //   Horner kernel: 8 CTAs per chain while all clusters run at once (up to 15
@@ -441,7 +449,6 @@ static bool chunked_ok(const Server& S, const Sched& sc, size_t count);
 // batch size.
 std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
     const size_t G = S.pp.n_packed, chain = std::min(S.pp.D, G);  // groups per response ciphertext
-    const double stream_bytes = 2.0 * (double)S.pp.db_rows * (double)S.pp.db_cols + (double)tp_dt_bytes(G);
     const char* const m = std::getenv("IPB_MATVEC");
     const char* const h = std::getenv("IPB_HORNER");
     const char* const t = std::getenv("IPB_TP_SMS");
@@ -462,7 +469,7 @@ std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
         if (k) sc.hchunks = std::max(0, std::min(std::atoi(k), kMaxHChunks));
         if (!sc.matvec_tc) continue;
         if (t) sc.tp_sms = std::max(0, std::min(std::atoi(t), S.num_sms - 1));
-        else if (sc.hchunks <= 1 && stream_bytes <= 8e9) sc.tp_sms = S.num_sms * 2 / 3;
+        else if (sc.hchunks <= 1) sc.tp_sms = default_tp_sms(S);
     }
     return out;
 }
@@ -575,6 +582,13 @@ static bool chunked_ok(const Server& S, const Sched& sc, size_t count) {
 }
 
 bool runs_chunked(const Server& S, const Sched& sc, size_t count) { return chunked_ok(S, sc, count); }
+
+void yield_default_split(const Server& S, Sched& sc, size_t count) {
+    if (std::getenv("IPB_TP_SMS") || sc.tp_sms != default_tp_sms(S)) return;
+    Sched whole = sc;
+    whole.tp_sms = 0;
+    if (!sc.matvec_tc || chunked_ok(S, whole, count)) sc = whole;
+}
 
 float time_plain_answer(Server& S) {
     IPB_CK(cudaSetDevice(S.device));
@@ -1546,16 +1560,18 @@ int ipir_b200_set_schedule(ipir_server* srv, size_t count, const ipir_serve_sche
     if (!srv || !sc) return 1;
     ipb::Server* S = srv->s;
     if (count == 0 || count > S->max_batch) return 2;
-    if (sc->matvec_tc < 0 || sc->matvec_tc > 1 || sc->horner_cluster < 0 || sc->horner_cluster > 2 ||
-        sc->tp_pass < 1 || sc->tp_pass > S->lane.gt_pass || sc->tp_sms < 0 || sc->tp_sms >= S->num_sms ||
-        (sc->tp_sms > 0 && !sc->matvec_tc) || (sc->slice != 0 && sc->slice != (int)ipb::kSliceQueries) ||
-        sc->hchunks < 0 || sc->hchunks > ipb::kMaxHChunks) {
+    ipb::Sched want{sc->matvec_tc, sc->tp_pass, sc->horner_cluster, sc->tp_sms, sc->slice, sc->hchunks};
+    ipb::yield_default_split(*S, want, count);
+    if (want.matvec_tc < 0 || want.matvec_tc > 1 || want.horner_cluster < 0 || want.horner_cluster > 2 ||
+        want.tp_pass < 1 || want.tp_pass > S->lane.gt_pass || want.tp_sms < 0 || want.tp_sms >= S->num_sms ||
+        (want.tp_sms > 0 && !want.matvec_tc) || (want.slice != 0 && want.slice != (int)ipb::kSliceQueries) ||
+        want.hchunks < 0 || want.hchunks > ipb::kMaxHChunks) {
         ipb::g_last_error =
             "ipir_b200_set_schedule: matvec_tc 0/1, horner_cluster 0/1/2, tp_pass 1..capacity, "
             "tp_sms 0..SMs-1 (0 with the CUDA-core mat-vec), slice 0/32, hchunks 0..16";
         return 2;
     }
-    S->sched[count] = ipb::Sched{sc->matvec_tc, sc->tp_pass, sc->horner_cluster, sc->tp_sms, sc->slice, sc->hchunks};
+    S->sched[count] = want;
     return 0;
 }
 

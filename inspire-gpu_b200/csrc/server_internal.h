@@ -283,6 +283,10 @@ int run_pipeline(const Server& S, Lane& L, const Sched& sc, size_t count, cudaSt
 // chain trailing the DB pass in group chunks (then the DB and Horner phases
 // cannot be run apart).
 bool runs_chunked(const Server& S, const Sched& sc, size_t count);
+// A schedule read back and changed still holds the default split of the SMs
+// (tp_sms): it gives way to what it excludes, chunks and the CUDA-core mat-vec.
+// Other values, IPB_TP_SMS among them, were asked for and stand.
+void yield_default_split(const Server& S, Sched& sc, size_t count);
 // Device time (ms, best of three after one warm run) of one plain answer
 // through the handle's own lane and schedule, on a stream of its own.
 float time_plain_answer(Server& S);

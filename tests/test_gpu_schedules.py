@@ -1,11 +1,10 @@
 """What the schedules of small databases promise beyond equal answers (those
 split the SMs between the tensor pass and the mat-vec by default)."""
-import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-R, G = 2048, 8
+R, G = 2048, 32
 
 
 @pytest.fixture(scope="module")
@@ -24,7 +23,7 @@ def queries():
 
 
 def test_stage_times_separate_the_two_passes(srv, queries):
-    """Timed, the tensor pass has its own stage: at least its 0.54 GB at the
+    """Timed, the tensor pass has its own stage: at least its 2.1 GB at the
     memory's nominal 8 TB/s."""
     assert srv.schedule(1)["tp_sms"] > 0
     want = srv.answer(queries[0])
@@ -33,5 +32,32 @@ def test_stage_times_separate_the_two_passes(srv, queries):
     st = srv.stage_times()
     srv.enable_stage_timing(False)
     assert (got == want).all()
-    assert st["collapse"] > 0.067, st
+    assert st["collapse"] > 0.26, st
     assert all(v > 0 for v in st.values()), st
+
+
+def test_a_schedule_read_back_takes_chunks_and_the_cuda_core_matvec(srv, queries):
+    """The default split of the SMs gives way to what it excludes; a split that
+    was asked for stands."""
+    first = srv.schedule(2)
+    want = srv.answer_batch(queries[:2])
+
+    def launches(**kw):
+        srv.set_schedule(2, **{**first, **kw})
+        n0 = srv.launch_count()
+        assert (srv.answer_batch(queries[:2]) == want).all(), kw
+        return srv.launch_count() - n0
+
+    split = first["tp_sms"]
+    assert split > 0 and first["hchunks"] == 0
+    whole = launches()
+    assert srv.schedule(2) == first
+    assert launches(hchunks=2) > whole       # two chunks: two mat-vecs, two finalizes
+    assert (srv.schedule(2)["tp_sms"], srv.schedule(2)["hchunks"]) == (0, 2)
+    launches(matvec_tc=0)
+    assert (srv.schedule(2)["tp_sms"], srv.schedule(2)["matvec_tc"]) == (0, 0)
+    assert launches(hchunks=2, tp_sms=40) == whole and srv.schedule(2)["tp_sms"] == 40
+    assert launches(hchunks=2, horner_cluster=0) == whole and srv.schedule(2)["tp_sms"] == split
+    with pytest.raises(Exception):
+        launches(matvec_tc=0, tp_sms=40)
+    srv.set_schedule(2, **first)
