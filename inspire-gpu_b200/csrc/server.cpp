@@ -5,9 +5,11 @@
 // Reference counterparts: src/gpu_protocol.cu (GpuServerCtx, gpu_preprocess,
 // gpu_setup_server, answer_one, gpu_answer_batch, caps, free) and
 // src/capi.cu (the C ABI server half).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -369,11 +371,47 @@ static void stage_queries(Server* S, const ipir_query_view* qs, size_t count) {
     S->staged = count;
 }
 
+// The range of pinned host memory (one allocation or registration) that holds
+// p, or size 0 for other memory.  The driver's entry point through the runtime:
+// the library needs no -lcuda.
+static void pinned_range(const void* p, uintptr_t& start, size_t& size) {
+    using Get = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const Get get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &r) == cudaSuccess &&
+                        r == cudaDriverEntryPointSuccess;
+        return ok ? reinterpret_cast<Get>(f) : nullptr;
+    }();
+    const CUdeviceptr at = (CUdeviceptr)(uintptr_t)p;
+    CUdeviceptr first = 0;
+    size = 0;
+    if (!get || get(&first, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+        size = 0;
+    start = (uintptr_t)first;
+}
+
+// Whether `count` rows of `width` words, `pitch` words apart from p on, are
+// parts of one array: of one pinned range at any pitch a 2-D copy takes, or of
+// pageable queries back to back.  Queries of separate allocations can have a
+// constant stride too (two always do), of any size, some pinned and some not.
+static bool one_array(const uint64_t* p, size_t pitch, size_t width, size_t count, size_t qstride) {
+    if (pitch > (size_t)INT32_MAX / 8) return false;
+    const uint64_t* const end = p + (count - 1) * pitch + width;
+    uintptr_t start = 0;
+    size_t size = 0;
+    pinned_range(p, start, size);
+    if (size) return (uintptr_t)end <= start + size;
+    pinned_range(end - 1, start, size);
+    return size == 0 && pitch == qstride;
+}
+
 // Host -> device copy of parts [p0, p0 + np) of every query (0, 1: the LWE
 // limbs; 2, 3, 4: KSK5, KSK-1, RGSW) into their place in the lane's flat
 // query buffer.  One 2-D copy when each query's parts are back to back in
-// host memory at a constant stride between queries (a flat batch array),
-// else one copy per host-contiguous run.
+// host memory at a constant stride between queries within one array, else one
+// copy per host-contiguous run.
 void stage_parts(const Server& S, const ipir_query_view* qs, size_t count, int p0, int np, cudaStream_t st) {
     const size_t R = S.pp.db_rows;
     const size_t len[5] = {R, R, kBlk, kBlk, 4 * kBlk};
@@ -389,9 +427,10 @@ void stage_parts(const Server& S, const ipir_query_view* qs, size_t count, int p
         for (int p = p0 + 1; p < p0 + np; ++p) strided = strided && ptr(i, p) == ptr(i, p - 1) + len[p - 1];
         if (i > 0) strided = strided && ptr(i, p0) - ptr(i - 1, p0) == ptr(1, p0) - ptr(0, p0);
     }
-    if (strided && count > 1 && ptr(1, p0) - ptr(0, p0) >= (ptrdiff_t)width) {
-        IPB_CK(cudaMemcpy2DAsync(S.lane.qraw + off[p0], S.qstride * 8, ptr(0, p0), (ptr(1, p0) - ptr(0, p0)) * 8,
-                                 width * 8, count, cudaMemcpyHostToDevice, st));
+    const ptrdiff_t pitch = count > 1 ? ptr(1, p0) - ptr(0, p0) : 0;
+    if (strided && pitch >= (ptrdiff_t)width && one_array(ptr(0, p0), (size_t)pitch, width, count, S.qstride)) {
+        IPB_CK(cudaMemcpy2DAsync(S.lane.qraw + off[p0], S.qstride * 8, ptr(0, p0), (size_t)pitch * 8, width * 8, count,
+                                 cudaMemcpyHostToDevice, st));
         return;
     }
     for (size_t i = 0; i < count; ++i) {
