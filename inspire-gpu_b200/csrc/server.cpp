@@ -393,9 +393,11 @@ static void pinned_range(const void* p, uintptr_t& start, size_t& size) {
 }
 
 // Whether `count` rows of `width` words, `pitch` words apart from p on, are
-// parts of one array: of one pinned range at any pitch a 2-D copy takes, or of
-// pageable queries back to back.  Queries of separate allocations can have a
-// constant stride too (two always do), of any size, some pinned and some not.
+// parts of one array: of one pinned range, at any pitch within a 2-D copy's
+// documented limit (driver 580 took 3.2 GB as well), or of pageable queries back
+// to back.  Queries of separate allocations can have a constant stride too (two
+// always do), some pinned and some not, and no copy is to rest on what the
+// driver makes of that.
 static bool one_array(const uint64_t* p, size_t pitch, size_t width, size_t count, size_t qstride) {
     if (pitch > (size_t)INT32_MAX / 8) return false;
     const uint64_t* const end = p + (count - 1) * pitch + width;

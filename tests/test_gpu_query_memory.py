@@ -35,7 +35,7 @@ def _placed(words, qs, step):
 @pytest.mark.parametrize("count", [2, 6])   # copied as a small batch, and in parts
 def test_queries_gigabytes_apart(env, count):
     s, qs, want = env
-    step = 3 << 27                            # 3.2 GB: beyond the pitch of a 2-D copy
+    step = 3 << 27                            # 3.2 GB: beyond the documented pitch of a 2-D copy
     words = _words(step * (count - 1) + qs.shape[1])
     assert (s.answer_batch(_placed(words, qs[:count], step)) == want[:count]).all()
 
