@@ -230,26 +230,25 @@ class CpuQuery:
     """The CPU restatement of the reference's server path (the oracle port:
     orc_answer = mat-vec over every DB column, the tensor pass of every group
     in parallel on all host threads, the full Horner chain) answering one
-    whole query, unsampled.  Geometry comes from the reference's own setup()
-    (its CPU library built from its sources); the DB, the precomputed
+    whole query, unsampled.  setup(n_entries, w) gives the geometry
+    [n_entries, w, R, C, G, D, cts]; the DB, the precomputed
     tensors and the query are synthetic residues (the work does not depend
     on their values).  If the host cannot hold the DB and the tensors, the
     1 GB geometry setup(2^25, 30) is used instead and the sample says so."""
 
-    def __init__(self, n_entries, w):
+    def __init__(self, setup, n_entries, w):
         sys.path.insert(0, os.path.join(REPO, "tests"))
-        from oracle_lib import PRE_A, PRE_D, PRE_F, Oracle, RefLib
+        from oracle_lib import PRE_A, PRE_D, PRE_F, Oracle
         self.o = Oracle()
         self.threads = self.o.L.orc_num_threads()
-        ref = RefLib()
-        geom = ref.setup(n_entries, w)
+        geom = setup(n_entries, w)
         need = lambda g: g[2] * g[3] * 2 + g[4] * (PRE_A + 2 * PRE_D + PRE_F) * 4
         avail = host_mem_available()
         self.note = ""
         if avail is not None and need(geom) > 0.7 * avail:
             self.note = (f"; host MemAvailable {avail / 1e9:.0f} GB cannot hold the {need(geom) / 1e9:.1f} GB "
                          f"geometry, so the 1 GB geometry setup(2^25, 30) is timed instead")
-            geom = ref.setup(1 << 25, 30)
+            geom = setup(1 << 25, 30)
         self.geom = geom
         _, _, R, Cc, G, D, ncts = geom
         self.R, self.C, self.D = R, Cc, D
@@ -290,10 +289,18 @@ class CpuQuery:
                 f"synthetic DB, tensors and query{self.note}")
 
 
-def cpu_baseline(n_entries, w, timed=2):
+def cpu_baseline(ib, n_entries, w, timed=2):
     """cpu_baseline of our arm's line: the same full CPU query, median of
-    `timed` runs after one untimed run."""
-    cq = CpuQuery(n_entries, w)
+    `timed` runs after one untimed run.  The line does without it where the
+    oracle is not built."""
+    def setup(n, w):
+        p = ib.setup(n, w)
+        return [p[k] for k in ("n_entries", "entry_bytes", "db_rows", "db_cols", "n_packed", "interp_d", "num_cts")]
+
+    try:
+        cq = CpuQuery(setup, n_entries, w)
+    except FileNotFoundError as e:
+        return {"unavailable": str(e)}
     cq.answer_s()
     ts = [cq.answer_s() for _ in range(timed)]
     t = statistics.median(ts)
@@ -318,11 +325,18 @@ def run_reference(args):
     """The reference has no CPU server of its own (docs/ARCHITECTURE.md:378-380),
     so its CPU path is the oracle port: one full query per step on all host
     threads.  Nothing of this build's library is loaded here: the geometry
-    comes from the reference's own setup()."""
+    comes from the reference's own setup(), in its CPU library built from its
+    sources."""
     rank, _, world = dist_env()
     if rank != 0:
         return
-    cq = CpuQuery(args.n_entries, args.entry_bytes)
+    sys.path.insert(0, os.path.join(REPO, "tests"))
+    from oracle_lib import RefLib
+    try:
+        cq = CpuQuery(RefLib().setup, args.n_entries, args.entry_bytes)
+    except FileNotFoundError as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     _, _, R, Cc, G, D, ncts = cq.geom
     params = {"n_entries": cq.geom[0], "entry_bytes": cq.geom[1], "db_rows": R, "db_cols": Cc, "n_packed": G,
               "interp_d": D, "num_cts": ncts}
@@ -609,7 +623,7 @@ def run_ours(args):
     if serving:
         line["serving"] = serving
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        line["cpu_baseline"] = cpu_baseline(args.n_entries, args.entry_bytes)
+        line["cpu_baseline"] = cpu_baseline(ib, args.n_entries, args.entry_bytes)
     srv.close()
     if rank == 0 and world == 1 and not args.no_configs:
         # the other configurations, shortened, so one default run records them all
