@@ -460,12 +460,12 @@ int lane_gt_pass(size_t cap) { return (int)std::min<size_t>(cap, (size_t)kTpMaxQ
 
 static bool chunked_ok(const Server& S, const Sched& sc, size_t count);
 
-// SMs for the tensor pass beside the mat-vec where nothing else is asked for
-// (default_sched has the measurements).
-static int default_tp_sms(const Server& S) {
-    const double stream_bytes =
-        2.0 * (double)S.pp.db_rows * (double)S.pp.db_cols + (double)tp_dt_bytes(S.pp.n_packed);
-    return stream_bytes <= 8e9 ? S.num_sms * 2 / 3 : 0;
+// SMs for the tensor pass beside the mat-vec for a batch of `count` where
+// nothing else is asked for (default_sched has the measurements).
+static int default_tp_sms(const Server& S, size_t count) {
+    const double db = 2.0 * (double)S.pp.db_rows * (double)S.pp.db_cols, dt = (double)tp_dt_bytes(S.pp.n_packed);
+    if (count > kSliceQueries || (S.pp.n_packed == 1 && db >= dt)) return 0;
+    return db + dt <= (count <= 1 || db >= dt ? 8e9 : count == 2 ? 4e9 : 2e9) ? S.num_sms * 2 / 3 : 0;
 }
 
 // Defaults per batch size, each line drawn where both sides measured alike
@@ -481,11 +481,18 @@ static int default_tp_sms(const Server& S) {
 //     8 chunks up to 2 queries (2: 3.82, 4 chunks 3.90), 4 beyond (8: 4.05 /
 //     4.30 with 8: the chains of a chunk hold their SMs longer).
 //   Tensor pass beside the mat-vec, on two SMs of three, where the two streams
-//     are short enough for launch ramps and tails to count (up to 8 GB
-//     together): 1 GB 293 -> 281 us at 1 query, 410 -> 390 at 32; 4 GB (6.4 GB
-//     together) 1077 -> 1047 and 1472 -> 1383; 1 group on 2048 rows 62 -> 52 at
-//     32.  Beyond, either order streams at the HBM rate: 128 groups on 2048 rows
-//     (9.7 GB) 1733 / 1726 and 1792 / 2022 at 8, 16 GB 4.02 / 4.03 ms.
+//     are short enough for launch ramps and tails to count (device times of
+//     staged batches, after / beside).  Database at least as long as its tensors:
+//     up to 8 GB together, 32768 rows: 0.8 GB 170 / 158 us at 1 query, 211 / 206
+//     at 32; 6.4 GB 1057 / 1035 and 1429 / 1325, at 8 even.  Tensors longer: 4 groups
+//     on 2048 rows 98 / 78 at 4 queries, 1.2 GB 287 / 282 at 8; from 3 queries up to
+//     2 GB (2048 rows, 2.4 GB: 497 / 518 at 4, 4.8 GB 933 / 1020 at 8), at 2 up to 4 GB
+//     (8192 rows, 3.2 GB 642 / 620, 6.4 GB 1121 / 1219), at 1 up to 8 GB (1113 / 1103).
+//     Not with the two-slice tensor pass of more than 32 queries (64: 1.2 GB 483 /
+//     527, 32768 rows 3.2 GB 1243 / 1262), nor for one group whose mat-vec is the longer
+//     (32768 rows: 70 / 73; the pass's 128 tiles take two rounds on 98 SMs).  Beyond 8 GB
+//     either order streams at the HBM rate (no geometry lies between 6.4 and 8.6 GB;
+//     9.7 GB 1733 / 1716 at 1 query, 1864-1930 / 2008 at 8).
 // IPB_MATVEC, IPB_HORNER, IPB_TP_SMS and IPB_HCHUNKS pin a choice for every
 // batch size.
 std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
@@ -510,7 +517,7 @@ std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
         if (k) sc.hchunks = std::max(0, std::min(std::atoi(k), kMaxHChunks));
         if (!sc.matvec_tc) continue;
         if (t) sc.tp_sms = std::max(0, std::min(std::atoi(t), S.num_sms - 1));
-        else if (sc.hchunks <= 1) sc.tp_sms = default_tp_sms(S);
+        else if (sc.hchunks <= 1) sc.tp_sms = default_tp_sms(S, c);
     }
     return out;
 }
@@ -552,6 +559,9 @@ int run_db_phase(const Server& S, Lane& L, const Sched& sc, size_t q_off, size_t
     // Horner stream while the mat-vec (DB only) starts on the other SMs; both
     // are persistent with one CTA per SM, so the mat-vec's remaining CTAs start
     // as the tensor pass's end.  Stage timing needs them one after the other.
+    // (While the mat-vec waits for LWE vectors to land, the tensor pass could have
+    // every SM: blocking answers at 32768 rows and 3.2 GB take 655 instead of 685 us
+    // at 8 queries, but a shard of 21 groups 750 instead of 713, 2048 rows 166 / 160.)
     const bool beside = !ev && sc.matvec_tc && sc.tp_sms > 0 && sc.tp_sms < S.num_sms && span > 0;
     auto tensor_pass = [&](cudaStream_t ts, int sms) {
         for (size_t c0 = 0; c0 < span; c0 += tp_pass) {
@@ -625,7 +635,7 @@ static bool chunked_ok(const Server& S, const Sched& sc, size_t count) {
 bool runs_chunked(const Server& S, const Sched& sc, size_t count) { return chunked_ok(S, sc, count); }
 
 void yield_default_split(const Server& S, Sched& sc, size_t count) {
-    if (std::getenv("IPB_TP_SMS") || sc.tp_sms != default_tp_sms(S)) return;
+    if (std::getenv("IPB_TP_SMS") || sc.tp_sms != default_tp_sms(S, count)) return;
     Sched whole = sc;
     whole.tp_sms = 0;
     if (!sc.matvec_tc || chunked_ok(S, whole, count)) sc = whole;
