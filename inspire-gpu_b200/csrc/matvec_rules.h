@@ -24,11 +24,15 @@ inline bool mv_kchunk_ok(size_t rows, int kchunk_rows) {
 // Tiles per work item for a pass of nq queries over a DB of ld columns per
 // row.  Two while their accumulators fit TMEM (18 queries), if the DB is small
 // enough for the tail of its few items to count or the batch large enough for
-// the planes to (up to 6 GB, or from 6 queries: over 16 GB 1 query takes 2.41 ms
-// with one tile and 2.48 with two, 4: 2.50 / 2.57, 8: 2.78 / 2.59), and if the
-// accumulators are double-buffered or an item long enough for that not to
-// matter (16 queries, 640 rows an item: 31 us with one tile, 36 with two; 2048
-// rows 214 / 217; 8192 rows 214 / 196).  pairs: the launch's tiles pair up
+// the planes to, and if the accumulators are double-buffered or an item long
+// enough for that not to matter (16 queries, 640 rows an item: 31 us with one
+// tile, 36 with two; 2048 rows 214 / 217; 8192 rows 214 / 196).
+// Both sides of the lines, 32768 rows, one tile / two.  By size, 1 query: 3.2 GB
+// 482 / 461 us, 4.3 677 / 648, 5.4 838 / 835 (5 queries 835 / 866), 6.4 1030 / 950,
+// 7.5 1155 / 1153, 8.6 1212 / 1235, 17.2 2380 / 2454: two gain up to 4.3 GB and lose
+// from 8.6, and between them the items' last wave decides.  By queries over 17.2
+// GB, ms: 2 2.48 / 2.54, 4 2.51 / 2.57, 5 2.68 / 2.59, 6 2.76 / 2.67, 8 2.82 / 2.68, 12
+// 2.90 / 2.85.  pairs: the launch's tiles pair up
 // (an even number of them in every column range).
 inline int mv_tiles(int nq, size_t rows, size_t ld, int kchunk_rows, bool pairs) {
     const int npad = (kPlanes * nq + 15) / 16 * 16;

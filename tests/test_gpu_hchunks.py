@@ -2,9 +2,11 @@
 hchunks: at most that many chunks): the tensor pass first, then the mat-vec
 and finalize chunk by chunk from the top group down, each chunk's Horner
 steps on a second stream resuming the chain from memory.  The chunks are
-whole waves of mat-vec work growing by one wave per chunk from the bottom
-(at 128 groups on 148 SMs: 119 + 9, 101 + 18 + 9 and 37 + 37 + 27 + 18 + 9
-for at most 2, 3 and 8 chunks; 4 + 4 at 8 groups).  Every chunking, with both cluster Horner kernels, through the blocking
+whole waves of mat-vec work growing by one wave per chunk from the bottom.
+At 128 groups on 148 SMs, for at most 2, 3 and 8 chunks: 110 + 18, 73 + 37
++ 18 and 18 + 55 + 37 + 18 up to 18 queries (two m' tiles per work item),
+119 + 9, 101 + 18 + 9 and 37 + 37 + 27 + 18 + 9 beyond; 8 groups are one
+chunk.  Every chunking, with both cluster Horner kernels, through the blocking
 answer (host views), the staged path (stage_views / run / fetch) and stage
 timing (which runs unchunked), gives the unchunked responses bit for bit,
 and those are pinned to the oracle and to extract()."""
