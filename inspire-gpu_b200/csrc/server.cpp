@@ -404,7 +404,7 @@ static bool one_array(const uint64_t* p, size_t pitch, size_t width, size_t coun
     uintptr_t start = 0;
     size_t size = 0;
     pinned_range(p, start, size);
-    if (size) return (uintptr_t)end <= start + size;
+    if (size) return (uintptr_t)p >= start && (uintptr_t)end <= start + size;
     pinned_range(end - 1, start, size);
     return size == 0 && pitch == qstride;
 }
