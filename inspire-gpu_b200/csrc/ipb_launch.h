@@ -122,6 +122,9 @@ cudaError_t launch_horner_cluster(const uint32_t* pre_a, const uint32_t* packed_
                                   size_t num_cts, uint64_t* resp, size_t resp_qstride, int nq, int* err,
                                   cudaStream_t s, HornerRange hr = HornerRange{});
 // Same on a cluster of eight CTAs per chain (polynomial x limb x digit).
+// Chains of 8 CTAs that the current device runs at once with an SM per CTA (15
+// on a whole B200; the GPCs' sizes decide).
+size_t horner_cl8_chains();
 cudaError_t launch_horner_cluster8(const uint32_t* pre_a, const uint32_t* packed_b, size_t pb_qstride,
                                    const uint32_t* rgsw32, const DevTables* T, size_t groups, size_t d_act,
                                    size_t num_cts, uint64_t* resp, size_t resp_qstride, int nq, int* err,

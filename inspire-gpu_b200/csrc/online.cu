@@ -11,6 +11,7 @@
 //             ExtProd chain (INTT, decomp, NTT, MAC) in shared memory
 // All arithmetic is exact mod q_l, so every output equals the reference's.
 #include <algorithm>
+#include <atomic>
 
 #include "ipb_common.cuh"
 #include "host_util.h"
@@ -585,6 +586,8 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 1)
 // step t - 2.  Half the warps per SM of the 4-CTA version, twice the SMs.
 constexpr size_t kHornerCl8Smem =
     2 * kN * sizeof(uint2) + (kNttBuf + 2 * kN + 2 * 3 * kN) * sizeof(uint32_t) + 64;
+constexpr size_t kHornerCl8AloneSmem = 116 * 1024;  // more than half an SM's
+static_assert(kHornerCl8Smem <= kHornerCl8AloneSmem, "room for the kernel's own");
 
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 1)
     horner_cl8_kernel(const uint32_t* __restrict__ pre_a, const uint32_t* __restrict__ packed_b, size_t pb_qstride,
@@ -898,6 +901,24 @@ cudaError_t launch_horner_cluster(const uint32_t* pre_a, const uint32_t* packed_
                              pb_qstride, rgsw32, T, groups, d_act, resp, resp_qstride, err, hr);
 }
 
+size_t horner_cl8_chains() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if ((n = known[dev].load()) > 0) return (size_t)n;
+    cudaLaunchConfig_t cfg{};  // the cluster's size is the kernel's own
+    cfg.gridDim = dim3(8);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = kHornerCl8AloneSmem;
+    if (allow_max_smem(horner_cl8_kernel) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, horner_cl8_kernel, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        return 0;
+    }
+    known[dev].store(n);
+    return (size_t)n;
+}
+
 cudaError_t launch_horner_cluster8(const uint32_t* pre_a, const uint32_t* packed_b, size_t pb_qstride,
                                    const uint32_t* rgsw32, const DevTables* T, size_t groups, size_t d_act,
                                    size_t num_cts, uint64_t* resp, size_t resp_qstride, int nq, int* err,
@@ -906,8 +927,15 @@ cudaError_t launch_horner_cluster8(const uint32_t* pre_a, const uint32_t* packed
     if (!horner_range_ok(hr, d_act)) return cudaErrorInvalidValue;
     cudaError_t e = allow_max_smem(horner_cl8_kernel);
     if (e) return e;
-    return launch_overlapped(horner_cl8_kernel, dim3((unsigned)(8 * num_cts), nq), 256, kHornerCl8Smem, s, pre_a,
-                             packed_b, pb_qstride, rgsw32, T, groups, d_act, resp, resp_qstride, err, hr);
+    // A whole chain starts while the kernel before it still holds SMs.  Two of its
+    // CTAs fit one SM, and clusters that are placed so share it for the whole chain
+    // (10 queries, 128 groups on 2048 rows: 2037 us, started late 1811).  Chains that
+    // can all have SMs of their own ask for so much shared memory that they get
+    // them (1810).
+    const bool alone = hr.i_first < 0 && hr.i_last == 0 && (size_t)nq * num_cts <= horner_cl8_chains();
+    return launch_overlapped(horner_cl8_kernel, dim3((unsigned)(8 * num_cts), nq), 256,
+                             alone ? kHornerCl8AloneSmem : kHornerCl8Smem, s, pre_a, packed_b, pb_qstride, rgsw32, T,
+                             groups, d_act, resp, resp_qstride, err, hr);
 }
 
 cudaError_t launch_ntt_batch(uint32_t* polys, size_t n, int limb_run, bool inverse, const DevTables* T,

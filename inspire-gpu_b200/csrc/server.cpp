@@ -470,9 +470,9 @@ static int default_tp_sms(const Server& S, size_t count) {
 
 // Defaults per batch size, each line drawn where both sides measured alike
 // (one GPU, medians of interleaved runs):
-//   Horner kernel: 8 CTAs per chain while all clusters run at once (up to 15
-//     chains, 3.2 us a step), 4 CTAs beyond (4.0 us; 16 chains of 8 CTAs take
-//     5.1 us).
+//   Horner kernel: 8 CTAs per chain while all clusters run at once with an SM
+//     per CTA (horner_cl8_chains, 15 here: 3.2 us a step at 1 to 15 chains), 4
+//     CTAs beyond (4.0 us; 16 chains of 8 CTAs take 5.1 us).
 //   Horner chain trailing the DB pass in chunks where a chunk's mat-vec lasts
 //     longer than its chain steps (32768 rows: 19 us a group against 4-11) and
 //     the chain is worth the extra launches: 128 groups, 16 GB: 1 query 3.69
@@ -497,6 +497,7 @@ static int default_tp_sms(const Server& S, size_t count) {
 // batch size.
 std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
     const size_t G = S.pp.n_packed, chain = std::min(S.pp.D, G);  // groups per response ciphertext
+    const size_t cl8_chains = horner_cl8_chains();
     const char* const m = std::getenv("IPB_MATVEC");
     const char* const h = std::getenv("IPB_HORNER");
     const char* const t = std::getenv("IPB_TP_SMS");
@@ -506,7 +507,7 @@ std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
         Sched& sc = out[c];
         sc.tp_pass = gt_pass;
         if (m) sc.matvec_tc = std::strcmp(m, "simt") != 0;
-        sc.horner_cluster = c * S.pp.num_cts <= 15 ? 2 : 1;
+        sc.horner_cluster = c * S.pp.num_cts <= cl8_chains ? 2 : 1;
         if (chain >= 64 && S.pp.db_rows >= 16384 && c <= std::min<size_t>(16, chain / 8)) {
             Sched chunked = sc;
             chunked.horner_cluster = 1;

@@ -61,3 +61,18 @@ def test_a_schedule_read_back_takes_chunks_and_the_cuda_core_matvec(srv, queries
     with pytest.raises(Exception):
         launches(matvec_tc=0, tp_sms=40)
     srv.set_schedule(2, **first)
+
+
+@pytest.mark.parametrize("count", [1, 15, 16, 17])
+def test_eight_cta_chains_alone_on_their_sms_and_not(count):
+    """Chains of 8 CTAs that all fit with an SM per CTA (15 on a whole B200), and
+    more, give the responses of the other Horner kernels."""
+    import inspire_b200 as ib
+    cols = 4 * ib.RING_N
+    qs = list(ib.synth_queries_host(R, 37, 0, count))
+    with ib.Server(R * cols // 64, 120, ib.fill_db(R * cols, 3), db_rows=R, max_batch=count, crs_seed=bytes(64)) as s:
+        got = []
+        for hc in (2, 1, 0):
+            s.set_schedule(count, horner_cluster=hc)
+            got.append(s.answer_batch(qs))
+    assert (got[0] == got[1]).all() and (got[0] == got[2]).all()
