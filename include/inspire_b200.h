@@ -263,9 +263,10 @@ int ipir_b200_fill_db_device(uint16_t* out, size_t count, uint64_t seed, void* s
  * the serving loop's lane batches), 0 off.  Defaults: horner_cluster 2 up to
  * 15 chains, else 1; hchunks 8 (4 above two queries) with horner_cluster 1 on
  * databases of at least 16384 rows with L >= 64, for batches of at most
- * min(16, L / 8) queries; otherwise tp_sms two thirds of the SMs, for up to 32
- * queries, where the database and its tensors take at most 8 GB (4 GB at 2
- * queries and 2 GB from 3 on where the tensors are the larger part).  Every schedule gives the same responses. */
+ * min(16, L / 8) queries; otherwise tp_sms two thirds of the SMs where the
+ * database and its tensors take at most 8 GB, for up to 32 queries (16 where the
+ * tensors are the larger part and the two take more than 1.5 GB).  Every schedule
+ * gives the same responses. */
 typedef struct {
     int matvec_tc;
     int tp_pass;

@@ -375,20 +375,19 @@ static void stage_queries(Server* S, const ipir_query_view* qs, size_t count) {
 // p, or size 0 for other memory.  The driver's entry point through the runtime:
 // the library needs no -lcuda.
 static void pinned_range(const void* p, uintptr_t& start, size_t& size) {
-    using Get = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    using Get = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
     static const Get get = [] {
         void* f = nullptr;
         cudaDriverEntryPointQueryResult r;
-        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &r) == cudaSuccess &&
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &r) == cudaSuccess &&
                         r == cudaDriverEntryPointSuccess;
         return ok ? reinterpret_cast<Get>(f) : nullptr;
     }();
-    const CUdeviceptr at = (CUdeviceptr)(uintptr_t)p;
+    CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
     CUdeviceptr first = 0;
     size = 0;
-    if (!get || get(&first, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
-        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
-        size = 0;
+    void* into[2] = {&first, &size};
+    if (!get || get(2, what, into, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) size = 0;
     start = (uintptr_t)first;
 }
 
@@ -465,7 +464,7 @@ static bool chunked_ok(const Server& S, const Sched& sc, size_t count);
 static int default_tp_sms(const Server& S, size_t count) {
     const double db = 2.0 * (double)S.pp.db_rows * (double)S.pp.db_cols, dt = (double)tp_dt_bytes(S.pp.n_packed);
     if (count > kSliceQueries || (S.pp.n_packed == 1 && db >= dt)) return 0;
-    return db + dt <= (count <= 1 || db >= dt ? 8e9 : count == 2 ? 4e9 : 2e9) ? S.num_sms * 2 / 3 : 0;
+    return db + dt <= (count <= 16 || db >= dt ? 8e9 : 1.5e9) ? S.num_sms * 2 / 3 : 0;
 }
 
 // Defaults per batch size, each line drawn where both sides measured alike
@@ -482,17 +481,17 @@ static int default_tp_sms(const Server& S, size_t count) {
 //     4.30 with 8: the chains of a chunk hold their SMs longer).
 //   Tensor pass beside the mat-vec, on two SMs of three, where the two streams
 //     are short enough for launch ramps and tails to count (device times of
-//     staged batches, after / beside).  Database at least as long as its tensors:
-//     up to 8 GB together, 32768 rows: 0.8 GB 170 / 158 us at 1 query, 211 / 206
-//     at 32; 6.4 GB 1057 / 1035 and 1429 / 1325, at 8 even.  Tensors longer: 4 groups
-//     on 2048 rows 98 / 78 at 4 queries, 1.2 GB 287 / 282 at 8; from 3 queries up to
-//     2 GB (2048 rows, 2.4 GB: 497 / 518 at 4, 4.8 GB 933 / 1020 at 8), at 2 up to 4 GB
-//     (8192 rows, 3.2 GB 642 / 620, 6.4 GB 1121 / 1219), at 1 up to 8 GB (1113 / 1103).
-//     Not with the two-slice tensor pass of more than 32 queries (64: 1.2 GB 483 /
-//     527, 32768 rows 3.2 GB 1243 / 1262), nor for one group whose mat-vec is the longer
-//     (32768 rows: 70 / 73; the pass's 128 tiles take two rounds on 98 SMs).  Beyond 8 GB
-//     either order streams at the HBM rate (no geometry lies between 6.4 and 8.6 GB;
-//     9.7 GB 1733 / 1716 at 1 query, 1864-1930 / 2008 at 8).
+//     staged batches, after / beside): up to 8 GB together and 16 queries.  4 groups
+//     on 2048 rows 93 / 78 us at 4 queries; 32768 rows 0.8 GB 170 / 157 at 1, 1.6 GB
+//     297 / 288 at 8, 6.4 GB 1054 / 1034 at 1 and 1174 / 1144 at 16; 8192 rows 6.4 GB
+//     1153 / 1141 at 8.  To 32 queries also where the database is at least as long
+//     as its tensors (32768 rows 6.4 GB 1361 / 1303; 16384 rows 4.3 GB 931 / 927);
+//     with the tensors longer up to 1.5 GB (2048 rows 1.2 GB 311 / 310; 8192 rows 1.6 GB
+//     379 / 385, 6.4 GB 1420 / 1496).  Not with the two-slice tensor pass of more than
+//     32 queries (64: 1.2 GB 485 / 528, 32768 rows 3.2 GB 1250 / 1270), nor for one
+//     group whose mat-vec is the longer (32768 rows: 70 / 72 at 1, 75 / 79 at 8; the
+//     pass's 128 tiles take two rounds on 98 SMs).  Beyond 8 GB either order streams
+//     at the HBM rate (no geometry lies between 6.4 and 8.6 GB).
 // IPB_MATVEC, IPB_HORNER, IPB_TP_SMS and IPB_HCHUNKS pin a choice for every
 // batch size.
 std::vector<Sched> default_sched(const Server& S, size_t cap, int gt_pass) {
